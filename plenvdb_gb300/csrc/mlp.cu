@@ -4,36 +4,20 @@
 // part W0[:,C0:]·PE(viewdir) + b0 computed once per ray (the reference
 // renderer hoists it the same way, renderer.cu:100-101).
 //
-// FP32 SIMT kernels: persistent CTAs over 64-row tiles; every thread owns a
-// 4-row x 8-column block (columns strided by 16 so the padded weight rows are
-// read without bank conflicts). The backward recomputes the activations of its
-// tile, and accumulates the weight gradients of all tiles it visits in
-// registers; per-CTA partials are summed in CTA order by k_wgrad_reduce, so the
-// weight gradients are deterministic for a given grid size.
+// The FP32 kernels are in mlp_f32.cu, the BF16 tensor-core kernels in
+// mlp_tc.cu; both leave per-CTA partial weight gradients that k_wgrad_reduce
+// sums in CTA order, so the weight gradients are deterministic for a given
+// grid size.
 #include <algorithm>
 
 #include "march.cuh"
+#include "mlp_f32.cuh"
 
 namespace pvdb {
 
-constexpr int kW = 128;       // hidden width
-constexpr int kTile = 64;     // rows per tile
-constexpr int kMaxC0 = 16;    // k0 channels
-constexpr int kMaxPe = 32;    // PE dims
-constexpr int kW1S = kW + 1;  // padded row stride of W1 in shared memory
-constexpr int kAS = kTile + 4;  // row stride of transposed activation tiles
-constexpr int kMlpThreads = 256;
-
-struct MlpArgs {
-  const float* w0; const float* b0;
-  const float* w1; const float* b1;
-  const float* w2; const float* b2;
-  int c0, dpe, din;  // din = c0 + dpe
-};
-
-// Flat parameter layout shared with the train step and the Python side:
-// [w0 (128 x din), b0 (128), w1 (128 x 128), b1 (128), w2 (3 x 128), b2 (3)].
-__host__ __device__ inline int64_t mlp_param_count(int din) { return int64_t(kW) * din + kW + kW * kW + kW + 3 * kW + 3; }
+constexpr int kW = 128;     // hidden width
+constexpr int kMaxC0 = 16;  // k0 channels
+constexpr int kMaxPe = 32;  // PE dims
 
 // PE of a unit view direction (dvgo.py:354-355): [d, sin(d*2^i), cos(d*2^i)]
 // with the frequencies innermost per axis: sin at 3 + a*npe + i, cos at
@@ -75,309 +59,6 @@ __global__ void __launch_bounds__(128)
     for (int q = 0; q < a.dpe; ++q) s = fmaf(wt[q][n], pe_s[rr][q], s);
     hpe[int64_t(r0 + rr) * kW + n] = b + s;
   }
-}
-
-struct MlpSmem {
-  float w1[kW * kW1S];
-  float w0k[kW * (kMaxC0 + 1)];
-  float w2[3 * kW];
-  float b1[kW];
-  float b2[4];
-  float x[kTile * kMaxC0];  // k0 rows of the tile
-  float h0t[kW * kAS];      // relu(layer 0), transposed [n][row]
-};
-
-__device__ void mlp_load_weights(MlpSmem& S, const MlpArgs& a) {
-  for (int i = threadIdx.x; i < kW * kW; i += blockDim.x) S.w1[(i / kW) * kW1S + (i % kW)] = a.w1[i];
-  for (int i = threadIdx.x; i < kW * a.c0; i += blockDim.x)
-    S.w0k[(i / a.c0) * (kMaxC0 + 1) + (i % a.c0)] = a.w0[(i / a.c0) * a.din + (i % a.c0)];
-  for (int i = threadIdx.x; i < 3 * kW; i += blockDim.x) S.w2[i] = a.w2[i];
-  for (int i = threadIdx.x; i < kW; i += blockDim.x) S.b1[i] = a.b1[i];
-  if (threadIdx.x < 3) S.b2[threadIdx.x] = a.b2[threadIdx.x];
-}
-
-// Layer 0 and layer 1 of one tile; returns relu(layer 1) in h1[4][8] for rows
-// ty*4+i and columns tx+16*j. Leaves relu(layer 0) in S.h0t.
-__device__ __forceinline__ void mlp_tile_forward(MlpSmem& S, const MlpArgs& a,
-                                                 const float* __restrict__ k0,
-                                                 const int32_t* __restrict__ ray,
-                                                 const float* __restrict__ hpe, int64_t row0,
-                                                 int64_t M, float h1[4][8]) {
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  for (int i = threadIdx.x; i < kTile * a.c0; i += blockDim.x) {
-    const int rr = i / a.c0, q = i % a.c0;
-    const int64_t m = row0 + rr;
-    S.x[rr * kMaxC0 + q] = m < M ? k0[m * a.c0 + q] : 0.f;
-  }
-  __syncthreads();
-  // layer 0
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int rr = ty * 4 + i;
-    const int64_t m = row0 + rr;
-    const int r = m < M ? ray[m] : -1;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int n = tx + 16 * j;
-      float z = r >= 0 ? hpe[int64_t(r) * kW + n] : 0.f;
-      for (int q = 0; q < a.c0; ++q) z = fmaf(S.w0k[n * (kMaxC0 + 1) + q], S.x[rr * kMaxC0 + q], z);
-      S.h0t[n * kAS + rr] = fmaxf(z, 0.f);
-    }
-  }
-  __syncthreads();
-  // layer 1
-  float acc[4][8];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
-#pragma unroll 4
-  for (int k = 0; k < kW; ++k) {
-    const float4 av = *reinterpret_cast<const float4*>(&S.h0t[k * kAS + ty * 4]);
-    const float aa[4] = {av.x, av.y, av.z, av.w};
-    float bb[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) bb[j] = S.w1[(tx + 16 * j) * kW1S + k];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(aa[i], bb[j], acc[i][j]);
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) h1[i][j] = fmaxf(acc[i][j] + S.b1[tx + 16 * j], 0.f);
-}
-
-// Layer 2 logits for rows ty*4+i: partial dot products over this thread's
-// columns, reduced over the 16 threads of the row group (xor within 16 lanes).
-__device__ __forceinline__ void mlp_logits(const MlpSmem& S, const float h1[4][8], float lg[4][3]) {
-  const int tx = threadIdx.x & 15;
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      float s = 0.f;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) s = fmaf(S.w2[c * kW + tx + 16 * j], h1[i][j], s);
-#pragma unroll
-      for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-      lg[i][c] = s + S.b2[c];
-    }
-}
-
-__global__ void __launch_bounds__(kMlpThreads, 1)
-    k_mlp_fwd_f32(MlpArgs a, const float* __restrict__ k0, const int32_t* __restrict__ ray,
-                  const float* __restrict__ hpe, const uint32_t* __restrict__ totals,
-                  float* rgb, int out_logits) {
-  grid_dep_sync();
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  MlpSmem& S = *reinterpret_cast<MlpSmem*>(smem_raw);
-  const int64_t M = totals[1];
-  const int64_t ntiles = (M + kTile - 1) / kTile;
-  if (blockIdx.x >= ntiles) return;
-  mlp_load_weights(S, a);
-  __syncthreads();
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const int64_t row0 = t * kTile;
-    float h1[4][8];
-    mlp_tile_forward(S, a, k0, ray, hpe, row0, M, h1);
-    float lg[4][3];
-    mlp_logits(S, h1, lg);
-    if (tx == 0) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int64_t m = row0 + ty * 4 + i;
-        if (m < M)
-#pragma unroll
-          for (int c = 0; c < 3; ++c)
-            rgb[m * 3 + c] = out_logits ? lg[i][c] : 1.f / (1.f + expf(-lg[i][c]));
-      }
-    }
-    __syncthreads();
-  }
-}
-
-struct MlpBwdSmem {
-  MlpSmem f;
-  float dl[kTile * 4];       // d logits [row][c]
-  float dz1t[kW * kAS];      // d(layer-1 pre-activation), transposed [n][row]
-  float dz0t[kW * kAS];      // d(layer-0 pre-activation), transposed [n][row]
-  float pe[kTile * kMaxPe];  // PE rows of the tile
-};
-
-// Per-CTA partial gradient layout (same as the flat parameter layout).
-__global__ void __launch_bounds__(kMlpThreads, 1)
-    k_mlp_bwd_f32(MlpArgs a, const float* __restrict__ k0, const int32_t* __restrict__ ray,
-                  const float* __restrict__ hpe, const float* __restrict__ pe_buf,
-                  const uint32_t* __restrict__ totals, const float* __restrict__ rgb,
-                  const float* __restrict__ grad_rgb, float* grad_k0, float* wpart) {
-  grid_dep_sync();
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  MlpBwdSmem& B = *reinterpret_cast<MlpBwdSmem*>(smem_raw);
-  MlpSmem& S = B.f;
-  const int64_t M = totals[1];
-  const int64_t ntiles = (M + kTile - 1) / kTile;
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  const int64_t P = mlp_param_count(a.din);
-  float* part = wpart + int64_t(blockIdx.x) * P;
-  float* pw0 = part;
-  float* pb0 = pw0 + kW * a.din;
-  float* pw1 = pb0 + kW;
-  float* pb1 = pw1 + kW * kW;
-  float* pw2 = pb1 + kW;
-  float* pb2 = pw2 + 3 * kW;
-  // accumulators: dW1 block (n = ty+16i, k = tx+16j), dW0 row n = tid>>1 half q,
-  // db0/db1 for n = tid>>1 (even threads), dW2/db2 entries tid, tid+256
-  float aw1[8][8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) aw1[i][j] = 0.f;
-  const int n0 = tid >> 1, qh = tid & 1;
-  const int qbeg = qh ? (a.din + 1) / 2 : 0, qend = qh ? a.din : (a.din + 1) / 2;
-  float aw0[24];
-#pragma unroll
-  for (int q = 0; q < 24; ++q) aw0[q] = 0.f;
-  float ab0 = 0.f, ab1 = 0.f;
-  float aw2[2] = {0.f, 0.f};
-  float ab2 = 0.f;
-  if (blockIdx.x < ntiles) {
-    mlp_load_weights(S, a);
-    __syncthreads();
-  }
-  for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const int64_t row0 = t * kTile;
-    // PE rows
-    for (int i = tid; i < kTile * a.dpe; i += blockDim.x) {
-      const int rr = i / a.dpe, q = i % a.dpe;
-      const int64_t m = row0 + rr;
-      B.pe[rr * kMaxPe + q] = m < M ? pe_buf[int64_t(ray[m]) * kMaxPe + q] : 0.f;
-    }
-    float h1[4][8];
-    mlp_tile_forward(S, a, k0, ray, hpe, row0, M, h1);
-    // d logits: sigmoid backward
-    if (tid < kTile * 3) {
-      const int rr = tid / 3, c = tid % 3;
-      const int64_t m = row0 + rr;
-      float d = 0.f;
-      if (m < M) {
-        const float y = rgb[m * 3 + c];
-        d = grad_rgb[m * 3 + c] * (1.f - y) * y;
-      }
-      B.dl[rr * 4 + c] = d;
-    }
-    __syncthreads();
-    // dz1 = (dl . W2) * relu'(h1); also dW2 needs h1: write h1 into dz0t scratch
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int rr = ty * 4 + i;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const int n = tx + 16 * j;
-        float g = 0.f;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) g = fmaf(B.dl[rr * 4 + c], S.w2[c * kW + n], g);
-        B.dz1t[n * kAS + rr] = h1[i][j] > 0.f ? g : 0.f;
-        B.dz0t[n * kAS + rr] = h1[i][j];
-      }
-    }
-    __syncthreads();
-    // dW2, db2 (entries e = c*128+n for c<3) and db2
-    for (int e = tid, s = 0; e < 3 * kW; e += blockDim.x, ++s) {
-      const int c = e / kW, n = e % kW;
-      float acc = 0.f;
-      for (int rr = 0; rr < kTile; ++rr) acc = fmaf(B.dl[rr * 4 + c], B.dz0t[n * kAS + rr], acc);
-      aw2[s] += acc;
-    }
-    if (tid < 3) {
-      float acc = 0.f;
-      for (int rr = 0; rr < kTile; ++rr) acc += B.dl[rr * 4 + tid];
-      ab2 += acc;
-    }
-    // dW1[n][k] += sum_row dz1[row][n] * h0[row][k]   (n = ty+16i, k = tx+16j)
-    for (int rr = 0; rr < kTile; ++rr) {
-      float av[8], bv[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) av[i] = B.dz1t[(ty + 16 * i) * kAS + rr];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) bv[j] = S.h0t[(tx + 16 * j) * kAS + rr];
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) aw1[i][j] = fmaf(av[i], bv[j], aw1[i][j]);
-    }
-    if (!qh) {
-      float acc = 0.f;
-      for (int rr = 0; rr < kTile; ++rr) acc += B.dz1t[n0 * kAS + rr];
-      ab1 += acc;
-    }
-    __syncthreads();  // dz0t scratch (h1) no longer needed
-    // dh0[row][k] = sum_n dz1[row][n] * W1[n][k]; dz0 = dh0 * relu'(h0)
-    {
-      float acc[4][8];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
-#pragma unroll 4
-      for (int n = 0; n < kW; ++n) {
-        const float4 av = *reinterpret_cast<const float4*>(&B.dz1t[n * kAS + ty * 4]);
-        const float aa[4] = {av.x, av.y, av.z, av.w};
-        float bb[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) bb[j] = S.w1[n * kW1S + tx + 16 * j];
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(aa[i], bb[j], acc[i][j]);
-      }
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const int k = tx + 16 * j, rr = ty * 4 + i;
-          B.dz0t[k * kAS + rr] = S.h0t[k * kAS + rr] > 0.f ? acc[i][j] : 0.f;
-        }
-    }
-    __syncthreads();
-    // dW0[n][q] += sum_row dz0[row][n] * x[row][q]  (x = [k0, pe]); db0
-    for (int rr = 0; rr < kTile; ++rr) {
-      const float g = B.dz0t[n0 * kAS + rr];
-#pragma unroll
-      for (int q = 0; q < 24; ++q) {
-        const int qq = qbeg + q;
-        if (qq < qend) {
-          const float xv = qq < a.c0 ? S.x[rr * kMaxC0 + qq] : B.pe[rr * kMaxPe + qq - a.c0];
-          aw0[q] = fmaf(g, xv, aw0[q]);
-        }
-      }
-      if (!qh) ab0 += g;
-    }
-    // grad_k0[row][q] = sum_n dz0[row][n] * W0[n][q]
-    for (int e = tid; e < kTile * a.c0; e += blockDim.x) {
-      const int rr = e / a.c0, q = e % a.c0;
-      const int64_t m = row0 + rr;
-      float acc = 0.f;
-      for (int n = 0; n < kW; ++n) acc = fmaf(B.dz0t[n * kAS + rr], S.w0k[n * (kMaxC0 + 1) + q], acc);
-      if (m < M) grad_k0[m * a.c0 + q] = acc;
-    }
-    __syncthreads();
-  }
-  // write this CTA's partials (zeros if it had no tile)
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) pw1[(ty + 16 * i) * kW + tx + 16 * j] = aw1[i][j];
-  for (int q = 0; q < 24; ++q)
-    if (qbeg + q < qend) pw0[n0 * a.din + qbeg + q] = aw0[q];
-  if (!qh) {
-    pb0[n0] = ab0;
-    pb1[n0] = ab1;
-  }
-  for (int e = tid, s = 0; e < 3 * kW; e += blockDim.x, ++s) pw2[e] = aw2[s];
-  if (tid < 3) pb2[tid] = ab2;
 }
 
 // Sum of the per-CTA partials: eight interleaved running sums (partials c,
@@ -493,11 +174,7 @@ int mlp_forward_impl(pvdb_march_s* m, const MlpArgs& a, const float* k0rows,
                                m->w.r_ray, pe, kMaxPe, m->w.totals, m->slots, rgb, 0,
                                &m->mlp_packed, &m->mlp_packed_cap, &m->mlp_xt, &m->mlp_xt_cap,
                                m->w.totals + 3, st, prepared ? 1 : 0, x_ready ? 1 : 0);
-  PVDB_SMEM_ATTR(k_mlp_fwd_f32, int(sizeof(MlpSmem)));
-  launch_k(k_mlp_fwd_f32, mlp_grid(), kMlpThreads, sizeof(MlpSmem), st, a, k0rows, m->w.r_ray, hpe,
-           m->w.totals, rgb, 0);
-  PVDB_CHECK_LAUNCH("k_mlp_fwd_f32");
-  return PVDB_OK;
+  return mlp_f32_forward(a, k0rows, m->w.r_ray, hpe, m->w.totals, rgb, 0, st);
 }
 
 // Rows from any producer (the merged renderer): k0rows [M, c0], ray [M] ->
@@ -534,11 +211,7 @@ int mlp_forward_rows(const MlpArgs& a, const float* k0rows, const int32_t* ray,
     return mlp_tc_forward_rows(a.w0, a.b0, a.w1, a.b1, a.w2, a.b2, a.c0, a.dpe, k0rows, ray, pe,
                                kMaxPe, totals, max_rows, out, out_logits, blob, blob_cap, xt,
                                xt_cap, err, st, 0, 0);
-  PVDB_SMEM_ATTR(k_mlp_fwd_f32, int(sizeof(MlpSmem)));
-  launch_k(k_mlp_fwd_f32, mlp_grid(), kMlpThreads, sizeof(MlpSmem), st, a, k0rows, ray, hpe, totals,
-           out, out_logits);
-  PVDB_CHECK_LAUNCH("k_mlp_fwd_f32(rows)");
-  return PVDB_OK;
+  return mlp_f32_forward(a, k0rows, ray, hpe, totals, out, out_logits, st);
 }
 
 int mlp_tc_backward_rows(const float* w0, const float* b0, const float* w1, const float* b1,
@@ -574,10 +247,9 @@ int mlp_backward_impl(pvdb_march_s* m, const MlpArgs& a, const float* k0rows, co
     PVDB_CHECK_LAUNCH("k_wgrad_reduce");
     return PVDB_OK;
   }
-  PVDB_SMEM_ATTR(k_mlp_bwd_f32, int(sizeof(MlpBwdSmem)));
-  launch_k(k_mlp_bwd_f32, G, kMlpThreads, sizeof(MlpBwdSmem), st, a, k0rows, m->w.r_ray, m->hpe,
-           m->hpe + size_t(m->max_rays) * kW, m->w.totals, rgb, grad_rgb, grad_k0, m->wpart);
-  PVDB_CHECK_LAUNCH("k_mlp_bwd_f32");
+  rc = mlp_f32_backward(a, k0rows, m->w.r_ray, m->hpe, m->hpe + size_t(m->max_rays) * kW,
+                        m->w.totals, rgb, grad_rgb, grad_k0, m->wpart, G, st);
+  if (rc) return rc;
   launch_k(k_wgrad_reduce, ceil_div(P, 32), 256, 0, st, m->wpart, G, P, grad_flat);
   PVDB_CHECK_LAUNCH("k_wgrad_reduce");
   return PVDB_OK;

@@ -1,0 +1,32 @@
+// The FP32 rgbnet kernels (mlp_f32.cu) as the rgbnet dispatch (mlp.cu) calls them.
+#pragma once
+#include "pvdb_internal.cuh"
+
+namespace pvdb {
+
+struct MlpArgs {
+  const float* w0; const float* b0;
+  const float* w1; const float* b1;
+  const float* w2; const float* b2;
+  int c0, dpe, din;  // din = c0 + dpe
+};
+
+// Flat parameter layout shared with the train step and the Python side:
+// [w0 (128 x din), b0 (128), w1 (128 x 128), b1 (128), w2 (3 x 128), b2 (3)].
+__host__ __device__ inline int64_t mlp_param_count(int din) {
+  return int64_t(128) * din + 128 + 128 * 128 + 128 + 3 * 128 + 3;
+}
+
+// rows: k0 [M, c0], ray [M], M = totals[1]; hpe [rays, 128]: the per-ray part
+// of layer 0; out [M, 3]: logits or their sigmoid.
+int mlp_f32_forward(const MlpArgs& a, const float* k0, const int32_t* ray, const float* hpe,
+                    const uint32_t* totals, float* out, int out_logits, cudaStream_t st);
+
+// grad_k0 [M, c0] and per-CTA partial weight gradients wpart [grid][param count]
+// in the flat layout; pe [rays, 32]: the per-ray PE.
+int mlp_f32_backward(const MlpArgs& a, const float* k0, const int32_t* ray, const float* hpe,
+                     const float* pe, const uint32_t* totals, const float* rgb,
+                     const float* grad_rgb, float* grad_k0, float* wpart, int grid,
+                     cudaStream_t st);
+
+}  // namespace pvdb
