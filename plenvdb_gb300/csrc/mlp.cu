@@ -22,23 +22,34 @@ constexpr int kMaxPe = 32;  // PE dims
 // PE of a unit view direction (dvgo.py:354-355): [d, sin(d*2^i), cos(d*2^i)]
 // with the frequencies innermost per axis: sin at 3 + a*npe + i, cos at
 // 3 + 3*npe + a*npe + i.
-// Per ray: pe[r][0:dpe] and hpe[r][n] = b0[n] + sum_q w0[n][c0+q] * pe[r][q].
-// A 128-thread block takes kPeRays rays: the PE part of W0 is staged
-// transposed in shared memory (coalesced), each PE component is evaluated
-// once, then thread n forms hpe[r][n] for the block's rays.
-constexpr int kPeRays = 32;
+// Per ray: pe[r][0:dpe] and (HPE) hpe[r][n] = b0[n] + sum_q w0[n][c0+q] * pe[r][q].
+// A 128-thread block takes kPeRays rays, without those whose entry of `need`
+// (NULL: all rays) is zero: each PE component is evaluated once, then thread n
+// forms hpe[r][n] with its PE weights in registers, four rays at a time (the
+// sums are chains of dependent FMAs; 16 rays a block keep a small batch spread
+// over the SMs).
+constexpr int kPeRays = 16;
+template <bool HPE>
 __global__ void __launch_bounds__(128)
     k_pe_hpe(const float* __restrict__ viewdirs, int R, int npe, MlpArgs a, float* pe_out,
-             float* hpe) {
-  grid_dep_sync();  // hpe == NULL: the PE only
-  __shared__ float wt[kMaxPe][kW];       // wt[q][n] = w0[n][c0+q]
-  __shared__ float pe_s[kPeRays][kMaxPe];
+             float* hpe, const uint32_t* __restrict__ need) {
+  grid_dep_sync();
+  __shared__ __align__(16) float pe_s[kPeRays][kMaxPe];
+  __shared__ int list[kPeRays];
+  __shared__ int count;
   const int n = threadIdx.x;
   const int r0 = blockIdx.x * kPeRays;
-  for (int q = 0; q < a.dpe; ++q) wt[q][n] = a.w0[n * a.din + a.c0 + q];
-  for (int e = n; e < kPeRays * a.dpe; e += kW) {
-    const int rr = e / a.dpe, q = e % a.dpe, r = r0 + rr;
-    if (r >= R) continue;
+  if (n < 32) {
+    const bool take = n < kPeRays && r0 + n < R && (!need || __ldg(need + r0 + n) != 0);
+    const unsigned m = __ballot_sync(0xffffffffu, take);
+    if (take) list[__popc(m & lanemask_lt())] = r0 + n;
+    if (n == 0) count = __popc(m);
+  }
+  for (int e = n; e < kPeRays * kMaxPe; e += kW) (&pe_s[0][0])[e] = 0.f;
+  __syncthreads();
+  const int nr = count;
+  for (int e = n; e < nr * a.dpe; e += kW) {
+    const int rr = e / a.dpe, q = e - rr * a.dpe, r = list[rr];
     float v;
     if (q < 3) {
       v = viewdirs[r * 3 + q];
@@ -51,14 +62,41 @@ __global__ void __launch_bounds__(128)
     pe_s[rr][q] = v;
     pe_out[int64_t(r) * kMaxPe + q] = v;
   }
-  __syncthreads();
-  if (!hpe) return;
+  if (!HPE) return;
+  float w[kMaxPe];
+#pragma unroll
+  for (int q = 0; q < kMaxPe; ++q) w[q] = q < a.dpe ? __ldg(a.w0 + n * a.din + a.c0 + q) : 0.f;
   const float b = a.b0[n];
-  for (int rr = 0; rr < kPeRays && r0 + rr < R; ++rr) {
-    float s = 0.f;
-    for (int q = 0; q < a.dpe; ++q) s = fmaf(wt[q][n], pe_s[rr][q], s);
-    hpe[int64_t(r0 + rr) * kW + n] = b + s;
+  __syncthreads();
+  for (int rr = 0; rr < nr; rr += 4) {
+    float s[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int q = 0; q < kMaxPe; q += 4) {
+      if (q >= a.dpe) break;  // (the padding columns are zero)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float4 p = *reinterpret_cast<const float4*>(&pe_s[rr + i][q]);
+        s[i] = fmaf(w[q], p.x, s[i]);
+        s[i] = fmaf(w[q + 1], p.y, s[i]);
+        s[i] = fmaf(w[q + 2], p.z, s[i]);
+        s[i] = fmaf(w[q + 3], p.w, s[i]);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (rr + i < nr) hpe[int64_t(list[rr + i]) * kW + n] = b + s[i];
   }
+}
+
+static int pe_launch(const float* viewdirs, int R, const MlpArgs& a, float* pe, float* hpe,
+                     const uint32_t* need, cudaStream_t st) {
+  const int npe = (a.dpe - 3) / 6;
+  if (hpe)
+    launch_k(k_pe_hpe<true>, ceil_div(R, kPeRays), kW, 0, st, viewdirs, R, npe, a, pe, hpe, need);
+  else
+    launch_k(k_pe_hpe<false>, ceil_div(R, kPeRays), kW, 0, st, viewdirs, R, npe, a, pe, hpe, need);
+  PVDB_CHECK_LAUNCH("k_pe_hpe");
+  return PVDB_OK;
 }
 
 // Sum of the per-CTA partials: eight interleaved running sums (partials c,
@@ -134,9 +172,7 @@ int mlp_prepare(pvdb_march_s* m, const MlpArgs& a, const float* viewdirs, int R,
   int rc = mlp_reserve(m, a.din);
   if (rc) return rc;
   float* pe = m->hpe + size_t(m->max_rays) * kW;
-  launch_k(k_pe_hpe, ceil_div(R, kPeRays), kW, 0, st, viewdirs, R, (a.dpe - 3) / 6, a, pe,
-           precision == 1 ? nullptr : m->hpe);
-  PVDB_CHECK_LAUNCH("k_pe_hpe");
+  if ((rc = pe_launch(viewdirs, R, a, pe, precision == 1 ? nullptr : m->hpe, nullptr, st))) return rc;
   if (precision == 1)
     return mlp_tc_pack(a.w0, a.b0, a.w1, a.b1, a.w2, a.b2, a.c0, a.dpe, &m->mlp_packed,
                        &m->mlp_packed_cap, st);
@@ -165,10 +201,8 @@ int mlp_forward_impl(pvdb_march_s* m, const MlpArgs& a, const float* k0rows,
   if (rc) return rc;
   float* hpe = m->hpe;
   float* pe = m->hpe + size_t(m->max_rays) * kW;
-  if (!prepared) {
-    launch_k(k_pe_hpe, ceil_div(R, kPeRays), kW, 0, st, viewdirs, R, (a.dpe - 3) / 6, a, pe, hpe);
-    PVDB_CHECK_LAUNCH("k_pe_hpe");
-  }
+  if (!prepared && (rc = pe_launch(viewdirs, R, a, pe, precision == 1 ? nullptr : hpe, nullptr, st)))
+    return rc;
   if (precision == 1)
     return mlp_tc_forward_rows(a.w0, a.b0, a.w1, a.b1, a.w2, a.b2, a.c0, a.dpe, k0rows,
                                m->w.r_ray, pe, kMaxPe, m->w.totals, m->slots, rgb, 0,
@@ -177,41 +211,23 @@ int mlp_forward_impl(pvdb_march_s* m, const MlpArgs& a, const float* k0rows,
   return mlp_f32_forward(a, k0rows, m->w.r_ray, hpe, m->w.totals, rgb, 0, st);
 }
 
-// Rows from any producer (the merged renderer): k0rows [M, c0], ray [M] ->
-// viewdirs [R,3]; M = totals[1]. hpe_buf holds R*(128+32) floats.
-// The per-ray PE alone into hpe_buf + R * 128 (stride kMaxPe floats): the
-// input of rgbnet X tiles that a caller builds itself.
-int mlp_pe_rows(const MlpArgs& a, const float* viewdirs, int R, float* hpe_buf, int* pe_stride,
-                cudaStream_t st) {
-  *pe_stride = kMaxPe;
-  if (R <= 0) return PVDB_OK;
-  launch_k(k_pe_hpe, ceil_div(R, kPeRays), kW, 0, st, viewdirs, R, (a.dpe - 3) / 6, a,
-           hpe_buf + size_t(R) * kW, nullptr);
-  PVDB_CHECK_LAUNCH("k_pe_hpe");
-  return PVDB_OK;
-}
-
-// x_ready (BF16 only): the X tiles in *xt are already built from the rows and
-// the PE (mlp_pe_rows), so neither is recomputed here.
+// Rows from the merged renderer; M = totals[1]. FP32: k0rows [M, c0], ray [M]
+// -> viewdirs [R,3], hpe_buf holds R*(128+32) floats; the rays whose entry of
+// `need` is zero have no row. BF16: the X tiles in *xt are already built.
 int mlp_forward_rows(const MlpArgs& a, const float* k0rows, const int32_t* ray,
-                     const float* viewdirs, int R, const uint32_t* totals, int64_t max_rows,
-                     float* out, int out_logits, float* hpe_buf, int precision, void** blob,
-                     size_t* blob_cap, void** xt, size_t* xt_cap, uint32_t* err,
-                     cudaStream_t st, int x_ready) {
+                     const float* viewdirs, int R, const uint32_t* need, const uint32_t* totals,
+                     int64_t max_rows, float* out, int out_logits, float* hpe_buf, int precision,
+                     void** blob, size_t* blob_cap, void** xt, size_t* xt_cap, uint32_t* err,
+                     cudaStream_t st) {
   if (R <= 0) return PVDB_OK;
-  float* hpe = hpe_buf;
-  float* pe = hpe_buf + size_t(R) * kW;
-  if (precision == 1 && x_ready)
-    return mlp_tc_forward_rows(a.w0, a.b0, a.w1, a.b1, a.w2, a.b2, a.c0, a.dpe, k0rows, ray, pe,
-                               kMaxPe, totals, max_rows, out, out_logits, blob, blob_cap, xt,
-                               xt_cap, err, st, 0, 1);
-  launch_k(k_pe_hpe, ceil_div(R, kPeRays), kW, 0, st, viewdirs, R, (a.dpe - 3) / 6, a, pe, hpe);
-  PVDB_CHECK_LAUNCH("k_pe_hpe");
   if (precision == 1)
-    return mlp_tc_forward_rows(a.w0, a.b0, a.w1, a.b1, a.w2, a.b2, a.c0, a.dpe, k0rows, ray, pe,
-                               kMaxPe, totals, max_rows, out, out_logits, blob, blob_cap, xt,
-                               xt_cap, err, st, 0, 0);
-  return mlp_f32_forward(a, k0rows, ray, hpe, totals, out, out_logits, st);
+    return mlp_tc_forward_rows(a.w0, a.b0, a.w1, a.b1, a.w2, a.b2, a.c0, a.dpe, k0rows, ray,
+                               nullptr, kMaxPe, totals, max_rows, out, out_logits, blob, blob_cap,
+                               xt, xt_cap, err, st, 0, 1);
+  float* pe = hpe_buf + size_t(R) * kW;
+  const int rc = pe_launch(viewdirs, R, a, pe, hpe_buf, need, st);
+  if (rc) return rc;
+  return mlp_f32_forward(a, k0rows, ray, hpe_buf, totals, out, out_logits, st);
 }
 
 int mlp_tc_backward_rows(const float* w0, const float* b0, const float* w1, const float* b1,
@@ -303,9 +319,10 @@ int pvdb_mlp_backward(pvdb_march m, const pvdb_mlp_weights* w, const float* k0,
   // backward does not rely on a preceding forward call of the same weights.
   rc = mlp_reserve(m, a.din);
   if (rc) return rc;
-  launch_k(k_pe_hpe, ceil_div(m->n_rays, kPeRays), kW, 0, st, viewdirs, m->n_rays, (a.dpe - 3) / 6,
-           a, m->hpe + size_t(m->max_rays) * kW, m->hpe);
-  PVDB_CHECK_LAUNCH("k_pe_hpe");
+  if (m->n_rays > 0 &&
+      (rc = pe_launch(viewdirs, m->n_rays, a, m->hpe + size_t(m->max_rays) * kW,
+                      precision == 1 ? nullptr : m->hpe, nullptr, as_stream(s))))
+    return rc;
   const int64_t P = mlp_param_count(a.din);
   float* flat = m->wpart + int64_t(mlp_grid()) * P;  // spare slot after the partials
   rc = mlp_backward_impl(m, a, k0 ? k0 : m->w.r_k0, rgb, grad_rgb, grad_k0, flat, precision, st,

@@ -2,7 +2,10 @@
 //
 // Data: an index leaf store (voxel -> row id, 0 = empty; the voxels with a row
 // are the active ones) plus per-row density and k0 features (FP32, or BF16
-// features with FP32 density).
+// features with FP32 density). Loading lays the density out per voxel of the
+// allocated leaves, and 12-channel features too, with one more record that
+// holds row 0 (every voxel outside the leaves): a trilinear corner is then one
+// load at its slot, not a row id and a load behind it.
 //
 // Per frame:
 //   k_render_march<COUNT>  one thread per pixel: get_rays (renderer.cu:122-167)
@@ -13,8 +16,11 @@
 //                          early stop at a colour sample once T < t_stop
 //                          (renderer.cu:240-266); counts colour samples
 //   device scan            per-pixel row offsets
-//   k_render_march<FILL>   the same march, writing each colour sample's k0 row
-//                          (renderer.cu:303-310) and weight
+//   k_render_march<FILL>   the same march, writing each colour sample's
+//                          distance, weight and pixel to its row
+//   k_render_pe / k_render_x (BF16), k_render_k0 (FP32)
+//                          per row: the trilinear features (renderer.cu:303-310)
+//                          into the rgbnet's X tiles or k0 rows
 //   rgbnet                 the MLP on all rows (PE part once per pixel)
 //   k_render_composite     per pixel: T*bg + sum_rows w/(1+exp(-logit)) in
 //                          sample order (final_render renderer.cu:112-119,
@@ -23,6 +29,7 @@
 // The reference runs the march twice with slightly different float
 // associations in the two passes; here both passes share one code path, so the
 // fill pass reproduces the count pass exactly.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -39,12 +46,10 @@ struct MlpArgs {
   int c0, dpe, din;
 };
 int mlp_forward_rows(const MlpArgs& a, const float* k0rows, const int32_t* ray,
-                     const float* viewdirs, int R, const uint32_t* totals, int64_t max_rows,
-                     float* out, int out_logits, float* hpe_buf, int precision, void** blob,
-                     size_t* blob_cap, void** xt, size_t* xt_cap, uint32_t* err,
-                     cudaStream_t st, int x_ready);
-int mlp_pe_rows(const MlpArgs& a, const float* viewdirs, int R, float* hpe_buf, int* pe_stride,
-                cudaStream_t st);
+                     const float* viewdirs, int R, const uint32_t* need, const uint32_t* totals,
+                     int64_t max_rows, float* out, int out_logits, float* hpe_buf, int precision,
+                     void** blob, size_t* blob_cap, void** xt, size_t* xt_cap, uint32_t* err,
+                     cudaStream_t st);
 
 struct RenderP {
   int H, W, inverse_y;
@@ -54,12 +59,16 @@ struct RenderP {
   float wsm1[3];
   float near_, far_, stepdist, shift, interval, thr, bg, t_stop;
   int dcol;
-  // index store
-  GridView idx;            // topology; values unused
-  const int32_t* rows;     // [nleaf*512] row id of every in-leaf voxel
-  const float* den;        // [N]
-  const float* col;        // [N*dcol] (storage 0)
-  const __nv_bfloat16* colh;  // [N*dcol] (storage 1)
+  // index store: nslots = nleaf * 512 voxel slots; record nslots of the
+  // per-voxel arrays holds row 0
+  GridView idx;               // topology; values unused
+  int64_t nslots;
+  const float* vden;          // [nslots + 1]
+  const float* vcol;          // [nslots + 1][12] (12 channels, storage 0)
+  const __nv_bfloat16* vcolh; // [nslots + 1][kHalfStride] (12 channels, storage 1)
+  const int32_t* rows;        // [nslots] row id of every in-leaf voxel (other channel counts)
+  const float* col;           // [N*dcol] (other channel counts, storage 0)
+  const __nv_bfloat16* colh;  // [N*dcol] (other channel counts, storage 1)
   int storage;
 };
 
@@ -67,146 +76,20 @@ struct RenderW {
   uint32_t* n;       // [HW] colour samples per pixel
   uint32_t* off;     // [HW]
   float* T;          // [HW]
-  float* viewdirs;   // [HW*3]
+  float* viewdirs;   // [HW*3] (pixels with colour samples)
   float* rk0;        // [cap*dcol]
   float* rw;         // [cap]
+  float* rt;         // [cap] distance along the pixel's ray
   int32_t* rpix;     // [cap]
-  uint32_t* totals;  // [0] unused, [1] total rows
   int64_t cap;
-  // BF16 rgbnet: the fill pass writes each colour sample's rgbnet input row
-  // ([k0 | PE | 1 | 0], BF16) into the X tiles instead of the FP32 k0 row
-  uint8_t* xt;       // [ceil(cap/128)] tiles, or NULL
-  const float* pe;   // [HW][pe_stride] per-pixel PE
-  int pe_stride, dpe;
 };
 
-__device__ __forceinline__ int32_t row_at(const RenderP& P, int i, int j, int k) {
-  const int s = slot_of(P.idx, i, j, k);
-  return s < 0 ? 0 : __ldg(P.rows + s);
-}
-
-__device__ __forceinline__ bool index_active(const RenderP& P, int i, int j, int k) {
-  const int l = leaf_of(P.idx, i, j, k);
-  if (l < 0) return false;
-  const int v = vox_offset(i, j, k);
-  return (__ldg(P.idx.mask + l * 8 + (v >> 6)) >> (v & 63)) & 1ull;
-}
-
-// 12-channel rows (the reference's k0): three float4, or three 8-byte BF16
-// quads per corner.
-__device__ __forceinline__ void fill_features12(const RenderP& P, const int32_t id[8],
-                                                const float sc[8], float acc[12]) {
-#pragma unroll
-  for (int c = 0; c < 8; ++c) {
-    float v[12];
-    if (P.storage == 0) {
-      const float4* src = reinterpret_cast<const float4*>(P.col + int64_t(id[c]) * 12);
-#pragma unroll
-      for (int b = 0; b < 3; ++b) {
-        const float4 f = __ldg(src + b);
-        v[4 * b] = f.x; v[4 * b + 1] = f.y; v[4 * b + 2] = f.z; v[4 * b + 3] = f.w;
-      }
-    } else {
-      const uint2* src = reinterpret_cast<const uint2*>(P.colh + int64_t(id[c]) * 12);
-#pragma unroll
-      for (int b = 0; b < 3; ++b) {
-        const uint2 h = __ldg(src + b);
-        v[4 * b] = __uint_as_float(h.x << 16);
-        v[4 * b + 1] = __uint_as_float(h.x & 0xFFFF0000u);
-        v[4 * b + 2] = __uint_as_float(h.y << 16);
-        v[4 * b + 3] = __uint_as_float(h.y & 0xFFFF0000u);
-      }
-    }
-#pragma unroll
-    for (int q = 0; q < 12; ++q)
-      acc[q] = c == 0 ? __fmul_rn(v[q], sc[0]) : __fmaf_rn(v[q], sc[c], acc[q]);
-  }
-}
-
-// Trilinear features of a colour sample (trigetColor, renderer.cu:303-310):
-// per channel c0*s0, then the fma chain over corners 1..7. 12-channel rows are
-// read with vector loads (three float4, or three 8-byte BF16 quads).
-__device__ __forceinline__ void fill_features(const RenderP& P, const int32_t id[8],
-                                              const float sc[8], float acc[16]) {
-  if (P.dcol == 12) {
-    fill_features12(P, id, sc, acc);
-    return;
-  }
-  for (int q = 0; q < P.dcol; ++q) {
-    float a;
-    if (P.storage == 0) {
-      a = __fmul_rn(__ldg(P.col + int64_t(id[0]) * P.dcol + q), sc[0]);
-      for (int c = 1; c < 8; ++c) a = __fmaf_rn(__ldg(P.col + int64_t(id[c]) * P.dcol + q), sc[c], a);
-    } else {
-      a = __fmul_rn(__bfloat162float(P.colh[int64_t(id[0]) * P.dcol + q]), sc[0]);
-      for (int c = 1; c < 8; ++c)
-        a = __fmaf_rn(__bfloat162float(P.colh[int64_t(id[c]) * P.dcol + q]), sc[c], a);
-    }
-    acc[q] = a;
-  }
-}
-
-// 12 k0 channels and 27 PE values (the rgbnet of the reference): the row is
-// 2 k0 chunks, the first of which carries PE 0..3, then pixel-constant chunks.
-__device__ __forceinline__ void write_x_row12(const RenderW& Wk, int64_t m, const float* k0v,
-                                              const uint4* pe_chunks) {
-  uint8_t* tile = Wk.xt + (m >> 7) * int64_t(kRgbXTile);
-  const int row = int(m & 127);
-  const uint4 c0 = make_uint4(tc::pack_bf16(k0v[0], k0v[1]), tc::pack_bf16(k0v[2], k0v[3]),
-                              tc::pack_bf16(k0v[4], k0v[5]), tc::pack_bf16(k0v[6], k0v[7]));
-  const uint4 c1 = make_uint4(tc::pack_bf16(k0v[8], k0v[9]), tc::pack_bf16(k0v[10], k0v[11]),
-                              pe_chunks[0].z, pe_chunks[0].w);
-  *reinterpret_cast<uint4*>(tile + tc::kmaj(row, 0, kRgbXK)) = c0;
-  *reinterpret_cast<uint4*>(tile + tc::kmaj(row, 8, kRgbXK)) = c1;
-#pragma unroll
-  for (int cb = 2; cb < 6; ++cb)
-    *reinterpret_cast<uint4*>(tile + tc::kmaj(row, 8 * cb, kRgbXK)) = pe_chunks[cb - 1];
-}
-
-// The BF16 X row m of pixel n: [k0 (dcol) | PE (dpe) | 1 | 0 ...] in the
-// canonical K-major tile layout; pe_bits holds the pixel's PE as BF16 pairs.
-__device__ __forceinline__ void write_x_row(const RenderW& Wk, int64_t m, int n,
-                                            const float* k0v, int dcol, const uint32_t* pe_bits) {
-  uint8_t* tile = Wk.xt + (m >> 7) * int64_t(kRgbXTile);
-  const int row = int(m & 127);
-  const int din = dcol + Wk.dpe;
-#pragma unroll
-  for (int cb = 0; cb < kRgbXK / 8; ++cb) {
-    uint32_t w4[4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      float v2[2];
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int q = 8 * cb + 2 * e + h;
-        v2[h] = q < dcol ? k0v[q < 16 ? q : 15] : q == din ? 1.f : 0.f;
-      }
-      uint32_t bits = tc::pack_bf16(v2[0], v2[1]);
-      // PE columns come pre-rounded from pe_bits
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int q = 8 * cb + 2 * e + h;
-        if (q >= dcol && q < din) {
-          const int pq = q - dcol;
-          const uint32_t pb = (pe_bits[pq >> 1] >> (16 * (pq & 1))) & 0xFFFFu;
-          bits = h == 0 ? ((bits & 0xFFFF0000u) | pb) : ((bits & 0x0000FFFFu) | (pb << 16));
-        }
-      }
-      w4[e] = bits;
-    }
-    *reinterpret_cast<uint4*>(tile + tc::kmaj(row, 8 * cb, kRgbXK)) =
-        make_uint4(w4[0], w4[1], w4[2], w4[3]);
-  }
-  (void)n;
-}
-
-template <bool FILL>
-__global__ void __launch_bounds__(128)
-    k_render_march(RenderP P, RenderW Wk) {
-  const int HW = P.H * P.W;
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= HW) return;
-  // get_rays (renderer.cu:134-151)
+// The ray of pixel n (get_rays, renderer.cu:134-151) in the unit-cube frame.
+struct PixelRay {
+  float rd[3], len, steplen;
+  float o[3], d[3];
+};
+__device__ __forceinline__ void pixel_ray(const RenderP& P, int n, PixelRay& r) {
   const float pi = float(n % P.W) + 0.5f, pj = float(n / P.W) + 0.5f;
   float dir[3];
   dir[0] = __fdiv_rn(pi - P.K[2], P.K[0]);
@@ -217,111 +100,118 @@ __global__ void __launch_bounds__(128)
     dir[1] = -__fdiv_rn(pj - P.K[5], P.K[4]);
     dir[2] = -1.f;
   }
-  float rd[3];
   for (int a = 0; a < 3; ++a)
-    rd[a] = __fmaf_rn(dir[2], P.c2w[4 * a + 2], __fmaf_rn(dir[1], P.c2w[4 * a + 1],
-                                                          __fmul_rn(dir[0], P.c2w[4 * a])));
-  const float len = sqrtf(__fmaf_rn(rd[2], rd[2], __fmaf_rn(rd[1], rd[1], __fmul_rn(rd[0], rd[0]))));
-  const float steplen = __fdiv_rn(P.stepdist, len);
-  float o[3], d[3];
+    r.rd[a] = __fmaf_rn(dir[2], P.c2w[4 * a + 2], __fmaf_rn(dir[1], P.c2w[4 * a + 1],
+                                                            __fmul_rn(dir[0], P.c2w[4 * a])));
+  r.len = sqrtf(__fmaf_rn(r.rd[2], r.rd[2],
+                          __fmaf_rn(r.rd[1], r.rd[1], __fmul_rn(r.rd[0], r.rd[0]))));
+  r.steplen = __fdiv_rn(P.stepdist, r.len);
   for (int a = 0; a < 3; ++a) {
     const float ext = P.mx[a] - P.mn[a];
-    o[a] = __fdiv_rn(P.c2w[4 * a + 3] - P.mn[a], ext);
-    d[a] = __fdiv_rn(rd[a], ext);
+    r.o[a] = __fdiv_rn(P.c2w[4 * a + 3] - P.mn[a], ext);
+    r.d[a] = __fdiv_rn(r.rd[a], ext);
   }
-  if (!FILL) {
-    for (int a = 0; a < 3; ++a) Wk.viewdirs[n * 3 + a] = __fdiv_rn(rd[a], len);
+}
+
+// Slots of the 8 corners of the sample's cell (int() truncation,
+// renderer.cu:271-300), P.nslots where a corner lies in no allocated leaf, and
+// their scales.
+__device__ __forceinline__ void cell_corners(const RenderP& P, const float xyz[3], int64_t s[8],
+                                             float sc[8]) {
+  const int i = int(xyz[0]), j = int(xyz[1]), k = int(xyz[2]);
+  int s8[8];
+  corner_slots(P.idx, i, j, k, s8);
+#pragma unroll
+  for (int c = 0; c < 8; ++c) s[c] = s8[c] < 0 ? P.nslots : int64_t(s8[c]);
+  corner_scales(xyz[0] - float(i), xyz[1] - float(j), xyz[2] - float(k), sc);
+}
+
+// One thread per pixel, 8 x 4 pixels a warp. Bound by instructions: most steps
+// of a ray lie in blocks of 8^3 voxels that no leaf covers, where every sample
+// is inactive. There the march only advances t (the same rounded additions, so
+// the later samples' positions are the same bits) until shortly before the
+// block's face, instead of testing each step: see the skip below.
+template <bool FILL>
+__global__ void __launch_bounds__(128)
+    k_render_march(RenderP P, RenderW Wk) {
+  const int warp = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int tiles_x = (P.W + 7) / 8;
+  const int px = (warp % tiles_x) * 8 + (lane & 7), py = (warp / tiles_x) * 4 + (lane >> 3);
+  if (px >= P.W || py >= P.H) return;
+  const int n = py * P.W + px;
+  uint32_t want = 0;
+  if (FILL) {
+    want = Wk.n[n];
+    if (want == 0) return;
   }
+  PixelRay r;
+  pixel_ray(P, n, r);
+  const float steplen = r.steplen;
   // get_tminmax against the unit cube (renderer.cu:50-64)
-  const float vx = d[0] == 0.f ? float(1e-6) : d[0];
-  const float vy = d[1] == 0.f ? float(1e-6) : d[1];
-  const float vz = d[2] == 0.f ? float(1e-6) : d[2];
-  const float ax = __fdiv_rn(1.f - o[0], vx), ay = __fdiv_rn(1.f - o[1], vy), az = __fdiv_rn(1.f - o[2], vz);
-  const float bx = __fdiv_rn(-o[0], vx), by = __fdiv_rn(-o[1], vy), bz = __fdiv_rn(-o[2], vz);
+  const float vx = r.d[0] == 0.f ? float(1e-6) : r.d[0];
+  const float vy = r.d[1] == 0.f ? float(1e-6) : r.d[1];
+  const float vz = r.d[2] == 0.f ? float(1e-6) : r.d[2];
+  const float ax = __fdiv_rn(1.f - r.o[0], vx), ay = __fdiv_rn(1.f - r.o[1], vy),
+              az = __fdiv_rn(1.f - r.o[2], vz);
+  const float bx = __fdiv_rn(-r.o[0], vx), by = __fdiv_rn(-r.o[1], vy),
+              bz = __fdiv_rn(-r.o[2], vz);
   const float tmin = fmaxf(fminf(fmaxf(fmaxf(fminf(ax, bx), fminf(ay, by)), fminf(az, bz)), P.far_), P.near_);
   const float tmax = fmaxf(fminf(fminf(fminf(fmaxf(ax, bx), fmaxf(ay, by)), fmaxf(az, bz)), P.far_), P.near_);
   float T = 1.f;
   uint32_t cnt = 0;
   const int64_t base = FILL ? int64_t(Wk.off[n]) : 0;
-  // BF16 fill: the pixel's PE, rounded to BF16 once — for 12 k0 channels and
-  // 27 PE values as the pixel-constant part of its X rows (pe_chunks[0].zw =
-  // PE 0..3, pe_chunks[1..4] = columns 16..47), else as BF16 pairs
-  const bool fast12 = FILL && Wk.xt && P.dcol == 12 && Wk.dpe == 27;
-  uint4 pe_chunks[5];
-  uint32_t pe_bits[16];
-  if (fast12) {
-    const float* pp = Wk.pe + int64_t(n) * Wk.pe_stride;
-    float pv[27];
-#pragma unroll
-    for (int q = 0; q < 27; ++q) pv[q] = pp[q];
-    pe_chunks[0] = make_uint4(0u, 0u, tc::pack_bf16(pv[0], pv[1]), tc::pack_bf16(pv[2], pv[3]));
-#pragma unroll
-    for (int cb = 2; cb < 5; ++cb) {  // columns 8cb .. 8cb+7 = PE 8cb-12 ..
-      uint32_t w4[4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int p0 = 8 * cb - 12 + 2 * e, p1 = p0 + 1;
-        const float a0 = p0 < 27 ? pv[p0 < 27 ? p0 : 0] : (p0 == 27 ? 1.f : 0.f);
-        const float a1 = p1 < 27 ? pv[p1 < 27 ? p1 : 0] : (p1 == 27 ? 1.f : 0.f);
-        w4[e] = tc::pack_bf16(a0, a1);
-      }
-      pe_chunks[cb - 1] = make_uint4(w4[0], w4[1], w4[2], w4[3]);
-    }
-    pe_chunks[4] = make_uint4(0u, 0u, 0u, 0u);
-  } else if (FILL && Wk.xt) {
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      const int q0 = 2 * i, q1 = 2 * i + 1;
-      const float a0 = q0 < Wk.dpe ? Wk.pe[int64_t(n) * Wk.pe_stride + q0] : 0.f;
-      const float a1 = q1 < Wk.dpe ? Wk.pe[int64_t(n) * Wk.pe_stride + q1] : 0.f;
-      pe_bits[i] = tc::pack_bf16(a0, a1);
-    }
-  }
-  if (FILL && Wk.xt) {
-    // the padding rows of the last tile are zero (block 0 writes them)
-    if (blockIdx.x == 0) {
-      const int64_t M = Wk.totals[1], Mpad = (M + 127) / 128 * 128;
-      const int64_t mz = M + threadIdx.x;
-      if (mz < Mpad) {  // Mpad <= the tiles reserved for cap rows
-        uint8_t* tile = Wk.xt + (mz >> 7) * int64_t(kRgbXTile);
-        for (int cb = 0; cb < kRgbXK / 8; ++cb)
-          *reinterpret_cast<uint4*>(tile + tc::kmaj(int(mz & 127), 8 * cb, kRgbXK)) =
-              make_uint4(0u, 0u, 0u, 0u);
-      }
-    }
-  }
   float t = tmin;
   // the reference loops while t < tmax; the iteration bound (the sample count
   // of the [tmin,tmax] chord plus slack) only guards against a step that no
   // longer advances t (non-finite or vanishing steplen)
   const float nsteps_f = (tmax - tmin) / steplen;
   const int max_it = (nsteps_f > 0.f && nsteps_f < 1e6f) ? int(nsteps_f) + 4 : 0;
+  // Skip: voxels advanced per step and its inverse per axis, and the most
+  // steps a skip may take: t's rounding (at most tmax 2^-23 per addition)
+  // stays below a quarter of a step
+  float inv[3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) inv[a] = 1.f / (r.d[a] * P.wsm1[a] * steplen);
+  const float most = fminf(0.25f * steplen / (tmax * 1.2e-7f), 4096.f);
   for (int it = 0; t < tmax && it < max_it; ++it) {
     t = __fadd_rn(t, steplen);
     float p[3];
-    for (int a = 0; a < 3; ++a) p[a] = __fmaf_rn(t, d[a], o[a]);
+    for (int a = 0; a < 3; ++a) p[a] = __fmaf_rn(t, r.d[a], r.o[a]);
     if ((0.f > p[0]) | (0.f > p[1]) | (0.f > p[2]) | (1.f < p[0]) | (1.f < p[1]) | (1.f < p[2]))
       continue;
     float xyz[3];
     for (int a = 0; a < 3; ++a) xyz[a] = __fmul_rn(p[a], P.wsm1[a]);
-    if (!index_active(P, __float2int_rn(xyz[0]), __float2int_rn(xyz[1]), __float2int_rn(xyz[2])))
+    const int ri = __float2int_rn(xyz[0]), rj = __float2int_rn(xyz[1]),
+              rk = __float2int_rn(xyz[2]);
+    const int leaf = leaf_of(P.idx, ri, rj, rk);
+    if (leaf < 0) {
+      // every sample whose rounded position stays in this block is inactive:
+      // the steps that keep it 0.01 voxel (above the rounding of xyz) and one
+      // step inside the faces at 8 b - 0.5 and 8 b + 7.5
+      float steps = most;
+      const int b[3] = {ri & ~7, rj & ~7, rk & ~7};
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        const float face = float(b[a]) + (inv[a] > 0.f ? 7.49f : -0.49f);
+        const float s = (face - xyz[a]) * inv[a];
+        if (s < steps) steps = s;  // (an axis that does not advance gives inf or NaN)
+      }
+      const int skip = int(fmaxf(steps, 0.f)) - 1;
+      for (int q = 0; q < skip; ++q) t = __fadd_rn(t, steplen);
+      it += max(skip, 0);
       continue;
-    // trigetDensity2 (renderer.cu:271-300): int() truncation, scales then sum
-    const int i = int(xyz[0]), j = int(xyz[1]), k = int(xyz[2]);
-    const float u = xyz[0] - float(i), v = xyz[1] - float(j), w = xyz[2] - float(k);
-    int32_t id[8];
-    id[0] = row_at(P, i, j, k);
-    id[1] = row_at(P, i, j, k + 1);
-    id[2] = row_at(P, i, j + 1, k + 1);
-    id[3] = row_at(P, i, j + 1, k);
-    id[4] = row_at(P, i + 1, j + 1, k);
-    id[5] = row_at(P, i + 1, j + 1, k + 1);
-    id[6] = row_at(P, i + 1, j, k + 1);
-    id[7] = row_at(P, i + 1, j, k);
+    }
+    const int v = vox_offset(ri, rj, rk);
+    if (!((__ldg(P.idx.mask + leaf * 8 + (v >> 6)) >> (v & 63)) & 1ull)) continue;
+    int64_t slot[8];
     float sc[8];
-    corner_scales(u, v, w, sc);
-    float sig = __fmul_rn(__ldg(P.den + id[0]), sc[0]);
-    for (int c = 1; c < 8; ++c) sig = __fmaf_rn(__ldg(P.den + id[c]), sc[c], sig);
+    cell_corners(P, xyz, slot, sc);
+    float val[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) val[c] = __ldg(P.vden + slot[c]);
+    float sig = __fmul_rn(val[0], sc[0]);
+#pragma unroll
+    for (int c = 1; c < 8; ++c) sig = __fmaf_rn(val[c], sc[c], sig);
     const float alpha = 1.f - powf(1.f + expf(sig + P.shift), -P.interval);
     if (alpha <= P.thr) continue;
     const float wt = T * alpha;
@@ -330,61 +220,231 @@ __global__ void __launch_bounds__(128)
     if (FILL) {
       const int64_t m = base + cnt;
       if (m < Wk.cap) {
-        if (Wk.xt && fast12) {
-          float acc[12];
-          fill_features12(P, id, sc, acc);
-          write_x_row12(Wk, m, acc, pe_chunks);
-        } else if (Wk.xt) {
-          float acc[16];
-          fill_features(P, id, sc, acc);
-          write_x_row(Wk, m, n, acc, P.dcol, pe_bits);
-        } else if (P.dcol == 12) {
-          float acc[12];
-          fill_features12(P, id, sc, acc);
-          float4* dst = reinterpret_cast<float4*>(Wk.rk0 + m * 12);
-#pragma unroll
-          for (int b = 0; b < 3; ++b)
-            dst[b] = make_float4(acc[4 * b], acc[4 * b + 1], acc[4 * b + 2], acc[4 * b + 3]);
-        } else {
-          float* dst = Wk.rk0 + m * P.dcol;
-          float acc[16];
-          fill_features(P, id, sc, acc);
-          for (int q = 0; q < P.dcol; ++q) dst[q] = acc[q];
-        }
         Wk.rw[m] = wt;
+        Wk.rt[m] = t;
         Wk.rpix[m] = n;
       }
     }
     ++cnt;
+    if (FILL && cnt == want) break;
     if (T < P.t_stop) break;
   }
   if (!FILL) {
     Wk.n[n] = cnt;
     Wk.T[n] = T;
+    if (cnt)
+      for (int a = 0; a < 3; ++a) Wk.viewdirs[n * 3 + a] = __fdiv_rn(r.rd[a], r.len);
   }
 }
 
-__global__ void k_render_composite(RenderP P, RenderW Wk, const float* __restrict__ logits,
-                                   float* image) {
-  const int HW = P.H * P.W;
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= HW) return;
-  const uint32_t cnt = Wk.n[n];
-  if (cnt == 0) {
-    image[n * 3] = image[n * 3 + 1] = image[n * 3 + 2] = P.bg;
+// The trilinear features of row m (trigetColor, renderer.cu:303-310): per
+// channel c0*s0, then the fma chain over corners 1..7, at the position the
+// march had (same arithmetic). CT = 12: vector loads of the per-voxel records;
+// 0: any channel count up to 16, by row id.
+template <int CT>
+__device__ __forceinline__ void row_features(const RenderP& P, const RenderW& Wk, int64_t m,
+                                             int n, float* acc) {
+  PixelRay r;
+  pixel_ray(P, n, r);
+  const float t = Wk.rt[m];
+  float xyz[3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) xyz[a] = __fmul_rn(__fmaf_rn(t, r.d[a], r.o[a]), P.wsm1[a]);
+  int64_t slot[8];
+  float sc[8];
+  cell_corners(P, xyz, slot, sc);
+  if (CT == 12) {
+    if (P.storage == 0) {
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        const float4* src = reinterpret_cast<const float4*>(P.vcol + slot[c] * 12);
+        float v[12];
+#pragma unroll
+        for (int b = 0; b < 3; ++b) *reinterpret_cast<float4*>(v + 4 * b) = __ldg(src + b);
+#pragma unroll
+        for (int q = 0; q < 12; ++q)
+          acc[q] = c == 0 ? __fmul_rn(v[q], sc[0]) : __fmaf_rn(v[q], sc[c], acc[q]);
+      }
+    } else {
+      uint4 lo[8];
+      uint2 hi[8];
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        const uint4* src = reinterpret_cast<const uint4*>(P.vcolh + slot[c] * kHalfStride);
+        lo[c] = __ldg(src);
+        hi[c] = __ldg(reinterpret_cast<const uint2*>(src + 1));
+      }
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        const uint32_t w[6] = {lo[c].x, lo[c].y, lo[c].z, lo[c].w, hi[c].x, hi[c].y};
+#pragma unroll
+        for (int q = 0; q < 12; ++q) {
+          const float v = __uint_as_float(q & 1 ? w[q >> 1] & 0xFFFF0000u : w[q >> 1] << 16);
+          acc[q] = c == 0 ? __fmul_rn(v, sc[0]) : __fmaf_rn(v, sc[c], acc[q]);
+        }
+      }
+    }
     return;
   }
-  const float tb = __fmul_rn(Wk.T[n], P.bg);
-  float acc[3] = {tb, tb, tb};
-  const int64_t off = Wk.off[n];
-  for (uint32_t j = 0; j < cnt; ++j) {
-    const int64_t m = off + j;
-    if (m >= Wk.cap) break;
-    const float w = Wk.rw[m];
-    for (int c = 0; c < 3; ++c)
-      acc[c] = __fadd_rn(acc[c], __fdiv_rn(w, 1.f + expf(-logits[m * 3 + c])));
+  int32_t id[8];
+#pragma unroll
+  for (int c = 0; c < 8; ++c) id[c] = slot[c] == P.nslots ? 0 : __ldg(P.rows + slot[c]);
+#pragma unroll
+  for (int q = 0; q < 16; ++q) {
+    if (q >= P.dcol) break;
+    float a = 0.f;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      const int64_t e = int64_t(id[c]) * P.dcol + q;
+      const float v = P.storage == 0 ? __ldg(P.col + e) : __bfloat162float(P.colh[e]);
+      a = c == 0 ? __fmul_rn(v, sc[0]) : __fmaf_rn(v, sc[c], a);
+    }
+    acc[q] = a;
   }
+}
+
+// FP32 rgbnet: the k0 rows.
+template <int CT>
+__global__ void __launch_bounds__(256)
+    k_render_k0(RenderP P, RenderW Wk, int64_t M) {
+  const int64_t m = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+  if (m >= M) return;
+  float acc[CT ? CT : 16];
+  row_features<CT>(P, Wk, m, Wk.rpix[m], acc);
+  if (CT == 12) {
+    float4* dst = reinterpret_cast<float4*>(Wk.rk0 + m * 12);
+#pragma unroll
+    for (int b = 0; b < 3; ++b)
+      dst[b] = make_float4(acc[4 * b], acc[4 * b + 1], acc[4 * b + 2], acc[4 * b + 3]);
+  } else {
+#pragma unroll
+    for (int q = 0; q < 16; ++q)
+      if (q < P.dcol) Wk.rk0[m * P.dcol + q] = acc[q < (CT ? CT : 16) ? q : 0];
+  }
+}
+
+// BF16 rgbnet: the pixel's part of its X rows ([0 (dcol) | PE | 1 | 0], 48
+// BF16 columns), for the pixels with colour samples; one thread per 8 columns.
+__global__ void __launch_bounds__(192)
+    k_render_pe(RenderP P, RenderW Wk, int npe, uint4* pex) {
+  const int64_t e = blockIdx.x * 192ll + threadIdx.x;
+  const int n = int(e / 6), cb = int(e % 6);
+  if (n >= P.H * P.W || Wk.n[n] == 0) return;
+  const int dpe = 3 + 6 * npe;
+  const float v[3] = {Wk.viewdirs[n * 3], Wk.viewdirs[n * 3 + 1], Wk.viewdirs[n * 3 + 2]};
+  uint32_t w[4];
+#pragma unroll
+  for (int h = 0; h < 4; ++h) {
+    float x2[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int q = 8 * cb + 2 * h + u - P.dcol;  // PE component (dvgo.py:354-355)
+      float x = q == dpe ? 1.f : 0.f;
+      if (q >= 0 && q < 3) {
+        x = q == 0 ? v[0] : q == 1 ? v[1] : v[2];
+      } else if (q >= 3 && q < dpe) {
+        const int qq = q - 3, cs = qq / (3 * npe), rem = qq - cs * 3 * npe, a = rem / npe,
+                  i = rem - a * npe;
+        const float f = (a == 0 ? v[0] : a == 1 ? v[1] : v[2]) * float(1 << i);
+        x = cs ? cosf(f) : sinf(f);
+      }
+      x2[u] = x;
+    }
+    w[h] = tc::pack_bf16(x2[0], x2[1]);
+  }
+  pex[e] = make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// BF16 rgbnet: row m of the X tiles, the features beside the pixel's part. The
+// padding rows of the last tile are zero.
+template <int CT>
+__global__ void __launch_bounds__(256)
+    k_render_x(RenderP P, RenderW Wk, int64_t M, const uint4* __restrict__ pex, uint8_t* xt) {
+  const int64_t m = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+  if (m >= (M + 127) / 128 * 128) return;
+  uint4 row[6];
+#pragma unroll
+  for (int cb = 0; cb < 6; ++cb) row[cb] = make_uint4(0u, 0u, 0u, 0u);
+  if (m < M) {
+    const int n = Wk.rpix[m];
+#pragma unroll
+    for (int cb = CT == 12 ? 1 : 0; cb < 6; ++cb) row[cb] = __ldg(pex + int64_t(n) * 6 + cb);
+    float acc[CT ? CT : 16];
+    row_features<CT>(P, Wk, m, n, acc);
+    if (CT == 12) {
+      row[0] = make_uint4(tc::pack_bf16(acc[0], acc[1]), tc::pack_bf16(acc[2], acc[3]),
+                          tc::pack_bf16(acc[4], acc[5]), tc::pack_bf16(acc[6], acc[7]));
+      row[1].x = tc::pack_bf16(acc[8], acc[9]);
+      row[1].y = tc::pack_bf16(acc[10], acc[11]);
+    } else {
+      uint32_t* w = reinterpret_cast<uint32_t*>(row);
+#pragma unroll
+      for (int q = 0; q < 16; ++q) {
+        if (q >= P.dcol) continue;
+        const uint32_t b = tc::pack_bf16(acc[q < (CT ? CT : 16) ? q : 0], 0.f) & 0xFFFFu;
+        w[q >> 1] = q & 1 ? (w[q >> 1] & 0x0000FFFFu) | (b << 16) : (w[q >> 1] & 0xFFFF0000u) | b;
+      }
+    }
+  }
+  uint8_t* tile = xt + (m >> 7) * int64_t(kRgbXTile);
+#pragma unroll
+  for (int cb = 0; cb < 6; ++cb)
+    *reinterpret_cast<uint4*>(tile + tc::kmaj(int(m & 127), 8 * cb, kRgbXK)) = row[cb];
+}
+
+// One thread per pixel; the rows of a block's pixels are contiguous, so the
+// block forms their contributions w / (1 + exp(-logit)) together, a row a
+// thread, in chunks through shared memory, and each pixel then adds its own in
+// sample order.
+constexpr int kCompRows = 1024;
+__global__ void __launch_bounds__(256)
+    k_render_composite(RenderP P, RenderW Wk, const float* __restrict__ logits, float* image) {
+  __shared__ float part[kCompRows * 3];
+  const int HW = P.H * P.W;
+  const int n = blockIdx.x * 256 + threadIdx.x;
+  const int last = min(blockIdx.x * 256 + 255, HW - 1);
+  const int64_t b0 = Wk.off[blockIdx.x * 256];
+  const int64_t b1 = min(int64_t(Wk.off[last]) + Wk.n[last], Wk.cap);
+  const uint32_t cnt = n < HW ? Wk.n[n] : 0;
+  const int64_t off = n < HW ? Wk.off[n] : 0;
+  float acc[3];
+  acc[0] = acc[1] = acc[2] = n < HW && cnt ? __fmul_rn(Wk.T[n], P.bg) : P.bg;
+  for (int64_t c0 = b0; c0 < b1; c0 += kCompRows) {
+    const int nr = int(min(int64_t(kCompRows), b1 - c0));
+    for (int e = threadIdx.x; e < nr * 3; e += 256)
+      part[e] = __fdiv_rn(__ldg(Wk.rw + c0 + e / 3), 1.f + expf(-__ldg(logits + c0 * 3 + e)));
+    __syncthreads();
+    const int j0 = int(max(off, c0) - c0), j1 = int(min(off + cnt, c0 + nr) - c0);
+    for (int j = j0; j < j1; ++j)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) acc[c] = __fadd_rn(acc[c], part[3 * j + c]);
+    __syncthreads();
+  }
+  if (n >= HW) return;
+#pragma unroll
   for (int c = 0; c < 3; ++c) image[n * 3 + c] = acc[c];
+}
+
+// Per-voxel records of the leaves from the rows (row id rows[s]; slot
+// nleaf * 512: row 0): density, and 12-channel features in FP32 or BF16
+// (nearest even).
+__global__ void k_fill_voxels(int64_t nslots, const int32_t* __restrict__ rows,
+                              const float* __restrict__ den, const float* __restrict__ col,
+                              float* vden, float* vcol, __nv_bfloat16* vcolh) {
+  const int64_t s = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+  if (s > nslots) return;
+  const int64_t id = s < nslots ? rows[s] : 0;
+  vden[s] = den[id];
+  if (vcol)
+    for (int q = 0; q < 12; ++q) vcol[s * 12 + q] = col[id * 12 + q];
+  if (vcolh)
+    for (int q = 0; q < kHalfStride; ++q)
+      vcolh[s * kHalfStride + q] = __float2bfloat16_rn(q < 12 ? col[id * 12 + q] : 0.f);
+}
+
+__global__ void k_to_bf16(const float* __restrict__ src, __nv_bfloat16* dst, int64_t n) {
+  const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+  if (i < n) dst[i] = __float2bfloat16_rn(src[i]);
 }
 
 __global__ void k_fill_rows(GridView g, int32_t* rows, const int32_t* __restrict__ dense, int rx,
@@ -405,10 +465,11 @@ struct pvdb_renderer_s {
   int dcol, dpe, dhid, dout;
   bool flags[5] = {false, false, false, false, false};
   pvdb_grid_s* topo = nullptr;
+  // 12 channels: per-voxel records only; other counts: row ids and rows
   int32_t* d_rows = nullptr;
-  float* d_den = nullptr;
-  float* d_col = nullptr;
-  __nv_bfloat16* d_colh = nullptr;
+  float* d_vden = nullptr;
+  float* d_col = nullptr;           // rows, or the per-voxel records
+  __nv_bfloat16* d_colh = nullptr;  // rows, or the per-voxel records
   int64_t nrows = 0;
   int storage = 0;
   float* d_params = nullptr;  // [w0 (dhid x din), b0, w1, b1, w2 (3 x dhid), b2]
@@ -429,6 +490,7 @@ struct pvdb_renderer_s {
   size_t scan_partial_cap = 0;
   float* d_rk0 = nullptr;
   float* d_rw = nullptr;
+  float* d_rt = nullptr;
   int32_t* d_rpix = nullptr;
   float* d_logits = nullptr;
   int64_t rows_cap = 0;
@@ -441,14 +503,15 @@ struct pvdb_renderer_s {
 static int renderer_grow_rows(pvdb_renderer_s* r, int64_t need) {
   if (need <= r->rows_cap) return PVDB_OK;
   const int64_t cap = std::max<int64_t>(need + need / 4, 1 << 20);
-  void* ptrs[] = {r->d_rk0, r->d_rw, r->d_rpix, r->d_logits};
+  void* ptrs[] = {r->d_rk0, r->d_rw, r->d_rt, r->d_rpix, r->d_logits};
   for (void* p : ptrs) dev_free(p);
-  r->d_rk0 = r->d_rw = r->d_logits = nullptr;
+  r->d_rk0 = r->d_rw = r->d_rt = r->d_logits = nullptr;
   r->d_rpix = nullptr;
   r->rows_cap = 0;
   int rc;
   if ((rc = dev_alloc((void**)&r->d_rk0, size_t(cap) * r->dcol * 4)) ||
       (rc = dev_alloc((void**)&r->d_rw, size_t(cap) * 4)) ||
+      (rc = dev_alloc((void**)&r->d_rt, size_t(cap) * 4)) ||
       (rc = dev_alloc((void**)&r->d_rpix, size_t(cap) * 4)) ||
       (rc = dev_alloc((void**)&r->d_logits, size_t(cap) * 12)))
     return rc;
@@ -486,9 +549,9 @@ int pvdb_renderer_create(int32_t dcol, int32_t dpe, int32_t dhid, int32_t dout,
 int pvdb_renderer_destroy(pvdb_renderer r) {
   if (!r) return PVDB_OK;
   pvdb_grid_destroy(r->topo);
-  void* ptrs[] = {r->d_rows, r->d_den, r->d_col, r->d_colh, r->d_params, r->d_n, r->d_off,
+  void* ptrs[] = {r->d_rows, r->d_vden, r->d_col, r->d_colh, r->d_params, r->d_n, r->d_off,
                   r->d_T, r->d_viewdirs, r->d_hpe, r->d_image, r->d_totals, r->scan_partial,
-                  r->d_rk0, r->d_rw, r->d_rpix, r->d_logits, r->d_packed, r->d_xt};
+                  r->d_rk0, r->d_rw, r->d_rt, r->d_rpix, r->d_logits, r->d_packed, r->d_xt};
   for (void* p : ptrs) dev_free(p);
   delete r;
   return PVDB_OK;
@@ -516,47 +579,65 @@ int pvdb_renderer_load_data(pvdb_renderer r, const int32_t reso[3], const int32_
   }
   pvdb_grid_destroy(r->topo);
   r->topo = nullptr;
+  r->flags[0] = false;  // until everything below is in place
   int rc = pvdb_grid_create_from_mask(reso, 1, 0.f, active.data(), PVDB_MEM_HOST, &r->topo);
   if (rc) return rc;
   dev_free(r->d_rows);
-  dev_free(r->d_den);
+  dev_free(r->d_vden);
   dev_free(r->d_col);
   dev_free(r->d_colh);
   r->d_rows = nullptr;
-  r->d_den = r->d_col = nullptr;
+  r->d_vden = r->d_col = nullptr;
   r->d_colh = nullptr;
   const int64_t ns = r->topo->nslots();
-  int32_t* d_dense = nullptr;
-  if ((rc = dev_alloc((void**)&r->d_rows, std::max<int64_t>(ns, 1) * 4)) ||
-      (rc = dev_alloc((void**)&d_dense, nvox * 4)) ||
-      (rc = dev_alloc((void**)&r->d_den, n_rows * 4))) {
-    dev_free(d_dense);
-    return rc;
-  }
-  const cudaMemcpyKind kind = mem == PVDB_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
-  PVDB_CHECK_CUDA(cudaMemcpy(d_dense, index, nvox * 4, kind));
-  if (ns) k_fill_rows<<<ceil_div(ns, 256), 256>>>(r->topo->view(), r->d_rows, d_dense, reso[0], reso[1], reso[2]);
-  PVDB_CHECK_LAUNCH("k_fill_rows");
-  PVDB_CHECK_CUDA(cudaDeviceSynchronize());
-  dev_free(d_dense);
-  PVDB_CHECK_CUDA(cudaMemcpy(r->d_den, density, n_rows * 4, kind));
   const size_t nf = size_t(n_rows) * r->dcol;
-  if (storage == 0) {
-    if ((rc = dev_alloc((void**)&r->d_col, nf * 4))) return rc;
-    PVDB_CHECK_CUDA(cudaMemcpy(r->d_col, features, nf * 4, kind));
-  } else {
-    std::vector<float> hf;
-    const float* f = features;
-    if (mem == PVDB_MEM_DEVICE) {
-      hf.resize(nf);
-      PVDB_CHECK_CUDA(cudaMemcpy(hf.data(), features, nf * 4, cudaMemcpyDeviceToHost));
-      f = hf.data();
+  const bool voxels = r->dcol == 12;
+  // device copies of the inputs, freed on every way out
+  struct Temp {
+    int32_t *dense = nullptr, *rows = nullptr;
+    float *den = nullptr, *col = nullptr;
+    ~Temp() {
+      dev_free(dense);
+      dev_free(rows);
+      dev_free(den);
+      dev_free(col);
     }
-    std::vector<__nv_bfloat16> hb(nf);
-    for (size_t q = 0; q < nf; ++q) hb[q] = __float2bfloat16_rn(f[q]);
-    if ((rc = dev_alloc((void**)&r->d_colh, nf * 2))) return rc;
-    PVDB_CHECK_CUDA(cudaMemcpy(r->d_colh, hb.data(), nf * 2, cudaMemcpyHostToDevice));
+  } tmp;
+  if ((rc = dev_alloc((void**)&tmp.rows, std::max<int64_t>(ns, 1) * 4)) ||
+      (rc = dev_alloc((void**)&tmp.dense, nvox * 4)) ||
+      (rc = dev_alloc((void**)&tmp.den, n_rows * 4)) ||
+      (rc = dev_alloc((void**)&tmp.col, nf * 4)) ||
+      (rc = dev_alloc((void**)&r->d_vden, (ns + 1) * 4)))
+    return rc;
+  if (storage == 0)
+    rc = dev_alloc((void**)&r->d_col, voxels ? size_t(ns + 1) * 48 : nf * 4);
+  else
+    rc = dev_alloc((void**)&r->d_colh, voxels ? size_t(ns + 1) * kHalfStride * 2 : nf * 2);
+  if (rc) return rc;
+  const cudaMemcpyKind kind = mem == PVDB_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
+  PVDB_CHECK_CUDA(cudaMemcpy(tmp.dense, index, nvox * 4, kind));
+  PVDB_CHECK_CUDA(cudaMemcpy(tmp.den, density, n_rows * 4, kind));
+  PVDB_CHECK_CUDA(cudaMemcpy(tmp.col, features, nf * 4, kind));
+  if (ns) {
+    k_fill_rows<<<ceil_div(ns, 256), 256>>>(r->topo->view(), tmp.rows, tmp.dense, reso[0], reso[1],
+                                            reso[2]);
+    PVDB_CHECK_LAUNCH("k_fill_rows");
   }
+  k_fill_voxels<<<ceil_div(ns + 1, 256), 256>>>(ns, tmp.rows, tmp.den, tmp.col, r->d_vden,
+                                                voxels ? r->d_col : nullptr,
+                                                voxels ? r->d_colh : nullptr);
+  PVDB_CHECK_LAUNCH("k_fill_voxels");
+  if (!voxels) {
+    if (storage == 0) {
+      PVDB_CHECK_CUDA(cudaMemcpy(r->d_col, tmp.col, nf * 4, cudaMemcpyDeviceToDevice));
+    } else {
+      k_to_bf16<<<ceil_div(nf, 256), 256>>>(tmp.col, r->d_colh, int64_t(nf));
+      PVDB_CHECK_LAUNCH("k_to_bf16");
+    }
+    r->d_rows = tmp.rows;
+    tmp.rows = nullptr;
+  }
+  PVDB_CHECK_CUDA(cudaDeviceSynchronize());
   r->nrows = n_rows;
   r->storage = storage;
   for (int a = 0; a < 3; ++a) r->reso[a] = reso[a];
@@ -680,21 +761,23 @@ int pvdb_renderer_render(pvdb_renderer r, int32_t precision, pvdb_stream s) {
   P.t_stop = r->t_stop;
   P.dcol = r->dcol;
   P.idx = r->topo->view();
+  P.nslots = r->topo->nslots();
+  P.vden = r->d_vden;
   P.rows = r->d_rows;
-  P.den = r->d_den;
-  P.col = r->d_col;
-  P.colh = r->d_colh;
+  P.vcol = P.col = r->d_col;
+  P.vcolh = P.colh = r->d_colh;
   P.storage = r->storage;
   RenderW Wk{};
   Wk.n = r->d_n;
   Wk.off = r->d_off;
   Wk.T = r->d_T;
   Wk.viewdirs = r->d_viewdirs;
-  Wk.totals = r->d_totals;
   const int HW = r->H * r->W;
   prof_begin_call();
   prof_mark(st, 0);
-  k_render_march<false><<<ceil_div(HW, 128), 128, 0, st>>>(P, Wk);
+  // 4 warps a block, 8 x 4 pixels a warp
+  const int march_grid = ceil_div(int64_t(ceil_div(r->W, 8)) * ceil_div(r->H, 4), 4);
+  k_render_march<false><<<march_grid, 128, 0, st>>>(P, Wk);
   PVDB_CHECK_LAUNCH("k_render_march<count>");
   prof_mark(st, 1);
   int rc = scan_exclusive_u32(r->d_n, r->d_off, HW, r->d_totals + 1, &r->scan_partial,
@@ -708,6 +791,7 @@ int pvdb_renderer_render(pvdb_renderer r, int32_t precision, pvdb_stream s) {
   if (rc) return rc;
   Wk.rk0 = r->d_rk0;
   Wk.rw = r->d_rw;
+  Wk.rt = r->d_rt;
   Wk.rpix = r->d_rpix;
   Wk.cap = r->rows_cap;
   MlpArgs a;
@@ -721,25 +805,36 @@ int pvdb_renderer_render(pvdb_renderer r, int32_t precision, pvdb_stream s) {
   a.c0 = r->dcol;
   a.dpe = r->dpe;
   a.din = din;
-  // BF16 rgbnet: the fill pass writes the X tiles (with the PE computed first)
-  const bool x_direct = precision == 1 && total > 0 && din + 1 <= kRgbXK;
-  if (x_direct) {
-    const int64_t ntiles = (r->rows_cap + 127) / 128;
-    if ((rc = dev_reserve(&r->d_xt, &r->xt_cap, size_t(ntiles) * kRgbXTile))) return rc;
-    int pe_stride = 0;
-    if ((rc = mlp_pe_rows(a, r->d_viewdirs, HW, r->d_hpe, &pe_stride, st))) return rc;
-    Wk.xt = static_cast<uint8_t*>(r->d_xt);
-    Wk.pe = r->d_hpe + size_t(HW) * H;
-    Wk.pe_stride = pe_stride;
-    Wk.dpe = r->dpe;
+  if (total) {
+    k_render_march<true><<<march_grid, 128, 0, st>>>(P, Wk);
+    PVDB_CHECK_LAUNCH("k_render_march<fill>");
+    const int64_t M = total;
+    const int rgrid = ceil_div((M + 127) / 128 * 128, 256);
+    if (precision == 1) {
+      const int64_t ntiles = (r->rows_cap + 127) / 128;
+      if ((rc = dev_reserve(&r->d_xt, &r->xt_cap, size_t(ntiles) * kRgbXTile))) return rc;
+      uint4* pex = reinterpret_cast<uint4*>(r->d_hpe);  // 96 of the 640 bytes a pixel
+      uint8_t* xt = static_cast<uint8_t*>(r->d_xt);
+      k_render_pe<<<ceil_div(int64_t(HW) * 6, 192), 192, 0, st>>>(P, Wk, (r->dpe - 3) / 6, pex);
+      PVDB_CHECK_LAUNCH("k_render_pe");
+      if (r->dcol == 12)
+        k_render_x<12><<<rgrid, 256, 0, st>>>(P, Wk, M, pex, xt);
+      else
+        k_render_x<0><<<rgrid, 256, 0, st>>>(P, Wk, M, pex, xt);
+      PVDB_CHECK_LAUNCH("k_render_x");
+    } else {
+      if (r->dcol == 12)
+        k_render_k0<12><<<rgrid, 256, 0, st>>>(P, Wk, M);
+      else
+        k_render_k0<0><<<rgrid, 256, 0, st>>>(P, Wk, M);
+      PVDB_CHECK_LAUNCH("k_render_k0");
+    }
   }
-  k_render_march<true><<<ceil_div(HW, 128), 128, 0, st>>>(P, Wk);
-  PVDB_CHECK_LAUNCH("k_render_march<fill>");
   prof_mark(st, 3);
   if (total) {
-    rc = mlp_forward_rows(a, r->d_rk0, r->d_rpix, r->d_viewdirs, HW, r->d_totals, r->rows_cap,
-                          r->d_logits, 1, r->d_hpe, precision, &r->d_packed, &r->packed_cap,
-                          &r->d_xt, &r->xt_cap, r->d_totals + 3, st, x_direct ? 1 : 0);
+    rc = mlp_forward_rows(a, r->d_rk0, r->d_rpix, r->d_viewdirs, HW, r->d_n, r->d_totals,
+                          r->rows_cap, r->d_logits, 1, r->d_hpe, precision, &r->d_packed,
+                          &r->packed_cap, &r->d_xt, &r->xt_cap, r->d_totals + 3, st);
     if (rc) return rc;
   }
   prof_mark(st, 4);
