@@ -158,8 +158,8 @@ int mlp_tc_pack(const float* w0, const float* b0, const float* w1, const float* 
 int mlp_tc_forward_rows(const float* w0, const float* b0, const float* w1, const float* b1,
                         const float* w2, const float* b2, int c0, int dpe, const float* k0rows,
                         const int32_t* ray, const float* pe, int pe_stride, const uint32_t* totals,
-                        int64_t max_rows, float* out, int out_logits, void** blob,
-                        size_t* blob_cap, void** xt, size_t* xt_cap, uint32_t* err,
+                        int64_t max_rows, float* out, const float* rw, void** blob, size_t* blob_cap,
+                        void** xt, size_t* xt_cap, uint32_t* err,
                         cudaStream_t st, int packed, int x_ready);
 
 // Inputs of the rgbnet that depend only on the rays and the weights: the
@@ -205,29 +205,30 @@ int mlp_forward_impl(pvdb_march_s* m, const MlpArgs& a, const float* k0rows,
     return rc;
   if (precision == 1)
     return mlp_tc_forward_rows(a.w0, a.b0, a.w1, a.b1, a.w2, a.b2, a.c0, a.dpe, k0rows,
-                               m->w.r_ray, pe, kMaxPe, m->w.totals, m->slots, rgb, 0,
+                               m->w.r_ray, pe, kMaxPe, m->w.totals, m->slots, rgb, nullptr,
                                &m->mlp_packed, &m->mlp_packed_cap, &m->mlp_xt, &m->mlp_xt_cap,
                                m->w.totals + 3, st, prepared ? 1 : 0, x_ready ? 1 : 0);
-  return mlp_f32_forward(a, k0rows, m->w.r_ray, hpe, m->w.totals, rgb, 0, st);
+  return mlp_f32_forward(a, k0rows, m->w.r_ray, hpe, m->w.totals, rgb, nullptr, st);
 }
 
-// Rows from the merged renderer; M = totals[1]. FP32: k0rows [M, c0], ray [M]
-// -> viewdirs [R,3], hpe_buf holds R*(128+32) floats; the rays whose entry of
+// Rows from the merged renderer; M = totals[1]; out [M, 3] gets each row's
+// contribution rw / (1 + exp(-logit)). FP32: k0rows [M, c0], ray [M] ->
+// viewdirs [R,3], hpe_buf holds R*(128+32) floats; the rays whose entry of
 // `need` is zero have no row. BF16: the X tiles in *xt are already built.
 int mlp_forward_rows(const MlpArgs& a, const float* k0rows, const int32_t* ray,
                      const float* viewdirs, int R, const uint32_t* need, const uint32_t* totals,
-                     int64_t max_rows, float* out, int out_logits, float* hpe_buf, int precision,
+                     int64_t max_rows, const float* rw, float* out, float* hpe_buf, int precision,
                      void** blob, size_t* blob_cap, void** xt, size_t* xt_cap, uint32_t* err,
                      cudaStream_t st) {
   if (R <= 0) return PVDB_OK;
   if (precision == 1)
     return mlp_tc_forward_rows(a.w0, a.b0, a.w1, a.b1, a.w2, a.b2, a.c0, a.dpe, k0rows, ray,
-                               nullptr, kMaxPe, totals, max_rows, out, out_logits, blob, blob_cap,
-                               xt, xt_cap, err, st, 0, 1);
+                               nullptr, kMaxPe, totals, max_rows, out, rw, blob, blob_cap, xt,
+                               xt_cap, err, st, 0, 1);
   float* pe = hpe_buf + size_t(R) * kW;
   const int rc = pe_launch(viewdirs, R, a, pe, hpe_buf, need, st);
   if (rc) return rc;
-  return mlp_f32_forward(a, k0rows, ray, hpe_buf, totals, out, out_logits, st);
+  return mlp_f32_forward(a, k0rows, ray, hpe_buf, totals, out, rw, st);
 }
 
 int mlp_tc_backward_rows(const float* w0, const float* b0, const float* w1, const float* b1,

@@ -147,7 +147,7 @@ __device__ __forceinline__ void fwd_tile(FwdSmem<CQ>& S, FwdGroupSmem<CQ>& G, in
                                          const MlpArgs& a, const float* __restrict__ k0,
                                          const int32_t* __restrict__ ray,
                                          const float* __restrict__ hpe, int64_t row0, int64_t M,
-                                         float* out, int out_logits) {
+                                         float* out, const float* rw) {
   constexpr int TR = RT == 2 ? 128 : 32;
   constexpr int ld = TR + 4;
   constexpr int kColWarps = RT == 2 ? 2 : 4;
@@ -220,7 +220,8 @@ __device__ __forceinline__ void fwd_tile(FwdSmem<CQ>& S, FwdGroupSmem<CQ>& G, in
 #pragma unroll
     for (int w = 1; w < kColWarps; ++w) s += red[w * TR * 3 + e];
     s += S.b2[e % 3];
-    if (row0 * 3 + e < M * 3) out[row0 * 3 + e] = out_logits ? s : 1.f / (1.f + expf(-s));
+    if (row0 * 3 + e < M * 3)
+      out[row0 * 3 + e] = __fdiv_rn(rw ? __ldg(rw + row0 + e / 3) : 1.f, 1.f + expf(-s));
   }
   bar_group(bar, kFwdGroup);  // the partials are read: the next tile's rows may land
 }
@@ -229,7 +230,7 @@ template <int CQ>
 __global__ void __launch_bounds__(kFwdThreads, 1)
     k_mlp_fwd_f32(MlpArgs a, const float* __restrict__ k0, const int32_t* __restrict__ ray,
                   const float* __restrict__ hpe, const uint32_t* __restrict__ totals, float* out,
-                  int out_logits) {
+                  const float* __restrict__ rw) {
   grid_dep_sync();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   FwdSmem<CQ>& S = *reinterpret_cast<FwdSmem<CQ>*>(smem_raw);
@@ -256,9 +257,9 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
   const int64_t u = int64_t(blockIdx.x) + int64_t(gridDim.x) * g;
   FwdGroupSmem<CQ>& G = S.g[g];
   for (int64_t i = u; i < P.full; i += units)
-    fwd_tile<2, 2, CQ>(S, G, 1 + g, t, a, k0, ray, hpe, i * 128, M, out, out_logits);
+    fwd_tile<2, 2, CQ>(S, G, 1 + g, t, a, k0, ray, hpe, i * 128, M, out, rw);
   for (int64_t r = P.row32 + u * 32; r < M; r += units * 32)
-    fwd_tile<1, 1, CQ>(S, G, 1 + g, t, a, k0, ray, hpe, r, M, out, out_logits);
+    fwd_tile<1, 1, CQ>(S, G, 1 + g, t, a, k0, ray, hpe, r, M, out, rw);
 }
 
 // ---------------------------------------------------------------- backward
@@ -655,10 +656,10 @@ static_assert(sizeof(FwdSmem<4>) <= 227 * 1024 && sizeof(BwdSmem<4>) <= 227 * 10
 
 template <int CQ>
 int fwd_launch(const MlpArgs& a, const float* k0, const int32_t* ray, const float* hpe,
-               const uint32_t* totals, float* out, int out_logits, cudaStream_t st) {
+               const uint32_t* totals, float* out, const float* rw, cudaStream_t st) {
   PVDB_SMEM_ATTR(k_mlp_fwd_f32<CQ>, int(sizeof(FwdSmem<CQ>)));
   launch_k(k_mlp_fwd_f32<CQ>, num_sms(), kFwdThreads, sizeof(FwdSmem<CQ>), st, a, k0, ray, hpe,
-           totals, out, out_logits);
+           totals, out, rw);
   PVDB_CHECK_LAUNCH("k_mlp_fwd_f32");
   return PVDB_OK;
 }
@@ -677,9 +678,9 @@ int bwd_launch(const MlpArgs& a, const BwdIn& in, const uint32_t* totals, float*
 // Up to 12 k0 channels (at most 39 input columns) or up to 16 (43): the
 // channel count padded to 12 or 16 with zeros.
 int mlp_f32_forward(const MlpArgs& a, const float* k0, const int32_t* ray, const float* hpe,
-                    const uint32_t* totals, float* out, int out_logits, cudaStream_t st) {
-  return a.c0 <= 12 ? fwd_launch<3>(a, k0, ray, hpe, totals, out, out_logits, st)
-                    : fwd_launch<4>(a, k0, ray, hpe, totals, out, out_logits, st);
+                    const uint32_t* totals, float* out, const float* rw, cudaStream_t st) {
+  return a.c0 <= 12 ? fwd_launch<3>(a, k0, ray, hpe, totals, out, rw, st)
+                    : fwd_launch<4>(a, k0, ray, hpe, totals, out, rw, st);
 }
 
 int mlp_f32_backward(const MlpArgs& a, const float* k0, const int32_t* ray, const float* hpe,

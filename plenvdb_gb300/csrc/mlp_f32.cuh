@@ -18,9 +18,9 @@ __host__ __device__ inline int64_t mlp_param_count(int din) {
 }
 
 // rows: k0 [M, c0], ray [M], M = totals[1]; hpe [rays, 128]: the per-ray part
-// of layer 0; out [M, 3]: logits or their sigmoid.
+// of layer 0; out [M, 3]: sigmoid of the logits, times rw [M] when given.
 int mlp_f32_forward(const MlpArgs& a, const float* k0, const int32_t* ray, const float* hpe,
-                    const uint32_t* totals, float* out, int out_logits, cudaStream_t st);
+                    const uint32_t* totals, float* out, const float* rw, cudaStream_t st);
 
 // grad_k0 [M, c0] and per-CTA partial weight gradients wpart [grid][param count]
 // in the flat layout; pe [rays, 32]: the per-ray PE.

@@ -6,17 +6,18 @@
 // is X = [k0 (c0) | PE (dpe) | 1 | 0...], 48 BF16 columns, so layer 0 is one
 // K=48 GEMM against W0f = [W0 | b0 | 0] (the bias rides on the ones column).
 //
-// Forward (k_mlp_fwd_tc: persistent CTAs, 8 warps, 2 CTAs per SM, 256 TMEM
-// columns each):
+// Forward (k_mlp_fwd_tc), per tile:
 //   L0  Z0 = X . W0f^T            3 MMAs (K=48)        H0 = relu(Z0)
 //   L1  Z1 = H0 . W1^T            8 MMAs (K=128)       H1 = relu(Z1 + b1)
 //   L2  Z2 = H1 . W2p^T           8 MMAs, N=16         rgb = sigmoid(Z2 + b2)
-// X tiles are built once per step (k_build_x) and each CTA fetches the next
-// tile's with a bulk copy while the current tile computes. One thread issues
-// the MMAs; completion is signalled through an
-// mbarrier (tcgen05.commit). Epilogues read TMEM with tcgen05.ld (warp w reads
-// lanes 32*(w%4).., columns 64*(w/4)..), apply bias/activation in FP32 and
-// store BF16 into shared memory in the canonical layout the next MMA reads.
+// X tiles are built beforehand and fetched with bulk copies. A tile is a chain
+// of three MMA batches and three epilogues, so the kernel is bound by that
+// chain's latency and by how many chains an SM keeps going: one persistent CTA
+// per SM shares the 48 KB of weights between four independent warpgroups, each
+// with its own tile, 128 TMEM columns (Z0, Z1 and Z2 in turn), barriers and
+// issuing thread. Epilogues read TMEM with tcgen05.ld (thread = tile row),
+// apply bias/activation in FP32 and store BF16 into shared memory in the
+// canonical layout the next MMA reads.
 #include <algorithm>
 
 #include "march.cuh"
@@ -27,7 +28,8 @@ namespace pvdb {
 namespace {
 
 constexpr int kW = 128;
-constexpr int kTcThreads = 256;
+constexpr int kFwdSlots = 4;                    // warpgroups, a tile in flight each
+constexpr int kFwdThreads = 128 * kFwdSlots;
 constexpr int kXK = kRgbXK;  // input columns of a row: k0 | PE | 1 | 0
 // packed weight blob (bytes, canonical K-major BF16 tiles)
 constexpr uint32_t kOffW0 = 0;                             // W0f  [128 n][48 q]
@@ -36,16 +38,16 @@ constexpr uint32_t kOffW2 = kOffW1 + 128 * 128 * 2;        // W2p  [16 c][128 k]
 constexpr uint32_t kPackFwdBytes = kOffW2 + 16 * 128 * 2;  // 49152
 // shared-memory layout of the forward kernel
 constexpr uint32_t kXTile = kRgbXTile;                // 12288 B: one X tile
-constexpr uint32_t kSmX = kPackFwdBytes;              // two X tiles [128 x 48] bf16
-constexpr uint32_t kSmH = kSmX + 2 * kXTile;          // H tile [128 x 128] bf16
-constexpr uint32_t kSmB1 = kSmH + 128 * 128 * 2;      // b1 f32[128]
-constexpr uint32_t kSmB2 = kSmB1 + 128 * 4;           // b2 f32[16]
-constexpr uint32_t kSmBar = kSmB2 + 16 * 4;           // mbarriers: MMA, X0, X1, weights (32 B)
-constexpr uint32_t kSmTmem = kSmBar + 32;             // TMEM base address (4 B)
-constexpr uint32_t kSmFlag = kSmTmem + 4;             // timeout flag (4 B)
-constexpr uint32_t kSmFwdBytes = kSmFlag + 16;
-static_assert(2 * kSmFwdBytes <= 228 * 1024, "two forward CTAs must fit on an SM");
-constexpr uint32_t kTmemCols = 256;
+constexpr uint32_t kSlotBytes = kXTile + 128 * 128 * 2;     // X [128 x 48], H [128 x 128] bf16
+constexpr uint32_t kSmSlots = kPackFwdBytes;
+constexpr uint32_t kSmB1 = kSmSlots + kFwdSlots * kSlotBytes;  // b1 f32[128]
+constexpr uint32_t kSmB2 = kSmB1 + 128 * 4;                    // b2 f32[16]
+constexpr uint32_t kSmBar = kSmB2 + 16 * 4;  // mbarriers: MMA, X per slot, then the weights
+constexpr uint32_t kSmTmem = kSmBar + 8 * (2 * kFwdSlots + 1);  // TMEM base address (4 B)
+constexpr uint32_t kSmFlag = kSmTmem + 4;                       // timeout flag per slot
+constexpr uint32_t kSmFwdBytes = kSmFlag + 4 * kFwdSlots;
+static_assert(kSlotBytes % 1024 == 0 && kSmFwdBytes <= 232448, "the forward CTA's shared memory");
+constexpr uint32_t kTmemCols = 128 * kFwdSlots;
 constexpr uint32_t kWaitIters = 1u << 22;
 
 struct MlpArgsTc {
@@ -77,16 +79,6 @@ __global__ void k_pack(MlpArgsTc a, uint8_t* blob) {
     const int n = t / 128, k = t % 128;
     w2[tc::kmaj(n, k, 128) / 2] = __float2bfloat16_rn(n < 3 ? a.w2[n * 128 + k] : 0.f);
   }
-}
-
-__device__ __forceinline__ bool wait_or_flag(uint64_t* bar, uint32_t parity, uint32_t* flag,
-                                             uint32_t* err) {
-  if (!tc::mbar_wait(bar, parity, kWaitIters)) {
-    atomicOr(flag, 1u);
-    if (err) atomicOr(err, 2u);
-  }
-  __syncthreads();
-  return *((volatile uint32_t*)flag) == 0;
 }
 
 // The rows' X tiles in global memory, tile after tile in the canonical BF16
@@ -162,36 +154,71 @@ __device__ __forceinline__ void store_relu32(uint8_t* tile, int row, int col0, i
         relu_pack8(v + 8 * c, bias, col0 + 8 * c);
 }
 
-__global__ void __launch_bounds__(kTcThreads, 2)
+// relu(Z [+ bias]) of this thread's row, 128 columns, as BF16 into the K-major
+// tile; the TMEM load of a chunk travels while the previous one is packed.
+__device__ __forceinline__ void epilogue_relu(uint32_t taddr, uint8_t* tile, int row,
+                                              const float* bias) {
+  uint32_t r[2][32];
+  tc::tmem_ld16_issue(taddr, r[0]);
+  tc::tmem_ld16_issue(taddr + 16, r[0] + 16);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    tc::tmem_wait_ld();
+    if (j < 3) {
+      tc::tmem_ld16_issue(taddr + 32 * (j + 1), r[(j + 1) & 1]);
+      tc::tmem_ld16_issue(taddr + 32 * (j + 1) + 16, r[(j + 1) & 1] + 16);
+    }
+    float v[32];
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[j & 1][i]);
+    store_relu32(tile, row, 32 * j, 128, v, bias);
+  }
+}
+
+__device__ __forceinline__ void slot_sync(int slot) {
+  asm volatile("bar.sync %0, 128;" ::"r"(1 + slot) : "memory");
+}
+
+// out [M, 3]: sigmoid(Z2 + b2), times rw [M] when given (a row's contribution to
+// its pixel).
+__global__ void __launch_bounds__(kFwdThreads, 1)
     k_mlp_fwd_tc(MlpArgsTc a, const uint8_t* __restrict__ blob, const uint8_t* __restrict__ xt,
-                 const uint32_t* __restrict__ totals, float* out, int out_logits, uint32_t* err) {
+                 const uint32_t* __restrict__ totals, float* out, const float* __restrict__ rw,
+                 uint32_t* err) {
   grid_dep_sync();
   extern __shared__ __align__(1024) uint8_t sm[];
   const int64_t M = totals[1];
   const int64_t ntiles = (M + 127) / 128;
   if (blockIdx.x >= ntiles) return;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  uint64_t* bar = reinterpret_cast<uint64_t*>(sm + kSmBar);
+  const int tid = threadIdx.x, slot = tid >> 7, row = tid & 127;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sm + kSmBar);
+  uint64_t* bar = bars + 2 * slot;       // this slot's MMAs
+  uint64_t* xbar = bars + 2 * slot + 1;  // this slot's X tile
+  uint64_t* wbar = bars + 2 * kFwdSlots;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + kSmTmem);
-  uint32_t* flag = reinterpret_cast<uint32_t*>(sm + kSmFlag);
+  uint32_t* flag = reinterpret_cast<uint32_t*>(sm + kSmFlag) + slot;
   float* b1s = reinterpret_cast<float*>(sm + kSmB1);
   float* b2s = reinterpret_cast<float*>(sm + kSmB2);
+  uint8_t* sx = sm + kSmSlots + slot * kSlotBytes;
+  uint8_t* sh = sx + kXTile;
+  // tile u, u + stride, ... per slot: the slots of different SMs come first
+  const int64_t u = int64_t(blockIdx.x) + int64_t(gridDim.x) * slot;
+  const int64_t stride = int64_t(gridDim.x) * kFwdSlots;
   if (tid < 128) b1s[tid] = a.b1[tid];
   if (tid < 16) b2s[tid] = tid < 3 ? a.b2[tid] : 0.f;
-  uint64_t* xbar = bar + 1;  // X tile barriers, one per buffer
-  uint64_t* wbar = bar + 3;  // the weight tiles
   if (tid == 0) {
+    tc::mbar_init(wbar, 1);
+    // the packed weights (48 KB) in one bulk copy, beside the first X tiles'
+    tc::mbar_expect_tx(wbar, kPackFwdBytes);
+    tc::bulk_g2s(sm, blob, kPackFwdBytes, wbar);
+  }
+  if (row == 0) {
     *flag = 0;
     tc::mbar_init(bar, 1);
     tc::mbar_init(xbar, 1);
-    tc::mbar_init(xbar + 1, 1);
-    tc::mbar_init(wbar, 1);
-    // the packed weights (48 KB) in one bulk copy, beside the first X tile's
-    tc::mbar_expect_tx(wbar, kPackFwdBytes);
-    tc::bulk_g2s(sm, blob, kPackFwdBytes, wbar);
-    x_fetch(sm + kSmX, xt, blockIdx.x, xbar);
+    if (u < ntiles) x_fetch(sx, xt, u, xbar);
   }
-  if (warp == 0) {
+  if (tid < 32) {
     tc::tmem_alloc(tmem_slot, kTmemCols);
     tc::tmem_relinquish();
   }
@@ -200,106 +227,97 @@ __global__ void __launch_bounds__(kTcThreads, 2)
   tc::fence_after();
   const uint32_t tmem = *tmem_slot;
   const uint32_t sbase = tc::smem_addr(sm);
+  const uint32_t xb = tc::smem_addr(sx), hb = tc::smem_addr(sh);
+  const uint32_t d = tmem + 128u * slot;                              // the slot's columns
+  const uint32_t t_lane = d + (uint32_t(row & ~31) << 16);           // this warp's lanes
   const uint32_t id_n128 = tc::idesc_bf16(128, 128);
   const uint32_t id_n16 = tc::idesc_bf16(128, 16);
-  const int q = warp & 3, half = warp >> 2;
-  const int row = 32 * q + lane;  // TMEM lane = tile row of this thread
-  const uint32_t t_lane = tmem + (uint32_t(32 * q) << 16);
-  uint32_t phase = 0, xph[2] = {0u, 0u};
-  bool ok = true;
-  int it = 0;
-  for (int64_t t = blockIdx.x; t < ntiles && ok; t += gridDim.x, ++it) {
-    const int64_t row0 = t * 128;
-    const int b = it & 1;
-    // the next tile's X travels while this tile computes (its buffer was last
-    // read by the previous tile's layer-0 MMA, complete)
-    if (tid == 0 && t + gridDim.x < ntiles) x_fetch(sm + kSmX + (b ^ 1) * kXTile, xt, t + gridDim.x, xbar + (b ^ 1));
-    ok = wait_or_flag(xbar + b, xph[b], flag, err);
-    if (!ok) break;
-    xph[b] ^= 1u;
-    if (it == 0 && !(ok = wait_or_flag(wbar, 0, flag, err))) break;
-    if (tid == 0) {
+  uint32_t phase = 0, xph = 0;
+  bool ok = true, x_out = false;
+  // a wait that gives up flags the slot; its threads leave together after the
+  // next slot barrier (what they read until then is in bounds, if wrong)
+  auto wait = [&](uint64_t* b, uint32_t parity) {
+    if (tc::mbar_wait(b, parity, kWaitIters)) return;
+    atomicOr(flag, 1u);
+    if (err) atomicOr(err, 2u);
+  };
+  auto slot_ok = [&]() {
+    tc::fence_before();
+    tc::fence_async_smem();
+    slot_sync(slot);
+    return *((volatile uint32_t*)flag) == 0;
+  };
+  for (int64_t t = u; t < ntiles; t += stride) {
+    if (row == 0) {
+      wait(xbar, xph);
+      if (t == u) wait(wbar, 0);
       tc::fence_after();
 #pragma unroll
       for (int s = 0; s < 3; ++s)
-        tc::mma_bf16(tmem, tc::make_desc(sbase + kSmX + b * kXTile + 256 * s, 128, 768),
+        tc::mma_bf16(d, tc::make_desc(xb + 256 * s, 128, 768),
                      tc::make_desc(sbase + kOffW0 + 256 * s, 128, 768), id_n128, s > 0);
       tc::mma_commit(bar);
     }
-    ok = wait_or_flag(bar, phase, flag, err);
-    phase ^= 1;
-    if (!ok) break;
+    xph ^= 1u;
+    wait(bar, phase);
+    phase ^= 1u;
     tc::fence_after();
+    // the X tile is read: the next one travels from here
+    x_out = t + stride < ntiles;
+    if (row == 0 && x_out) x_fetch(sx, xt, t + stride, xbar);
     // ---- H0 = relu(Z0)
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      float v[32];
-      tc::tmem_ld32(t_lane + uint32_t(64 * half + 32 * j), v);
-      store_relu32(sm + kSmH, row, 64 * half + 32 * j, 128, v, nullptr);
-    }
-    tc::fence_before();
-    tc::fence_async_smem();
-    __syncthreads();
-    if (tid == 0) {
+    epilogue_relu(t_lane, sh, row, nullptr);
+    if (!(ok = slot_ok())) break;
+    if (row == 0) {
       tc::fence_after();
 #pragma unroll
       for (int s = 0; s < 8; ++s)
-        tc::mma_bf16(tmem + 128, tc::make_desc(sbase + kSmH + 256 * s, 128, 2048),
+        tc::mma_bf16(d, tc::make_desc(hb + 256 * s, 128, 2048),
                      tc::make_desc(sbase + kOffW1 + 256 * s, 128, 2048), id_n128, s > 0);
       tc::mma_commit(bar);
     }
-    ok = wait_or_flag(bar, phase, flag, err);
-    phase ^= 1;
-    if (!ok) break;
+    wait(bar, phase);
+    phase ^= 1u;
     tc::fence_after();
     // ---- H1 = relu(Z1 + b1), over H0
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      float v[32];
-      tc::tmem_ld32(t_lane + 128u + uint32_t(64 * half + 32 * j), v);
-      store_relu32(sm + kSmH, row, 64 * half + 32 * j, 128, v, b1s);
-    }
-    tc::fence_before();
-    tc::fence_async_smem();
-    __syncthreads();
-    if (tid == 0) {
+    epilogue_relu(t_lane, sh, row, b1s);
+    if (!(ok = slot_ok())) break;
+    if (row == 0) {
       tc::fence_after();
 #pragma unroll
       for (int s = 0; s < 8; ++s)
-        tc::mma_bf16(tmem, tc::make_desc(sbase + kSmH + 256 * s, 128, 2048),
+        tc::mma_bf16(d, tc::make_desc(hb + 256 * s, 128, 2048),
                      tc::make_desc(sbase + kOffW2 + 256 * s, 128, 2048), id_n16, s > 0);
       tc::mma_commit(bar);
     }
-    ok = wait_or_flag(bar, phase, flag, err);
-    phase ^= 1;
-    if (!ok) break;
+    wait(bar, phase);
+    phase ^= 1u;
     tc::fence_after();
-    // ---- logits (warps 0-3 hold all 16 columns of their rows)
-    if (half == 0) {
-      float v[16];
-      tc::tmem_ld16(t_lane, v);
-      const int64_t m = row0 + row;
-      if (m < M) {
+    // ---- logits
+    float v[16];
+    tc::tmem_ld16(t_lane, v);
+    const int64_t m = t * 128 + row;
+    if (m < M) {
+      const float w = rw ? __ldg(rw + m) : 1.f;
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          const float lg = v[c] + b2s[c];
-          out[m * 3 + c] = out_logits ? lg : 1.f / (1.f + expf(-lg));
-        }
+      for (int c = 0; c < 3; ++c) {
+        const float lg = v[c] + b2s[c];
+        out[m * 3 + c] = __fdiv_rn(w, 1.f + expf(-lg));
       }
     }
-    tc::fence_before();
-    __syncthreads();
+    if (!(ok = slot_ok())) break;
   }
   if (!ok) {
-    // a wait gave up: give the MMAs and X copies in flight one more bounded
+    // a wait gave up: give the MMAs and the X copy in flight one more bounded
     // wait before their TMEM and shared memory are released
     tc::mbar_wait(bar, phase ^ 1u, kWaitIters);
-    tc::mbar_wait(xbar, xph[0], kWaitIters);
-    tc::mbar_wait(xbar + 1, xph[1], kWaitIters);
+    if (x_out) tc::mbar_wait(xbar, xph, kWaitIters);
     tc::mbar_wait(wbar, 0, kWaitIters);
   }
+  tc::fence_before();
   __syncthreads();
-  if (warp == 0) tc::tmem_dealloc(tmem, kTmemCols);
+  tc::fence_after();
+  if (tid < 32) tc::tmem_dealloc(tmem, kTmemCols);
 }
 
 // ---------------------------------------------------------------- backward
@@ -851,8 +869,8 @@ int mlp_tc_build_x(int c0, int dpe, const float* k0rows, const int32_t* ray, con
 int mlp_tc_forward_rows(const float* w0, const float* b0, const float* w1, const float* b1,
                         const float* w2, const float* b2, int c0, int dpe, const float* k0rows,
                         const int32_t* ray, const float* pe, int pe_stride, const uint32_t* totals,
-                        int64_t max_rows, float* out, int out_logits, void** blob,
-                        size_t* blob_cap, void** xt, size_t* xt_cap, uint32_t* err,
+                        int64_t max_rows, float* out, const float* rw, void** blob, size_t* blob_cap,
+                        void** xt, size_t* xt_cap, uint32_t* err,
                         cudaStream_t st, int packed, int x_ready) {
   int rc = PVDB_OK;
   if (!packed && (rc = mlp_tc_pack(w0, b0, w1, b1, w2, b2, c0, dpe, blob, blob_cap, st)))
@@ -862,9 +880,9 @@ int mlp_tc_forward_rows(const float* w0, const float* b0, const float* w1, const
     return rc;
   MlpArgsTc a{w0, b0, w1, b1, w2, b2, c0, dpe, c0 + dpe};
   PVDB_SMEM_ATTR(k_mlp_fwd_tc, int(kSmFwdBytes));
-  launch_k(k_mlp_fwd_tc, 2 * num_sms(), kTcThreads, kSmFwdBytes, st, a,
+  launch_k(k_mlp_fwd_tc, num_sms(), kFwdThreads, kSmFwdBytes, st, a,
            static_cast<const uint8_t*>(*blob), static_cast<const uint8_t*>(*xt), totals, out,
-           out_logits, err);
+           rw, err);
   PVDB_CHECK_LAUNCH("k_mlp_fwd_tc");
   return PVDB_OK;
 }

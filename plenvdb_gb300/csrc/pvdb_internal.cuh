@@ -210,20 +210,41 @@ __device__ __forceinline__ void corner_delta(int c, int& di, int& dj, int& dk) {
 __device__ __forceinline__ int ifloor(float x) { return int(floorf(x)); }
 
 // Slots of the 8 trilinear corners of cell (i,j,k) in the reference's corner
-// order (see corner_delta), -1 where a corner lies in no allocated leaf. When
-// the cell does not cross a leaf face ((i|j|k) & 7 < 7 per axis) all corners
-// share one leaf: one table lookup, and the offsets follow from the voxel
-// layout (+64 x, +8 y, +1 z).
+// order (see corner_delta), -1 where a corner lies in no allocated leaf. The
+// leaf table is read once, and again only for the axes along which the cell
+// crosses a leaf face (offset 7): a third of the samples do, so nearly every
+// warp has some, and predicated loads cost those warps less than a second path
+// with eight full lookups. The offsets follow from the voxel layout (+64 x,
+// +8 y, +1 z; a crossing wraps its axis to 0).
 __device__ __forceinline__ void corner_slots(const GridView& g, int i, int j, int k, int s[8]) {
-  if ((i & 7) != 7 && (j & 7) != 7 && (k & 7) != 7) {
-    const int l = leaf_of(g, i, j, k);
-    const int b = l < 0 ? -1 : ((l << 9) | vox_offset(i, j, k));
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      int di, dj, dk;
-      corner_delta(c, di, dj, dk);
-      s[c] = b < 0 ? -1 : b + (di << 6) + (dj << 3) + dk;
-    }
+  const bool cx = (i & 7) == 7, cy = (j & 7) == 7, cz = (k & 7) == 7;
+  const int lx = i >> 3, ly = j >> 3, lz = k >> 3;
+  if ((unsigned)lx < (unsigned)(g.ldim[0] - int(cx)) &&
+      (unsigned)ly < (unsigned)(g.ldim[1] - int(cy)) &&
+      (unsigned)lz < (unsigned)(g.ldim[2] - int(cz))) {
+    const int sx = g.ldim[1] * g.ldim[2], sy = g.ldim[2];
+    const int32_t* t = g.table + (lx * g.ldim[1] + ly) * g.ldim[2] + lz;
+    const int l000 = __ldg(t);
+    int l001 = l000, l010 = l000, l100 = l000;
+    if (cz) l001 = __ldg(t + 1);
+    if (cy) l010 = __ldg(t + sy);
+    if (cx) l100 = __ldg(t + sx);
+    int l011 = cy ? l010 : l001, l101 = cx ? l100 : l001, l110 = cx ? l100 : l010;
+    if (cy && cz) l011 = __ldg(t + sy + 1);
+    if (cx && cz) l101 = __ldg(t + sx + 1);
+    if (cx && cy) l110 = __ldg(t + sx + sy);
+    int l111 = cx ? (cy ? l110 : l101) : l011;
+    if (cx && cy && cz) l111 = __ldg(t + sx + sy + 1);
+    const int o = vox_offset(i, j, k);
+    const int ox = o + (cx ? -448 : 64), dy = cy ? -56 : 8, dz = cz ? -7 : 1;
+    s[0] = l000 < 0 ? -1 : (l000 << 9) + o;
+    s[1] = l001 < 0 ? -1 : (l001 << 9) + o + dz;
+    s[2] = l011 < 0 ? -1 : (l011 << 9) + o + dy + dz;
+    s[3] = l010 < 0 ? -1 : (l010 << 9) + o + dy;
+    s[4] = l110 < 0 ? -1 : (l110 << 9) + ox + dy;
+    s[5] = l111 < 0 ? -1 : (l111 << 9) + ox + dy + dz;
+    s[6] = l101 < 0 ? -1 : (l101 << 9) + ox + dz;
+    s[7] = l100 < 0 ? -1 : (l100 << 9) + ox;
   } else {
 #pragma unroll
     for (int c = 0; c < 8; ++c) {

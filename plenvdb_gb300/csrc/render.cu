@@ -17,13 +17,14 @@
 //                          (renderer.cu:240-266); counts colour samples
 //   device scan            per-pixel row offsets
 //   k_render_march<FILL>   the same march, writing each colour sample's
-//                          distance, weight and pixel to its row
+//                          position, weight and pixel to its row
 //   k_render_pe / k_render_x (BF16), k_render_k0 (FP32)
 //                          per row: the trilinear features (renderer.cu:303-310)
 //                          into the rgbnet's X tiles or k0 rows
-//   rgbnet                 the MLP on all rows (PE part once per pixel)
-//   k_render_composite     per pixel: T*bg + sum_rows w/(1+exp(-logit)) in
-//                          sample order (final_render renderer.cu:112-119,
+//   rgbnet                 the MLP on all rows (PE part once per pixel), each
+//                          row's w/(1+exp(-logit))
+//   k_render_composite     per pixel: T*bg + the sum of its rows in sample
+//                          order (final_render renderer.cu:112-119,
 //                          deterministic instead of atomics); bg alone when the
 //                          pixel has no colour sample (renderer.cu:325-329).
 // The reference runs the march twice with slightly different float
@@ -47,7 +48,7 @@ struct MlpArgs {
 };
 int mlp_forward_rows(const MlpArgs& a, const float* k0rows, const int32_t* ray,
                      const float* viewdirs, int R, const uint32_t* need, const uint32_t* totals,
-                     int64_t max_rows, float* out, int out_logits, float* hpe_buf, int precision,
+                     int64_t max_rows, const float* rw, float* out, float* hpe_buf, int precision,
                      void** blob, size_t* blob_cap, void** xt, size_t* xt_cap, uint32_t* err,
                      cudaStream_t st);
 
@@ -61,6 +62,8 @@ struct RenderP {
   int dcol;
   // index store: nslots = nleaf * 512 voxel slots; record nslots of the
   // per-voxel arrays holds row 0
+  // (the leaf table holds -d for a block with no leaf, d the Chebyshev distance
+  // in blocks to the nearest leaf)
   GridView idx;               // topology; values unused
   int64_t nslots;
   const float* vden;          // [nslots + 1]
@@ -79,7 +82,7 @@ struct RenderW {
   float* viewdirs;   // [HW*3] (pixels with colour samples)
   float* rk0;        // [cap*dcol]
   float* rw;         // [cap]
-  float* rt;         // [cap] distance along the pixel's ray
+  float* rxyz;       // [cap*3] index-space position
   int32_t* rpix;     // [cap]
   int64_t cap;
 };
@@ -126,24 +129,62 @@ __device__ __forceinline__ void cell_corners(const RenderP& P, const float xyz[3
   corner_scales(xyz[0] - float(i), xyz[1] - float(j), xyz[2] - float(k), sc);
 }
 
-// One thread per pixel, 8 x 4 pixels a warp. Bound by instructions: most steps
-// of a ray lie in blocks of 8^3 voxels that no leaf covers, where every sample
-// is inactive. There the march only advances t (the same rounded additions, so
-// the later samples' positions are the same bits) until shortly before the
-// block's face, instead of testing each step: see the skip below.
+// kLanes lanes per pixel, each with one of the next kLanes samples: a sample's
+// lookups and its alpha are a chain of dependent loads and slow math, and with
+// one lane a pixel the march was bound by that chain (and by pixels of a warp
+// entering the scene at different steps). The lanes' alphas are then taken in
+// sample order. Where no leaf is near, the march only advances t (the same
+// rounded additions, so the later samples' positions are the same bits) until
+// shortly before the faces of the empty region.
+//
+// advance: t after n additions of step, each rounded. While t stays between
+// two powers of two its ulp u is fixed, so every addition adds the same
+// multiple of u, su = (t + step) - t, and m of them add m su exactly; the one
+// exception is a step whose remainder is exactly half an ulp (ties go to the
+// even neighbour), which takes the additions one by one, as does a t near the
+// next power of two.
+__device__ __forceinline__ float half_ulp(float t) {
+  return __uint_as_float((__float_as_uint(t) & 0x7F800000u) - (24u << 23));
+}
+__device__ __forceinline__ float next_pow2(float t) {
+  return __uint_as_float((__float_as_uint(t) & 0x7F800000u) + 0x00800000u);
+}
+__device__ __forceinline__ bool steps_exact(float t, float step, float su) {
+  return t > 1e-20f && t < 1e20f && su > 0.f && fabsf(step - su) != half_ulp(t);
+}
+__device__ __forceinline__ float advance(float t, float step, int n) {
+  while (n > 0) {
+    float t1 = __fadd_rn(t, step);
+    --n;
+    const float su = t1 - t;
+    if (n > 0 && steps_exact(t, step, su)) {
+      const float room = (next_pow2(t) - t1) / su * 0.999f - 1.f;
+      const int m = room < float(n) ? int(room) : n;
+      if (m > 0) {
+        t1 = __fmaf_rn(float(m), su, t1);
+        n -= m;
+      }
+    }
+    t = t1;
+  }
+  return t;
+}
+
+constexpr int kLanes = 8;
+constexpr int kTileW = 2, kTileH = 32 / kLanes / kTileW;  // pixels of a warp
+
 template <bool FILL>
 __global__ void __launch_bounds__(128)
     k_render_march(RenderP P, RenderW Wk) {
   const int warp = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  const int tiles_x = (P.W + 7) / 8;
-  const int px = (warp % tiles_x) * 8 + (lane & 7), py = (warp / tiles_x) * 4 + (lane >> 3);
-  if (px >= P.W || py >= P.H) return;
-  const int n = py * P.W + px;
-  uint32_t want = 0;
-  if (FILL) {
-    want = Wk.n[n];
-    if (want == 0) return;
-  }
+  const int j = lane & (kLanes - 1), g = lane / kLanes, first = lane & ~(kLanes - 1);
+  const int tiles_x = (P.W + kTileW - 1) / kTileW;
+  const int px = (warp % tiles_x) * kTileW + g % kTileW,
+            py = (warp / tiles_x) * kTileH + g / kTileW;
+  const bool in_image = px < P.W && py < P.H;
+  const int n = in_image ? py * P.W + px : 0;
+  const uint32_t want = FILL && in_image ? Wk.n[n] : 0;
+  const int64_t base = FILL ? int64_t(Wk.off[n]) : 0;
   PixelRay r;
   pixel_ray(P, n, r);
   const float steplen = r.steplen;
@@ -159,81 +200,130 @@ __global__ void __launch_bounds__(128)
   const float tmax = fmaxf(fminf(fminf(fminf(fmaxf(ax, bx), fmaxf(ay, by)), fmaxf(az, bz)), P.far_), P.near_);
   float T = 1.f;
   uint32_t cnt = 0;
-  const int64_t base = FILL ? int64_t(Wk.off[n]) : 0;
-  float t = tmin;
   // the reference loops while t < tmax; the iteration bound (the sample count
   // of the [tmin,tmax] chord plus slack) only guards against a step that no
   // longer advances t (non-finite or vanishing steplen)
   const float nsteps_f = (tmax - tmin) / steplen;
   const int max_it = (nsteps_f > 0.f && nsteps_f < 1e6f) ? int(nsteps_f) + 4 : 0;
-  // Skip: voxels advanced per step and its inverse per axis, and the most
-  // steps a skip may take: t's rounding (at most tmax 2^-23 per addition)
-  // stays below a quarter of a step
+  // skips: the inverse of the voxels advanced per step, and the most steps a
+  // skip may take: t's rounding (at most tmax 2^-23 per addition) stays below
+  // a quarter of a step
   float inv[3];
 #pragma unroll
   for (int a = 0; a < 3; ++a) inv[a] = 1.f / (r.d[a] * P.wsm1[a] * steplen);
   const float most = fminf(0.25f * steplen / (tmax * 1.2e-7f), 4096.f);
-  for (int it = 0; t < tmax && it < max_it; ++it) {
-    t = __fadd_rn(t, steplen);
-    float p[3];
-    for (int a = 0; a < 3; ++a) p[a] = __fmaf_rn(t, r.d[a], r.o[a]);
-    if ((0.f > p[0]) | (0.f > p[1]) | (0.f > p[2]) | (1.f < p[0]) | (1.f < p[1]) | (1.f < p[2]))
-      continue;
-    float xyz[3];
-    for (int a = 0; a < 3; ++a) xyz[a] = __fmul_rn(p[a], P.wsm1[a]);
-    const int ri = __float2int_rn(xyz[0]), rj = __float2int_rn(xyz[1]),
-              rk = __float2int_rn(xyz[2]);
-    const int leaf = leaf_of(P.idx, ri, rj, rk);
-    if (leaf < 0) {
-      // every sample whose rounded position stays in this block is inactive:
-      // the steps that keep it 0.01 voxel (above the rounding of xyz) and one
-      // step inside the faces at 8 b - 0.5 and 8 b + 7.5
-      float steps = most;
-      const int b[3] = {ri & ~7, rj & ~7, rk & ~7};
-#pragma unroll
-      for (int a = 0; a < 3; ++a) {
-        const float face = float(b[a]) + (inv[a] > 0.f ? 7.49f : -0.49f);
-        const float s = (face - xyz[a]) * inv[a];
-        if (s < steps) steps = s;  // (an axis that does not advance gives inf or NaN)
+  float t = tmin;  // of the last sample taken, `it` samples so far
+  int it = 0;
+  bool run = in_image && (!FILL || want > 0) && t < tmax && max_it > 0;
+  while (__any_sync(0xffffffffu, run)) {
+    // this lane's sample: j + 1 steps on
+    float tj, prev = t;
+    {
+      const float t1 = __fadd_rn(t, steplen), su = t1 - t;
+      if (steps_exact(t, steplen, su) && t1 + float(kLanes) * su < next_pow2(t)) {
+        tj = __fmaf_rn(float(j), su, t1);
+        if (j) prev = __fmaf_rn(float(j - 1), su, t1);
+      } else {
+        tj = t1;
+        for (int q = 1; q <= j; ++q) {
+          prev = tj;
+          tj = __fadd_rn(tj, steplen);
+        }
       }
-      const int skip = int(fmaxf(steps, 0.f)) - 1;
-      for (int q = 0; q < skip; ++q) t = __fadd_rn(t, steplen);
-      it += max(skip, 0);
-      continue;
     }
-    const int v = vox_offset(ri, rj, rk);
-    if (!((__ldg(P.idx.mask + leaf * 8 + (v >> 6)) >> (v & 63)) & 1ull)) continue;
-    int64_t slot[8];
-    float sc[8];
-    cell_corners(P, xyz, slot, sc);
-    float val[8];
+    bool kept = false;
+    float alpha = 0.f, xyz[3], skip_f = 0.f;
+    float p[3];
 #pragma unroll
-    for (int c = 0; c < 8; ++c) val[c] = __ldg(P.vden + slot[c]);
-    float sig = __fmul_rn(val[0], sc[0]);
+    for (int a = 0; a < 3; ++a) {
+      p[a] = __fmaf_rn(tj, r.d[a], r.o[a]);
+      xyz[a] = __fmul_rn(p[a], P.wsm1[a]);
+    }
+    if (run && prev < tmax && it + j < max_it &&
+        !((0.f > p[0]) | (0.f > p[1]) | (0.f > p[2]) | (1.f < p[0]) | (1.f < p[1]) |
+          (1.f < p[2]))) {
+      const int ri = __float2int_rn(xyz[0]), rj = __float2int_rn(xyz[1]),
+                rk = __float2int_rn(xyz[2]);
+      const int leaf = leaf_of(P.idx, ri, rj, rk);
+      if (leaf < 0) {
+        // every sample whose rounded position stays in the blocks nearer than
+        // the nearest leaf is inactive: the steps that keep it 0.01 voxel
+        // (above the rounding of xyz) and one step inside their outer faces
+        skip_f = most;
+        const int b[3] = {ri & ~7, rj & ~7, rk & ~7};
+        const float far = -8.f * float(leaf + 1);  // the further blocks, in voxels
 #pragma unroll
-    for (int c = 1; c < 8; ++c) sig = __fmaf_rn(val[c], sc[c], sig);
-    const float alpha = 1.f - powf(1.f + expf(sig + P.shift), -P.interval);
-    if (alpha <= P.thr) continue;
-    const float wt = T * alpha;
-    T = T * (1.f - alpha);
-    if (wt <= P.thr) continue;
-    if (FILL) {
-      const int64_t m = base + cnt;
+        for (int a = 0; a < 3; ++a) {
+          const float face = float(b[a]) + (inv[a] > 0.f ? 7.49f + far : -0.49f - far);
+          const float s = (face - xyz[a]) * inv[a];
+          if (s < skip_f) skip_f = s;  // (an axis that does not advance gives inf or NaN)
+        }
+      } else {
+        const int v = vox_offset(ri, rj, rk);
+        if ((__ldg(P.idx.mask + leaf * 8 + (v >> 6)) >> (v & 63)) & 1ull) {
+          int64_t slot[8];
+          float sc[8];
+          cell_corners(P, xyz, slot, sc);
+          float val[8];
+#pragma unroll
+          for (int c = 0; c < 8; ++c) val[c] = __ldg(P.vden + slot[c]);
+          float sig = __fmul_rn(val[0], sc[0]);
+#pragma unroll
+          for (int c = 1; c < 8; ++c) sig = __fmaf_rn(val[c], sc[c], sig);
+          alpha = 1.f - powf(1.f + expf(sig + P.shift), -P.interval);
+          kept = !(alpha <= P.thr);
+        }
+      }
+    }
+    // the kept samples in order (the same in every lane of the pixel)
+    unsigned rem = (__ballot_sync(0xffffffffu, kept) >> first) & ((1u << kLanes) - 1u);
+    float wt = 0.f;
+    uint32_t row = 0;
+    bool col = false;
+    while (__any_sync(0xffffffffu, rem != 0u)) {
+      const int q = rem ? __ffs(rem) - 1 : 0;
+      const float a = __shfl_sync(0xffffffffu, alpha, first + q);
+      if (rem) {
+        rem &= rem - 1;
+        const float w = T * a;
+        T = T * (1.f - a);
+        if (!(w <= P.thr)) {
+          if (j == q) {
+            wt = w;
+            row = cnt;
+            col = true;
+          }
+          ++cnt;
+          if (T < P.t_stop || (FILL && cnt == want)) {
+            rem = 0u;
+            run = false;
+          }
+        }
+      }
+    }
+    if (FILL && col) {
+      const int64_t m = base + row;
       if (m < Wk.cap) {
         Wk.rw[m] = wt;
-        Wk.rt[m] = t;
         Wk.rpix[m] = n;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) Wk.rxyz[m * 3 + a] = xyz[a];
       }
     }
-    ++cnt;
-    if (FILL && cnt == want) break;
-    if (T < P.t_stop) break;
+    t = __shfl_sync(0xffffffffu, tj, first + kLanes - 1);
+    it += kLanes;
+    const int skip = int(fmaxf(__shfl_sync(0xffffffffu, skip_f, first + kLanes - 1), 0.f)) - 1;
+    t = advance(t, steplen, skip);
+    it += max(skip, 0);
+    run = run && t < tmax && it < max_it;
   }
-  if (!FILL) {
-    Wk.n[n] = cnt;
-    Wk.T[n] = T;
-    if (cnt)
-      for (int a = 0; a < 3; ++a) Wk.viewdirs[n * 3 + a] = __fdiv_rn(r.rd[a], r.len);
+  if (!FILL && in_image) {
+    if (j == 0) {
+      Wk.n[n] = cnt;
+      Wk.T[n] = T;
+    }
+    if (cnt && j < 3)
+      Wk.viewdirs[n * 3 + j] = __fdiv_rn(j == 0 ? r.rd[0] : j == 1 ? r.rd[1] : r.rd[2], r.len);
   }
 }
 
@@ -243,13 +333,9 @@ __global__ void __launch_bounds__(128)
 // 0: any channel count up to 16, by row id.
 template <int CT>
 __device__ __forceinline__ void row_features(const RenderP& P, const RenderW& Wk, int64_t m,
-                                             int n, float* acc) {
-  PixelRay r;
-  pixel_ray(P, n, r);
-  const float t = Wk.rt[m];
-  float xyz[3];
-#pragma unroll
-  for (int a = 0; a < 3; ++a) xyz[a] = __fmul_rn(__fmaf_rn(t, r.d[a], r.o[a]), P.wsm1[a]);
+                                             float* acc) {
+  const float xyz[3] = {__ldg(Wk.rxyz + m * 3), __ldg(Wk.rxyz + m * 3 + 1),
+                        __ldg(Wk.rxyz + m * 3 + 2)};
   int64_t slot[8];
   float sc[8];
   cell_corners(P, xyz, slot, sc);
@@ -310,7 +396,7 @@ __global__ void __launch_bounds__(256)
   const int64_t m = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   if (m >= M) return;
   float acc[CT ? CT : 16];
-  row_features<CT>(P, Wk, m, Wk.rpix[m], acc);
+  row_features<CT>(P, Wk, m, acc);
   if (CT == 12) {
     float4* dst = reinterpret_cast<float4*>(Wk.rk0 + m * 12);
 #pragma unroll
@@ -370,7 +456,7 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
     for (int cb = CT == 12 ? 1 : 0; cb < 6; ++cb) row[cb] = __ldg(pex + int64_t(n) * 6 + cb);
     float acc[CT ? CT : 16];
-    row_features<CT>(P, Wk, m, n, acc);
+    row_features<CT>(P, Wk, m, acc);
     if (CT == 12) {
       row[0] = make_uint4(tc::pack_bf16(acc[0], acc[1]), tc::pack_bf16(acc[2], acc[3]),
                           tc::pack_bf16(acc[4], acc[5]), tc::pack_bf16(acc[6], acc[7]));
@@ -392,37 +478,28 @@ __global__ void __launch_bounds__(256)
     *reinterpret_cast<uint4*>(tile + tc::kmaj(int(m & 127), 8 * cb, kRgbXK)) = row[cb];
 }
 
-// One thread per pixel; the rows of a block's pixels are contiguous, so the
-// block forms their contributions w / (1 + exp(-logit)) together, a row a
-// thread, in chunks through shared memory, and each pixel then adds its own in
-// sample order.
-constexpr int kCompRows = 1024;
-__global__ void __launch_bounds__(256)
-    k_render_composite(RenderP P, RenderW Wk, const float* __restrict__ logits, float* image) {
-  __shared__ float part[kCompRows * 3];
-  const int HW = P.H * P.W;
-  const int n = blockIdx.x * 256 + threadIdx.x;
-  const int last = min(blockIdx.x * 256 + 255, HW - 1);
-  const int64_t b0 = Wk.off[blockIdx.x * 256];
-  const int64_t b1 = min(int64_t(Wk.off[last]) + Wk.n[last], Wk.cap);
-  const uint32_t cnt = n < HW ? Wk.n[n] : 0;
-  const int64_t off = n < HW ? Wk.off[n] : 0;
-  float acc[3];
-  acc[0] = acc[1] = acc[2] = n < HW && cnt ? __fmul_rn(Wk.T[n], P.bg) : P.bg;
-  for (int64_t c0 = b0; c0 < b1; c0 += kCompRows) {
-    const int nr = int(min(int64_t(kCompRows), b1 - c0));
-    for (int e = threadIdx.x; e < nr * 3; e += 256)
-      part[e] = __fdiv_rn(__ldg(Wk.rw + c0 + e / 3), 1.f + expf(-__ldg(logits + c0 * 3 + e)));
-    __syncthreads();
-    const int j0 = int(max(off, c0) - c0), j1 = int(min(off + cnt, c0 + nr) - c0);
-    for (int j = j0; j < j1; ++j)
+// One thread per pixel and channel adds the pixel's rows in sample order, eight
+// loads in flight (part [M, 3]: the rows' contributions).
+__global__ void __launch_bounds__(192)
+    k_render_composite(RenderP P, RenderW Wk, const float* __restrict__ part, float* image) {
+  const int64_t e = blockIdx.x * 192ll + threadIdx.x;
+  const int n = int(e / 3);
+  if (n >= P.H * P.W) return;
+  const uint32_t cnt = Wk.n[n];
+  float acc = P.bg;
+  if (cnt) {
+    acc = __fmul_rn(Wk.T[n], P.bg);
+    const float* src = part + int64_t(Wk.off[n]) * 3 + (e - 3ll * n);
+    for (uint32_t j0 = 0; j0 < cnt; j0 += 8) {
+      float v[8];
 #pragma unroll
-      for (int c = 0; c < 3; ++c) acc[c] = __fadd_rn(acc[c], part[3 * j + c]);
-    __syncthreads();
+      for (uint32_t q = 0; q < 8; ++q) v[q] = j0 + q < cnt ? __ldg(src + (j0 + q) * 3) : 0.f;
+#pragma unroll
+      for (uint32_t q = 0; q < 8; ++q)
+        if (j0 + q < cnt) acc = __fadd_rn(acc, v[q]);
+    }
   }
-  if (n >= HW) return;
-#pragma unroll
-  for (int c = 0; c < 3; ++c) image[n * 3 + c] = acc[c];
+  image[e] = acc;
 }
 
 // Per-voxel records of the leaves from the rows (row id rows[s]; slot
@@ -490,9 +567,9 @@ struct pvdb_renderer_s {
   size_t scan_partial_cap = 0;
   float* d_rk0 = nullptr;
   float* d_rw = nullptr;
-  float* d_rt = nullptr;
+  float* d_rxyz = nullptr;
   int32_t* d_rpix = nullptr;
-  float* d_logits = nullptr;
+  float* d_part = nullptr;
   int64_t rows_cap = 0;
   void* d_packed = nullptr;  // BF16 weight tiles of the tensor-core rgbnet
   size_t packed_cap = 0;
@@ -500,20 +577,50 @@ struct pvdb_renderer_s {
   size_t xt_cap = 0;
 };
 
+// The leaf table with -d in the blocks that have no leaf, d the Chebyshev
+// distance in blocks to the nearest one (two passes over half of the 26
+// neighbours each).
+static std::vector<int32_t> leaf_distances(const pvdb_grid_s* g) {
+  const int L[3] = {g->ldim[0], g->ldim[1], g->ldim[2]};
+  std::vector<int32_t> t = g->h_table;
+  const int32_t none = -(std::max(L[0], std::max(L[1], L[2])) + 1);
+  for (int32_t& v : t)
+    if (v < 0) v = none;
+  auto at = [&](int x, int y, int z) -> int32_t& { return t[(int64_t(x) * L[1] + y) * L[2] + z]; };
+  auto relax = [&](int x, int y, int z, int sign) {
+    int32_t& v = at(x, y, z);
+    if (v >= 0) return;
+    for (int q = 0; q < 13; ++q) {  // the neighbours before this one in the pass's order
+      const int dx = sign * (q / 9 - 1), dy = sign * (q / 3 % 3 - 1), dz = sign * (q % 3 - 1);
+      const int a = x + dx, b = y + dy, c = z + dz;
+      if (a < 0 || b < 0 || c < 0 || a >= L[0] || b >= L[1] || c >= L[2]) continue;
+      const int32_t w = at(a, b, c);
+      v = std::max(v, w >= 0 ? -1 : w - 1);
+    }
+  };
+  for (int x = 0; x < L[0]; ++x)
+    for (int y = 0; y < L[1]; ++y)
+      for (int z = 0; z < L[2]; ++z) relax(x, y, z, 1);
+  for (int x = L[0] - 1; x >= 0; --x)
+    for (int y = L[1] - 1; y >= 0; --y)
+      for (int z = L[2] - 1; z >= 0; --z) relax(x, y, z, -1);
+  return t;
+}
+
 static int renderer_grow_rows(pvdb_renderer_s* r, int64_t need) {
   if (need <= r->rows_cap) return PVDB_OK;
   const int64_t cap = std::max<int64_t>(need + need / 4, 1 << 20);
-  void* ptrs[] = {r->d_rk0, r->d_rw, r->d_rt, r->d_rpix, r->d_logits};
+  void* ptrs[] = {r->d_rk0, r->d_rw, r->d_rxyz, r->d_rpix, r->d_part};
   for (void* p : ptrs) dev_free(p);
-  r->d_rk0 = r->d_rw = r->d_rt = r->d_logits = nullptr;
+  r->d_rk0 = r->d_rw = r->d_rxyz = r->d_part = nullptr;
   r->d_rpix = nullptr;
   r->rows_cap = 0;
   int rc;
   if ((rc = dev_alloc((void**)&r->d_rk0, size_t(cap) * r->dcol * 4)) ||
       (rc = dev_alloc((void**)&r->d_rw, size_t(cap) * 4)) ||
-      (rc = dev_alloc((void**)&r->d_rt, size_t(cap) * 4)) ||
+      (rc = dev_alloc((void**)&r->d_rxyz, size_t(cap) * 12)) ||
       (rc = dev_alloc((void**)&r->d_rpix, size_t(cap) * 4)) ||
-      (rc = dev_alloc((void**)&r->d_logits, size_t(cap) * 12)))
+      (rc = dev_alloc((void**)&r->d_part, size_t(cap) * 12)))
     return rc;
   r->rows_cap = cap;
   return PVDB_OK;
@@ -551,7 +658,7 @@ int pvdb_renderer_destroy(pvdb_renderer r) {
   pvdb_grid_destroy(r->topo);
   void* ptrs[] = {r->d_rows, r->d_vden, r->d_col, r->d_colh, r->d_params, r->d_n, r->d_off,
                   r->d_T, r->d_viewdirs, r->d_hpe, r->d_image, r->d_totals, r->scan_partial,
-                  r->d_rk0, r->d_rw, r->d_rt, r->d_rpix, r->d_logits, r->d_packed, r->d_xt};
+                  r->d_rk0, r->d_rw, r->d_rxyz, r->d_rpix, r->d_part, r->d_packed, r->d_xt};
   for (void* p : ptrs) dev_free(p);
   delete r;
   return PVDB_OK;
@@ -582,6 +689,11 @@ int pvdb_renderer_load_data(pvdb_renderer r, const int32_t reso[3], const int32_
   r->flags[0] = false;  // until everything below is in place
   int rc = pvdb_grid_create_from_mask(reso, 1, 0.f, active.data(), PVDB_MEM_HOST, &r->topo);
   if (rc) return rc;
+  {
+    const std::vector<int32_t> table = leaf_distances(r->topo);
+    PVDB_CHECK_CUDA(cudaMemcpy(r->topo->d_table, table.data(), table.size() * 4,
+                               cudaMemcpyHostToDevice));
+  }
   dev_free(r->d_rows);
   dev_free(r->d_vden);
   dev_free(r->d_col);
@@ -775,8 +887,8 @@ int pvdb_renderer_render(pvdb_renderer r, int32_t precision, pvdb_stream s) {
   const int HW = r->H * r->W;
   prof_begin_call();
   prof_mark(st, 0);
-  // 4 warps a block, 8 x 4 pixels a warp
-  const int march_grid = ceil_div(int64_t(ceil_div(r->W, 8)) * ceil_div(r->H, 4), 4);
+  // 4 warps a block
+  const int march_grid = ceil_div(int64_t(ceil_div(r->W, kTileW)) * ceil_div(r->H, kTileH), 4);
   k_render_march<false><<<march_grid, 128, 0, st>>>(P, Wk);
   PVDB_CHECK_LAUNCH("k_render_march<count>");
   prof_mark(st, 1);
@@ -791,7 +903,7 @@ int pvdb_renderer_render(pvdb_renderer r, int32_t precision, pvdb_stream s) {
   if (rc) return rc;
   Wk.rk0 = r->d_rk0;
   Wk.rw = r->d_rw;
-  Wk.rt = r->d_rt;
+  Wk.rxyz = r->d_rxyz;
   Wk.rpix = r->d_rpix;
   Wk.cap = r->rows_cap;
   MlpArgs a;
@@ -833,12 +945,13 @@ int pvdb_renderer_render(pvdb_renderer r, int32_t precision, pvdb_stream s) {
   prof_mark(st, 3);
   if (total) {
     rc = mlp_forward_rows(a, r->d_rk0, r->d_rpix, r->d_viewdirs, HW, r->d_n, r->d_totals,
-                          r->rows_cap, r->d_logits, 1, r->d_hpe, precision, &r->d_packed,
+                          r->rows_cap, r->d_rw, r->d_part, r->d_hpe, precision, &r->d_packed,
                           &r->packed_cap, &r->d_xt, &r->xt_cap, r->d_totals + 3, st);
     if (rc) return rc;
   }
   prof_mark(st, 4);
-  k_render_composite<<<ceil_div(HW, 256), 256, 0, st>>>(P, Wk, r->d_logits, r->d_image);
+  k_render_composite<<<ceil_div(int64_t(HW) * 3, 192), 192, 0, st>>>(P, Wk, r->d_part,
+                                                                     r->d_image);
   PVDB_CHECK_LAUNCH("k_render_composite");
   prof_mark(st, 5);
   return PVDB_OK;
