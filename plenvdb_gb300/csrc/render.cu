@@ -8,16 +8,14 @@
 // load at its slot, not a row id and a load behind it.
 //
 // Per frame:
-//   k_render_march<COUNT>  one thread per pixel: get_rays (renderer.cu:122-167)
+//   k_render_march         a warp per 32 pixels: get_rays (renderer.cu:122-167)
 //                          in the unit-cube frame, t += steplen before each
 //                          sample, skip when isActive(rint(xyz)) is false,
 //                          index-grid trilinear density (int() truncation,
 //                          renderer.cu:271-300), raw2alpha, both thresholds,
 //                          early stop at a colour sample once T < t_stop
-//                          (renderer.cu:240-266); counts colour samples
-//   device scan            per-pixel row offsets
-//   k_render_march<FILL>   the same march, writing each colour sample's
-//                          position, weight and pixel to its row
+//                          (renderer.cu:240-266); appends each colour sample's
+//                          position, weight and pixel to the frame's rows
 //   k_render_pe / k_render_x (BF16), k_render_k0 (FP32)
 //                          per row: the trilinear features (renderer.cu:303-310)
 //                          into the rgbnet's X tiles or k0 rows
@@ -27,9 +25,12 @@
 //                          order (final_render renderer.cu:112-119,
 //                          deterministic instead of atomics); bg alone when the
 //                          pixel has no colour sample (renderer.cu:325-329).
-// The reference runs the march twice with slightly different float
-// associations in the two passes; here both passes share one code path, so the
-// fill pass reproduces the count pass exactly.
+// The reference marches twice, counting the samples first. Here the rows need
+// no order among the pixels: a warp takes rows from a counter for every batch
+// of samples it has finished and links its batches, and the composite walks
+// them. Where a row lies varies from run to run; its value and the order a
+// pixel's rows are added in do not. A frame with more rows than the buffers
+// hold is marched again after they have grown.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -75,10 +76,20 @@ struct RenderP {
   int storage;
 };
 
+// The colour samples one warp of the march finished together.
+struct RenderBatch {
+  uint32_t row0;    // first row; pixel l's rows follow those of the pixels before it
+  int32_t next;     // the warp's next batch, -1: none
+  uint8_t cnt[32];  // rows per pixel of the warp
+};
+
 struct RenderW {
   uint32_t* n;       // [HW] colour samples per pixel
-  uint32_t* off;     // [HW]
   float* T;          // [HW]
+  uint32_t* totals;  // [1] rows, [2] batches
+  int32_t* head;     // [warps] first batch of each warp, -1: none
+  RenderBatch* batch;  // [bcap]
+  int64_t bcap;
   float* viewdirs;   // [HW*3] (pixels with colour samples)
   float* rk0;        // [cap*dcol]
   float* rw;         // [cap]
@@ -129,14 +140,6 @@ __device__ __forceinline__ void cell_corners(const RenderP& P, const float xyz[3
   corner_scales(xyz[0] - float(i), xyz[1] - float(j), xyz[2] - float(k), sc);
 }
 
-// kLanes lanes per pixel, each with one of the next kLanes samples: a sample's
-// lookups and its alpha are a chain of dependent loads and slow math, and with
-// one lane a pixel the march was bound by that chain (and by pixels of a warp
-// entering the scene at different steps). The lanes' alphas are then taken in
-// sample order. Where no leaf is near, the march only advances t (the same
-// rounded additions, so the later samples' positions are the same bits) until
-// shortly before the faces of the empty region.
-//
 // advance: t after n additions of step, each rounded. While t stays between
 // two powers of two its ulp u is fixed, so every addition adds the same
 // multiple of u, su = (t + step) - t, and m of them add m su exactly; the one
@@ -170,21 +173,37 @@ __device__ __forceinline__ float advance(float t, float step, int n) {
   return t;
 }
 
-constexpr int kLanes = 8;
-constexpr int kTileW = 2, kTileH = 32 / kLanes / kTileW;  // pixels of a warp
+// A warp marches 8 x 4 pixels. Of a ray's samples, few are active (17 of 295 on
+// the 160^3 benchmark scene), and an active one costs several times the test of
+// an inactive one, so the two are kept apart: each lane tests its own pixel's
+// samples and lists up to kListed active ones; the warp then evaluates the
+// listed samples of all its pixels, a sample a lane; and each lane takes its
+// alphas in order. Where no leaf is near, the march only advances t until
+// shortly before the faces of the empty region.
+// (One lane a pixel evaluating samples as it met them, and eight lanes a pixel,
+// both took 600 us on the 800x800 benchmark frame.)
+constexpr int kListed = 16;
+constexpr int kTileW = 8, kTileH = 4;
+constexpr uint8_t kNoRow = 255;
 
-template <bool FILL>
+struct MarchList {
+  float t[kListed][32];
+  float alpha[kListed][32];    // then the weight
+  uint8_t rank[kListed][32];   // row within the pixel's rows of the batch
+  uint16_t entry[kListed * 32];  // 32 * index + lane of the e-th listed sample
+};
+
 __global__ void __launch_bounds__(128)
     k_render_march(RenderP P, RenderW Wk) {
+  __shared__ MarchList lists[4];
+  MarchList& L = lists[threadIdx.x >> 5];
   const int warp = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  const int j = lane & (kLanes - 1), g = lane / kLanes, first = lane & ~(kLanes - 1);
-  const int tiles_x = (P.W + kTileW - 1) / kTileW;
-  const int px = (warp % tiles_x) * kTileW + g % kTileW,
-            py = (warp / tiles_x) * kTileH + g / kTileW;
+  const int tiles_x = (P.W + kTileW - 1) / kTileW, tiles = tiles_x * ((P.H + kTileH - 1) / kTileH);
+  if (warp >= tiles) return;
+  const int px = (warp % tiles_x) * kTileW + lane % kTileW,
+            py = (warp / tiles_x) * kTileH + lane / kTileW;
   const bool in_image = px < P.W && py < P.H;
   const int n = in_image ? py * P.W + px : 0;
-  const uint32_t want = FILL && in_image ? Wk.n[n] : 0;
-  const int64_t base = FILL ? int64_t(Wk.off[n]) : 0;
   PixelRay r;
   pixel_ray(P, n, r);
   const float steplen = r.steplen;
@@ -198,13 +217,12 @@ __global__ void __launch_bounds__(128)
               bz = __fdiv_rn(-r.o[2], vz);
   const float tmin = fmaxf(fminf(fmaxf(fmaxf(fminf(ax, bx), fminf(ay, by)), fminf(az, bz)), P.far_), P.near_);
   const float tmax = fmaxf(fminf(fminf(fminf(fmaxf(ax, bx), fmaxf(ay, by)), fmaxf(az, bz)), P.far_), P.near_);
-  float T = 1.f;
-  uint32_t cnt = 0;
   // the reference loops while t < tmax; the iteration bound (the sample count
   // of the [tmin,tmax] chord plus slack) only guards against a step that no
   // longer advances t (non-finite or vanishing steplen)
   const float nsteps_f = (tmax - tmin) / steplen;
-  const int max_it = (nsteps_f > 0.f && nsteps_f < 1e6f) ? int(nsteps_f) + 4 : 0;
+  const int max_it =
+      in_image && nsteps_f > 0.f && nsteps_f < 1e6f ? int(nsteps_f) + 4 : 0;
   // skips: the inverse of the voxels advanced per step, and the most steps a
   // skip may take: t's rounding (at most tmax 2^-23 per addition) stays below
   // a quarter of a step
@@ -212,36 +230,26 @@ __global__ void __launch_bounds__(128)
 #pragma unroll
   for (int a = 0; a < 3; ++a) inv[a] = 1.f / (r.d[a] * P.wsm1[a] * steplen);
   const float most = fminf(0.25f * steplen / (tmax * 1.2e-7f), 4096.f);
-  float t = tmin;  // of the last sample taken, `it` samples so far
+  float T = 1.f;
+  uint32_t cnt = 0;
+  float t = tmin;
   int it = 0;
-  bool run = in_image && (!FILL || want > 0) && t < tmax && max_it > 0;
-  while (__any_sync(0xffffffffu, run)) {
-    // this lane's sample: j + 1 steps on
-    float tj, prev = t;
-    {
-      const float t1 = __fadd_rn(t, steplen), su = t1 - t;
-      if (steps_exact(t, steplen, su) && t1 + float(kLanes) * su < next_pow2(t)) {
-        tj = __fmaf_rn(float(j), su, t1);
-        if (j) prev = __fmaf_rn(float(j - 1), su, t1);
-      } else {
-        tj = t1;
-        for (int q = 1; q <= j; ++q) {
-          prev = tj;
-          tj = __fadd_rn(tj, steplen);
-        }
-      }
-    }
-    bool kept = false;
-    float alpha = 0.f, xyz[3], skip_f = 0.f;
-    float p[3];
+  int32_t last = -1;  // the warp's last batch
+  bool stop = false;
+  for (;;) {
+    // this pixel's next active samples
+    int c = 0;
+    while (c < kListed && !stop && t < tmax && it < max_it) {
+      t = __fadd_rn(t, steplen);
+      ++it;
+      float p[3], xyz[3];
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      p[a] = __fmaf_rn(tj, r.d[a], r.o[a]);
-      xyz[a] = __fmul_rn(p[a], P.wsm1[a]);
-    }
-    if (run && prev < tmax && it + j < max_it &&
-        !((0.f > p[0]) | (0.f > p[1]) | (0.f > p[2]) | (1.f < p[0]) | (1.f < p[1]) |
-          (1.f < p[2]))) {
+      for (int a = 0; a < 3; ++a) {
+        p[a] = __fmaf_rn(t, r.d[a], r.o[a]);
+        xyz[a] = __fmul_rn(p[a], P.wsm1[a]);
+      }
+      if ((0.f > p[0]) | (0.f > p[1]) | (0.f > p[2]) | (1.f < p[0]) | (1.f < p[1]) | (1.f < p[2]))
+        continue;
       const int ri = __float2int_rn(xyz[0]), rj = __float2int_rn(xyz[1]),
                 rk = __float2int_rn(xyz[2]);
       const int leaf = leaf_of(P.idx, ri, rj, rk);
@@ -249,81 +257,134 @@ __global__ void __launch_bounds__(128)
         // every sample whose rounded position stays in the blocks nearer than
         // the nearest leaf is inactive: the steps that keep it 0.01 voxel
         // (above the rounding of xyz) and one step inside their outer faces
-        skip_f = most;
+        float steps = most;
         const int b[3] = {ri & ~7, rj & ~7, rk & ~7};
-        const float far = -8.f * float(leaf + 1);  // the further blocks, in voxels
+        const float out = -8.f * float(leaf + 1);  // the further blocks, in voxels
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
-          const float face = float(b[a]) + (inv[a] > 0.f ? 7.49f + far : -0.49f - far);
+          const float face = float(b[a]) + (inv[a] > 0.f ? 7.49f + out : -0.49f - out);
           const float s = (face - xyz[a]) * inv[a];
-          if (s < skip_f) skip_f = s;  // (an axis that does not advance gives inf or NaN)
+          if (s < steps) steps = s;  // (an axis that does not advance gives inf or NaN)
         }
-      } else {
-        const int v = vox_offset(ri, rj, rk);
-        if ((__ldg(P.idx.mask + leaf * 8 + (v >> 6)) >> (v & 63)) & 1ull) {
-          int64_t slot[8];
-          float sc[8];
-          cell_corners(P, xyz, slot, sc);
-          float val[8];
-#pragma unroll
-          for (int c = 0; c < 8; ++c) val[c] = __ldg(P.vden + slot[c]);
-          float sig = __fmul_rn(val[0], sc[0]);
-#pragma unroll
-          for (int c = 1; c < 8; ++c) sig = __fmaf_rn(val[c], sc[c], sig);
-          alpha = 1.f - powf(1.f + expf(sig + P.shift), -P.interval);
-          kept = !(alpha <= P.thr);
-        }
+        const int skip = int(fmaxf(steps, 0.f)) - 1;
+        t = advance(t, steplen, skip);
+        it += max(skip, 0);
+        continue;
       }
+      const int v = vox_offset(ri, rj, rk);
+      if (!((__ldg(P.idx.mask + leaf * 8 + (v >> 6)) >> (v & 63)) & 1ull)) continue;
+      L.t[c][lane] = t;
+      ++c;
     }
-    // the kept samples in order (the same in every lane of the pixel)
-    unsigned rem = (__ballot_sync(0xffffffffu, kept) >> first) & ((1u << kLanes) - 1u);
-    float wt = 0.f;
-    uint32_t row = 0;
-    bool col = false;
-    while (__any_sync(0xffffffffu, rem != 0u)) {
-      const int q = rem ? __ffs(rem) - 1 : 0;
-      const float a = __shfl_sync(0xffffffffu, alpha, first + q);
-      if (rem) {
-        rem &= rem - 1;
-        const float w = T * a;
-        T = T * (1.f - a);
+    // the listed samples of all pixels, pixel after pixel
+    int end = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int x = __shfl_up_sync(0xffffffffu, end, o);
+      if (lane >= o) end += x;
+    }
+    const int total = __shfl_sync(0xffffffffu, end, 31);
+    if (total == 0) break;  // every pixel is done
+    for (int i = 0; i < c; ++i) L.entry[end - c + i] = uint16_t(32 * i + lane);
+    __syncwarp();
+    for (int e0 = 0; e0 < total; e0 += 32) {
+      const int e = e0 + lane;
+      const int en = L.entry[min(e, total - 1)], i = en >> 5, l = en & 31;
+      const float dx = __shfl_sync(0xffffffffu, r.d[0], l),
+                  dy = __shfl_sync(0xffffffffu, r.d[1], l),
+                  dz = __shfl_sync(0xffffffffu, r.d[2], l);
+      const float te = L.t[i][l];
+      const float xyz[3] = {__fmul_rn(__fmaf_rn(te, dx, r.o[0]), P.wsm1[0]),
+                            __fmul_rn(__fmaf_rn(te, dy, r.o[1]), P.wsm1[1]),
+                            __fmul_rn(__fmaf_rn(te, dz, r.o[2]), P.wsm1[2])};
+      int64_t slot[8];
+      float sc[8];
+      cell_corners(P, xyz, slot, sc);
+      float val[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) val[q] = __ldg(P.vden + slot[q]);
+      float sig = __fmul_rn(val[0], sc[0]);
+#pragma unroll
+      for (int q = 1; q < 8; ++q) sig = __fmaf_rn(val[q], sc[q], sig);
+      const float alpha = 1.f - powf(1.f + expf(sig + P.shift), -P.interval);
+      if (e < total) L.alpha[i][l] = alpha;
+    }
+    __syncwarp();
+    // each pixel's samples in order
+    int k = 0;
+    for (int i = 0; i < c; ++i) {
+      uint8_t rank = kNoRow;
+      const float alpha = L.alpha[i][lane];
+      if (!stop && !(alpha <= P.thr)) {
+        const float w = T * alpha;
+        T = T * (1.f - alpha);
         if (!(w <= P.thr)) {
-          if (j == q) {
-            wt = w;
-            row = cnt;
-            col = true;
-          }
-          ++cnt;
-          if (T < P.t_stop || (FILL && cnt == want)) {
-            rem = 0u;
-            run = false;
-          }
+          L.alpha[i][lane] = w;
+          rank = uint8_t(k++);
+          stop = T < P.t_stop;
         }
       }
+      L.rank[i][lane] = rank;
     }
-    if (FILL && col) {
-      const int64_t m = base + row;
-      if (m < Wk.cap) {
-        Wk.rw[m] = wt;
-        Wk.rpix[m] = n;
+    cnt += k;
+    // rows for the colour samples
+    int kend = k;
 #pragma unroll
-        for (int a = 0; a < 3; ++a) Wk.rxyz[m * 3 + a] = xyz[a];
+    for (int o = 1; o < 32; o <<= 1) {
+      const int x = __shfl_up_sync(0xffffffffu, kend, o);
+      if (lane >= o) kend += x;
+    }
+    const int rows = __shfl_sync(0xffffffffu, kend, 31);
+    if (rows == 0) continue;
+    uint32_t row0 = 0, id = 0;
+    if (lane == 0) {
+      row0 = atomicAdd(Wk.totals + 1, uint32_t(rows));
+      id = atomicAdd(Wk.totals + 2, 1u);
+    }
+    row0 = __shfl_sync(0xffffffffu, row0, 0);
+    id = __shfl_sync(0xffffffffu, id, 0);
+    if (id < Wk.bcap) {
+      RenderBatch& B = Wk.batch[id];
+      B.cnt[lane] = uint8_t(k);
+      if (lane == 0) {
+        B.row0 = row0;
+        B.next = -1;
+        if (last >= 0)
+          Wk.batch[last].next = int32_t(id);
+        else
+          Wk.head[warp] = int32_t(id);
+        last = int32_t(id);
       }
     }
-    t = __shfl_sync(0xffffffffu, tj, first + kLanes - 1);
-    it += kLanes;
-    const int skip = int(fmaxf(__shfl_sync(0xffffffffu, skip_f, first + kLanes - 1), 0.f)) - 1;
-    t = advance(t, steplen, skip);
-    it += max(skip, 0);
-    run = run && t < tmax && it < max_it;
-  }
-  if (!FILL && in_image) {
-    if (j == 0) {
-      Wk.n[n] = cnt;
-      Wk.T[n] = T;
+    __syncwarp();
+    const int64_t m0 = int64_t(row0) + kend - k;  // this pixel's first row
+    for (int e0 = 0; e0 < total; e0 += 32) {
+      const int e = e0 + lane;
+      const int en = L.entry[min(e, total - 1)], i = en >> 5, l = en & 31;
+      const int64_t ml = __shfl_sync(0xffffffffu, m0, l);
+      const float dx = __shfl_sync(0xffffffffu, r.d[0], l),
+                  dy = __shfl_sync(0xffffffffu, r.d[1], l),
+                  dz = __shfl_sync(0xffffffffu, r.d[2], l);
+      const int nl = __shfl_sync(0xffffffffu, n, l);
+      const uint8_t rank = L.rank[i][l];
+      const int64_t m = ml + rank;
+      if (e >= total || rank == kNoRow || m >= Wk.cap) continue;
+      const float te = L.t[i][l];
+      Wk.rw[m] = L.alpha[i][l];
+      Wk.rpix[m] = nl;
+      Wk.rxyz[m * 3] = __fmul_rn(__fmaf_rn(te, dx, r.o[0]), P.wsm1[0]);
+      Wk.rxyz[m * 3 + 1] = __fmul_rn(__fmaf_rn(te, dy, r.o[1]), P.wsm1[1]);
+      Wk.rxyz[m * 3 + 2] = __fmul_rn(__fmaf_rn(te, dz, r.o[2]), P.wsm1[2]);
     }
-    if (cnt && j < 3)
-      Wk.viewdirs[n * 3 + j] = __fdiv_rn(j == 0 ? r.rd[0] : j == 1 ? r.rd[1] : r.rd[2], r.len);
+    __syncwarp();
+  }
+  if (lane == 0 && last < 0) Wk.head[warp] = -1;
+  if (in_image) {
+    Wk.n[n] = cnt;
+    Wk.T[n] = T;
+    if (cnt)
+#pragma unroll
+      for (int a = 0; a < 3; ++a) Wk.viewdirs[n * 3 + a] = __fdiv_rn(r.rd[a], r.len);
   }
 }
 
@@ -478,28 +539,60 @@ __global__ void __launch_bounds__(256)
     *reinterpret_cast<uint4*>(tile + tc::kmaj(int(m & 127), 8 * cb, kRgbXK)) = row[cb];
 }
 
-// One thread per pixel and channel adds the pixel's rows in sample order, eight
-// loads in flight (part [M, 3]: the rows' contributions).
-__global__ void __launch_bounds__(192)
+// A warp per warp of the march, a lane per pixel: adds the pixel's rows batch
+// after batch, in sample order (part [M, 3]: the rows' contributions). Bound by
+// the chain batch header -> rows -> next batch: the next header travels while a
+// batch's rows, loaded together, are added.
+__global__ void __launch_bounds__(128)
     k_render_composite(RenderP P, RenderW Wk, const float* __restrict__ part, float* image) {
-  const int64_t e = blockIdx.x * 192ll + threadIdx.x;
-  const int n = int(e / 3);
-  if (n >= P.H * P.W) return;
-  const uint32_t cnt = Wk.n[n];
-  float acc = P.bg;
-  if (cnt) {
-    acc = __fmul_rn(Wk.T[n], P.bg);
-    const float* src = part + int64_t(Wk.off[n]) * 3 + (e - 3ll * n);
-    for (uint32_t j0 = 0; j0 < cnt; j0 += 8) {
-      float v[8];
-#pragma unroll
-      for (uint32_t q = 0; q < 8; ++q) v[q] = j0 + q < cnt ? __ldg(src + (j0 + q) * 3) : 0.f;
-#pragma unroll
-      for (uint32_t q = 0; q < 8; ++q)
-        if (j0 + q < cnt) acc = __fadd_rn(acc, v[q]);
-    }
+  const int warp = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int tiles_x = (P.W + kTileW - 1) / kTileW, tiles = tiles_x * ((P.H + kTileH - 1) / kTileH);
+  if (warp >= tiles) return;
+  const int px = (warp % tiles_x) * kTileW + lane % kTileW,
+            py = (warp / tiles_x) * kTileH + lane / kTileW;
+  const bool in_image = px < P.W && py < P.H;
+  const int64_t n = in_image ? int64_t(py) * P.W + px : 0;
+  int32_t b = Wk.head[warp];
+  float acc[3];
+  acc[0] = acc[1] = acc[2] = in_image && Wk.n[n] ? __fmul_rn(Wk.T[n], P.bg) : P.bg;
+  uint32_t cnt = 0, row0 = 0;
+  int32_t next = -1;
+  if (b >= 0) {
+    cnt = Wk.batch[b].cnt[lane];
+    row0 = Wk.batch[b].row0;
+    next = Wk.batch[b].next;
   }
-  image[e] = acc;
+  while (b >= 0) {
+    uint32_t cnt_n = 0, row0_n = 0;
+    int32_t next_n = -1;
+    if (next >= 0) {
+      cnt_n = Wk.batch[next].cnt[lane];
+      row0_n = Wk.batch[next].row0;
+      next_n = Wk.batch[next].next;
+    }
+    uint32_t end = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t x = __shfl_up_sync(0xffffffffu, end, o);
+      if (lane >= o) end += x;
+    }
+    const float* src = part + (int64_t(row0) + end - cnt) * 3;
+    float v[kListed * 3];
+#pragma unroll
+    for (uint32_t q = 0; q < kListed * 3; ++q) v[q] = q < cnt * 3 ? __ldg(src + q) : 0.f;
+#pragma unroll
+    for (uint32_t q = 0; q < kListed; ++q)
+      if (q < cnt)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) acc[c] = __fadd_rn(acc[c], v[3 * q + c]);
+    b = next;
+    cnt = cnt_n;
+    row0 = row0_n;
+    next = next_n;
+  }
+  if (in_image)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) image[n * 3 + c] = acc[c];
 }
 
 // Per-voxel records of the leaves from the rows (row id rows[s]; slot
@@ -557,14 +650,14 @@ struct pvdb_renderer_s {
   float c2w[16];
   // frame buffers
   uint32_t* d_n = nullptr;
-  uint32_t* d_off = nullptr;
+  int32_t* d_head = nullptr;
+  RenderBatch* d_batch = nullptr;
+  int64_t batch_cap = 0;
   float* d_T = nullptr;
   float* d_viewdirs = nullptr;
   float* d_hpe = nullptr;
   float* d_image = nullptr;
   uint32_t* d_totals = nullptr;
-  uint32_t* scan_partial = nullptr;
-  size_t scan_partial_cap = 0;
   float* d_rk0 = nullptr;
   float* d_rw = nullptr;
   float* d_rxyz = nullptr;
@@ -576,6 +669,17 @@ struct pvdb_renderer_s {
   void* d_xt = nullptr;      // BF16 X tiles of the rows (tensor-core rgbnet)
   size_t xt_cap = 0;
 };
+
+static int renderer_grow_batches(pvdb_renderer_s* r, int64_t need) {
+  if (need <= r->batch_cap) return PVDB_OK;
+  const int64_t cap = need + need / 4 + 4096;
+  dev_free(r->d_batch);
+  r->d_batch = nullptr;
+  r->batch_cap = 0;
+  const int rc = dev_alloc((void**)&r->d_batch, size_t(cap) * sizeof(RenderBatch));
+  if (!rc) r->batch_cap = cap;
+  return rc;
+}
 
 // The leaf table with -d in the blocks that have no leaf, d the Chebyshev
 // distance in blocks to the nearest one (two passes over half of the 26
@@ -656,8 +760,8 @@ int pvdb_renderer_create(int32_t dcol, int32_t dpe, int32_t dhid, int32_t dout,
 int pvdb_renderer_destroy(pvdb_renderer r) {
   if (!r) return PVDB_OK;
   pvdb_grid_destroy(r->topo);
-  void* ptrs[] = {r->d_rows, r->d_vden, r->d_col, r->d_colh, r->d_params, r->d_n, r->d_off,
-                  r->d_T, r->d_viewdirs, r->d_hpe, r->d_image, r->d_totals, r->scan_partial,
+  void* ptrs[] = {r->d_rows, r->d_vden, r->d_col, r->d_colh, r->d_params, r->d_n, r->d_head,
+                  r->d_T, r->d_viewdirs, r->d_hpe, r->d_image, r->d_totals, r->d_batch,
                   r->d_rk0, r->d_rw, r->d_rxyz, r->d_rpix, r->d_part, r->d_packed, r->d_xt};
   for (void* p : ptrs) dev_free(p);
   delete r;
@@ -812,12 +916,14 @@ int pvdb_renderer_set_kwargs(pvdb_renderer r, float near_, float far_, float ste
   r->t_stop = t_stop;
   if (h != r->H || w != r->W || !r->d_n) {
     const size_t HW = size_t(h) * w;
-    void* ptrs[] = {r->d_n, r->d_off, r->d_T, r->d_viewdirs, r->d_hpe, r->d_image};
+    void* ptrs[] = {r->d_n, r->d_head, r->d_T, r->d_viewdirs, r->d_hpe, r->d_image};
     for (void* p : ptrs) dev_free(p);
-    r->d_n = r->d_off = nullptr;
+    r->d_n = nullptr;
+    r->d_head = nullptr;
     r->d_T = r->d_viewdirs = r->d_hpe = r->d_image = nullptr;
     int rc;
-    if ((rc = dev_alloc((void**)&r->d_n, HW * 4)) || (rc = dev_alloc((void**)&r->d_off, HW * 4)) ||
+    if ((rc = dev_alloc((void**)&r->d_n, HW * 4)) || (rc = dev_alloc((void**)&r->d_head,
+                        size_t(ceil_div(w, kTileW)) * ceil_div(h, kTileH) * 4)) ||
         (rc = dev_alloc((void**)&r->d_T, HW * 4)) ||
         (rc = dev_alloc((void**)&r->d_viewdirs, HW * 12)) ||
         (rc = dev_alloc((void**)&r->d_hpe, HW * (128 + 32) * 4)) ||
@@ -881,31 +987,39 @@ int pvdb_renderer_render(pvdb_renderer r, int32_t precision, pvdb_stream s) {
   P.storage = r->storage;
   RenderW Wk{};
   Wk.n = r->d_n;
-  Wk.off = r->d_off;
   Wk.T = r->d_T;
+  Wk.totals = r->d_totals;
+  Wk.head = r->d_head;
   Wk.viewdirs = r->d_viewdirs;
   const int HW = r->H * r->W;
+  const int tiles = ceil_div(r->W, kTileW) * ceil_div(r->H, kTileH);
   prof_begin_call();
   prof_mark(st, 0);
-  // 4 warps a block
-  const int march_grid = ceil_div(int64_t(ceil_div(r->W, kTileW)) * ceil_div(r->H, kTileH), 4);
-  k_render_march<false><<<march_grid, 128, 0, st>>>(P, Wk);
-  PVDB_CHECK_LAUNCH("k_render_march<count>");
-  prof_mark(st, 1);
-  int rc = scan_exclusive_u32(r->d_n, r->d_off, HW, r->d_totals + 1, &r->scan_partial,
-                              &r->scan_partial_cap, st);
+  int rc = renderer_grow_rows(r, 1);
+  if (!rc) rc = renderer_grow_batches(r, tiles);
   if (rc) return rc;
-  prof_mark(st, 2);
   uint32_t total = 0;
-  PVDB_CHECK_CUDA(cudaMemcpyAsync(&total, r->d_totals + 1, 4, cudaMemcpyDeviceToHost, st));
-  PVDB_CHECK_CUDA(cudaStreamSynchronize(st));
-  rc = renderer_grow_rows(r, int64_t(total) + 1);
-  if (rc) return rc;
+  for (;;) {
+    Wk.rw = r->d_rw;
+    Wk.rxyz = r->d_rxyz;
+    Wk.rpix = r->d_rpix;
+    Wk.cap = r->rows_cap;
+    Wk.batch = r->d_batch;
+    Wk.bcap = r->batch_cap;
+    PVDB_CHECK_CUDA(cudaMemsetAsync(r->d_totals, 0, 16, st));
+    k_render_march<<<ceil_div(tiles, 4), 128, 0, st>>>(P, Wk);
+    PVDB_CHECK_LAUNCH("k_render_march");
+    uint32_t tot[2] = {0, 0};
+    PVDB_CHECK_CUDA(cudaMemcpyAsync(tot, r->d_totals + 1, 8, cudaMemcpyDeviceToHost, st));
+    PVDB_CHECK_CUDA(cudaStreamSynchronize(st));
+    total = tot[0];
+    if (int64_t(tot[0]) <= r->rows_cap && int64_t(tot[1]) <= r->batch_cap) break;
+    // the counts do not depend on the buffers: one more march holds them
+    if ((rc = renderer_grow_rows(r, tot[0])) || (rc = renderer_grow_batches(r, tot[1]))) return rc;
+  }
+  prof_mark(st, 1);
+  prof_mark(st, 2);
   Wk.rk0 = r->d_rk0;
-  Wk.rw = r->d_rw;
-  Wk.rxyz = r->d_rxyz;
-  Wk.rpix = r->d_rpix;
-  Wk.cap = r->rows_cap;
   MlpArgs a;
   const int din = r->dcol + r->dpe, H = r->dhid;
   a.w0 = r->d_params;
@@ -918,8 +1032,6 @@ int pvdb_renderer_render(pvdb_renderer r, int32_t precision, pvdb_stream s) {
   a.dpe = r->dpe;
   a.din = din;
   if (total) {
-    k_render_march<true><<<march_grid, 128, 0, st>>>(P, Wk);
-    PVDB_CHECK_LAUNCH("k_render_march<fill>");
     const int64_t M = total;
     const int rgrid = ceil_div((M + 127) / 128 * 128, 256);
     if (precision == 1) {
@@ -950,8 +1062,7 @@ int pvdb_renderer_render(pvdb_renderer r, int32_t precision, pvdb_stream s) {
     if (rc) return rc;
   }
   prof_mark(st, 4);
-  k_render_composite<<<ceil_div(int64_t(HW) * 3, 192), 192, 0, st>>>(P, Wk, r->d_part,
-                                                                     r->d_image);
+  k_render_composite<<<ceil_div(tiles, 4), 128, 0, st>>>(P, Wk, r->d_part, r->d_image);
   PVDB_CHECK_LAUNCH("k_render_composite");
   prof_mark(st, 5);
   return PVDB_OK;
