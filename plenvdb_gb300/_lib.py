@@ -251,7 +251,7 @@ def stream_of(x=None) -> int | None:
     """The current torch CUDA stream handle (None = legacy default stream)."""
     try:
         import torch
-        if torch.cuda.is_available() and torch.cuda.is_initialized():
+        if torch.cuda.is_initialized():
             return torch.cuda.current_stream().cuda_stream
     except Exception:
         pass

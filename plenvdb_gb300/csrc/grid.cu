@@ -152,9 +152,13 @@ __global__ void k_sample1(GridView g, const float* __restrict__ xs, const float*
 }
 
 // Multi-channel trilinear (colorvdb.cu:81-111): per corner the scale is formed
-// first, then out[c] += value[c]*scale in corner order.
-__global__ void k_sampleC(GridView g, const float* __restrict__ xs, const float* __restrict__ ys,
-                          const float* __restrict__ zs, int64_t n, float* out) {
+// first, then out[c] += value[c]*scale in corner order. CT = 12: the channels
+// in 16-byte loads and stores (out on a 16-byte boundary); 0: any count. A
+// 4-byte load per corner and channel made the general form issue-bound.
+template <int CT>
+__global__ void __launch_bounds__(256)
+    k_sampleC(GridView g, const float* __restrict__ xs, const float* __restrict__ ys,
+              const float* __restrict__ zs, int64_t n, float* out) {
   grid_dep_sync();
   int64_t p = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   if (p >= n) return;
@@ -163,11 +167,30 @@ __global__ void k_sampleC(GridView g, const float* __restrict__ xs, const float*
   float sc[8];
   corner_scales(x - float(i), y - float(j), z - float(k), sc);
   int slots[8];
+  corner_slots(g, i, j, k, slots);
+  if (CT == 12) {
+    float r[12];
 #pragma unroll
-  for (int c = 0; c < 8; ++c) {
-    int di, dj, dk;
-    corner_delta(c, di, dj, dk);
-    slots[c] = slot_of(g, i + di, j + dj, k + dk);
+    for (int q = 0; q < 12; ++q) r[q] = 0.f;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      float v[12];
+      if (slots[c] >= 0) {
+        const float4* src = reinterpret_cast<const float4*>(g.data + int64_t(slots[c]) * 12);
+#pragma unroll
+        for (int b = 0; b < 3; ++b) *reinterpret_cast<float4*>(v + 4 * b) = __ldg(src + b);
+      } else {
+#pragma unroll
+        for (int q = 0; q < 12; ++q) v[q] = g.background;
+      }
+#pragma unroll
+      for (int q = 0; q < 12; ++q) r[q] = __fadd_rn(r[q], __fmul_rn(v[q], sc[c]));
+    }
+    float4* dst = reinterpret_cast<float4*>(out + p * 12);
+#pragma unroll
+    for (int b = 0; b < 3; ++b)
+      dst[b] = make_float4(r[4 * b], r[4 * b + 1], r[4 * b + 2], r[4 * b + 3]);
+    return;
   }
   for (int ch = 0; ch < g.C; ++ch) {
     float r = 0.f;
@@ -201,6 +224,17 @@ __global__ void k_zero_grad(GridView g, const uint8_t* __restrict__ touched) {
   if (touched && !touched[leaf]) return;
   if (!is_active(g, leaf, vox)) return;
   for (int c = 0; c < g.C; ++c) g.grad[n * g.C + c] = 0.f;
+}
+
+// The same for 12 channels, a thread per 16 bytes (a thread per voxel stores
+// 4-byte words 48 bytes apart: 14.7 us for the 160^3 benchmark grid).
+__global__ void k_zero_grad_c12(GridView g, const uint8_t* __restrict__ touched) {
+  grid_dep_sync();
+  const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x, n = i / 3;
+  if (n >= int64_t(g.nleaf) * kLeafVox) return;
+  const int leaf = int(n >> 9), vox = int(n & 511);
+  if (touched && !touched[leaf]) return;
+  if (is_active(g, leaf, vox)) reinterpret_cast<float4*>(g.grad)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
 __global__ void k_clear_touched(uint8_t* t, int n) {
@@ -880,8 +914,10 @@ int pvdb_grid_sample(pvdb_grid g, const float* xs, const float* ys, const float*
   }
   if (g->C == 1)
     launch_k(k_sample1, ceil_div(n, 256), 256, 0, st, g->view(), dx, dy, dz, n, dout);
+  else if (g->C == 12 && (reinterpret_cast<uintptr_t>(dout) & 15u) == 0)
+    launch_k(k_sampleC<12>, ceil_div(n, 256), 256, 0, st, g->view(), dx, dy, dz, n, dout);
   else
-    launch_k(k_sampleC, ceil_div(n, 256), 256, 0, st, g->view(), dx, dy, dz, n, dout);
+    launch_k(k_sampleC<0>, ceil_div(n, 256), 256, 0, st, g->view(), dx, dy, dz, n, dout);
   PVDB_CHECK_LAUNCH("k_sample");
   if (mem == PVDB_MEM_HOST) {
     PVDB_CHECK_CUDA(cudaMemcpyAsync(out, dout, n * 4 * g->C, cudaMemcpyDeviceToHost, st));
@@ -972,8 +1008,11 @@ int pvdb_grid_zero_grad(pvdb_grid g, pvdb_stream s) {
   cudaStream_t st = as_stream(s);
   const int64_t ns = g->nslots();
   if (ns) {
-    launch_k(k_zero_grad, ceil_div(ns, 256), 256, 0, st, g->view(),
-             g->all_touched ? nullptr : g->d_touched);
+    const uint8_t* touched = g->all_touched ? nullptr : g->d_touched;
+    if (g->C == 12)
+      launch_k(k_zero_grad_c12, ceil_div(ns * 3, 256), 256, 0, st, g->view(), touched);
+    else
+      launch_k(k_zero_grad, ceil_div(ns, 256), 256, 0, st, g->view(), touched);
     PVDB_CHECK_LAUNCH("k_zero_grad");
     launch_k(k_clear_touched, ceil_div(g->nleaf, 256), 256, 0, st, g->d_touched, g->nleaf);
     PVDB_CHECK_LAUNCH("k_clear_touched");

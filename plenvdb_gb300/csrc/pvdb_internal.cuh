@@ -104,6 +104,14 @@ struct ReduceScratch {
   size_t hist_cap = 0;
   uint32_t* partial = nullptr; // scan partials
   size_t partial_cap = 0;
+  // point backward: per cell of the lattice its first sorted point and the end
+  // of its points (zero between calls); the sorted points' records; the count
+  // of points with a gradient (capacities in bytes)
+  uint2* cells = nullptr;
+  size_t cells_cap = 0;
+  float4* rec = nullptr;
+  size_t rec_cap = 0;
+  uint32_t* npts = nullptr;
 };
 
 }  // namespace pvdb

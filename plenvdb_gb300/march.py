@@ -42,6 +42,21 @@ def march_params(xyz_min, xyz_max, near, stepdist, act_shift, interval, fast_col
     return p
 
 
+class _MarchHandle:
+    """Owns one pvdb_march; the workspace and every tensor over its memory hold it."""
+
+    def __init__(self, h):
+        self.h = h
+
+    def __del__(self):
+        try:
+            if self.h:
+                L.load().pvdb_march_destroy(self.h)
+                self.h = C.c_void_p(None)
+        except Exception:
+            pass
+
+
 class MarchWorkspace:
     """Owns a pvdb_march workspace for up to max_rays rays."""
 
@@ -56,6 +71,8 @@ class MarchWorkspace:
         out = C.c_void_p()
         L.call("pvdb_march_create", self.max_rays, self.samples_cap, C.byref(out))
         self.h = out
+        self._handle = _MarchHandle(out)
+        self._storage = {}
         self.generation = 0
         self.k0_channels = 0
         self.n_rays = 0
@@ -66,14 +83,6 @@ class MarchWorkspace:
         """Stage the density leaves of the forward's density pass in shared
         memory (bulk copies); bitwise the same results."""
         L.call("pvdb_march_set_leaf_staging", self.h, 1 if on else 0)
-
-    def __del__(self):
-        try:
-            if self.h:
-                L.load().pvdb_march_destroy(self.h)
-                self.h = C.c_void_p(None)
-        except Exception:
-            pass
 
     def views(self) -> L.MarchViews:
         v = L.MarchViews()
@@ -91,20 +100,32 @@ class MarchWorkspace:
         L.call("pvdb_march_stats", self.h, C.byref(k), C.byref(r), C.byref(e), L.stream_of())
         return k.value, r.value, e.value
 
+    def _tensor(self, name: str, ptr: int, capacity: int, shape, dtype: str):
+        """A tensor over the library's array `name`. The array's storage is wrapped
+        once (again if the library has moved or grown it): wrapping costs several
+        times what a tensor on an existing storage does. Each call gives a tensor
+        of its own, not a view of another one."""
+        known = self._storage.get(name)
+        if known is None or known[0] != (ptr, capacity):
+            base = device_view(ptr, (capacity,), dtype, self._handle)
+            known = self._storage[name] = ((ptr, capacity), base)
+        base = known[1]
+        return base.new_empty(0).set_(base.untyped_storage(), 0, shape)
+
     def rows(self, M: int, C0: int):
-        """Torch views of the colour rows of the last forward."""
+        """Torch tensors over the colour rows of the last forward."""
         v = self.views()
-        R = self.n_rays
+        R, cap = self.n_rays, v.rows_capacity
         out = {
-            "alphainv_last": device_view(v.alphainv_last, (R,), "float32", self),
-            "n_color": device_view(v.n_color, (R,), "int32", self),
-            "weight": device_view(v.weight, (M,), "float32", self),
-            "alpha": device_view(v.alpha, (M,), "float32", self),
-            "ray_id": device_view(v.ray_id, (M,), "int32", self),
-            "step_id": device_view(v.step_id, (M,), "int32", self),
+            "alphainv_last": self._tensor("T", v.alphainv_last, self.max_rays, (R,), "float32"),
+            "n_color": self._tensor("n", v.n_color, self.max_rays, (R,), "int32"),
+            "weight": self._tensor("w", v.weight, cap, (M,), "float32"),
+            "alpha": self._tensor("a", v.alpha, cap, (M,), "float32"),
+            "ray_id": self._tensor("r", v.ray_id, cap, (M,), "int32"),
+            "step_id": self._tensor("s", v.step_id, cap, (M,), "int32"),
         }
         if C0:
-            out["k0"] = device_view(v.k0, (M, C0), "float32", self)
+            out["k0"] = self._tensor("k0", v.k0, cap * C0, (M, C0), "float32")
         return out
 
 
@@ -136,6 +157,7 @@ class MarchSample(torch.autograd.Function):
         ctx.M, ctx.R, ctx.C0 = M, R, C0
         k0_rows = rows["k0"] if C0 else torch.zeros(M, 0, device=rays_o.device)
         ctx.mark_non_differentiable(rows["ray_id"])
+        ctx.set_materialize_grads(False)  # an unused output's gradient stays None
         return rows["weight"], rows["alphainv_last"], k0_rows, rows["ray_id"]
 
     @staticmethod
@@ -143,15 +165,14 @@ class MarchSample(torch.autograd.Function):
         ws = ctx.ws
         if ws.generation != ctx.gen:
             raise RuntimeError("march workspace was reused before this backward ran")
-        dev = torch.device("cuda")
-        gw = (g_weight if g_weight is not None else torch.zeros(ctx.M, device=dev)).float().contiguous()
-        gl = (g_last if g_last is not None else torch.zeros(ctx.R, device=dev)).float().contiguous()
+        # (the library takes a missing gradient as zero)
+        gw, gl = (g.float().contiguous() if g is not None else None for g in (g_weight, g_last))
         gk = None
         if ctx.k0 is not None and g_k0 is not None:
             gk = g_k0.float().contiguous()
         L.call("pvdb_march_backward", ws.h, ctx.density.handle,
-               ctx.k0.handle if ctx.k0 is not None else None, L.ptr(gw), L.ptr(gl),
-               L.ptr(gk) if gk is not None else None, L.stream_of())
+               ctx.k0.handle if ctx.k0 is not None else None, L.ptr(gw), L.ptr(gl), L.ptr(gk),
+               L.stream_of())
         return (None,) * 8
 
 
@@ -188,7 +209,9 @@ class RgbNetFn(torch.autograd.Function):
         if ws.generation != ctx.gen:
             raise RuntimeError("march workspace was reused before this backward ran")
         M = rgb.shape[0]
-        grads = [torch.zeros_like(t) for t in (w0, b0, w1, b1, w2, b2)]
+        # (with rows, the kernels write every weight gradient)
+        new = torch.empty_like if M else torch.zeros_like
+        grads = [new(t) for t in (w0, b0, w1, b1, w2, b2)]
         gk0 = torch.zeros(M, ctx.c0, device=rgb.device, dtype=torch.float32)
         if M:
             s = _mlp_struct(w0, b0, w1, b1, w2, b2, ctx.c0, ctx.pe)
