@@ -48,6 +48,26 @@ __device__ __forceinline__ void bar_group(int id, int threads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
+// Two FP32 FMAs in one instruction (each rounded as fmaf): half the issue slots
+// and register reads of two fmaf. Row pairs come packed from 16-byte loads, the
+// other factor is duplicated. In the forward's product loop it reached 108
+// against 103 FMAs per clock and SM; in the backward's, beside its resident
+// accumulators, the duplicates spilled and cost what they gave.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ f32x2 dup2(float v) {
+  f32x2 d;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(d) : "f"(v));
+  return d;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+
 // One step of a reduce-scatter over lanes that differ in `mask`: the first
 // N/2 entries of v become the sums of the half this lane keeps.
 template <int N>
@@ -85,26 +105,30 @@ __device__ __forceinline__ void layer0(float* h0, int ld, const float* w0k, cons
   float w[4 * CQ];
 #pragma unroll
   for (int q = 0; q < 4 * CQ; ++q) w[q] = w0k[q * kW + n];
-#pragma unroll 2
-  for (int r = r0; r < r0 + kRows; r += 4) {
-    float z[4];
+  constexpr int kB = kRows < 16 ? kRows : 16;  // rows whose hpe loads are in flight together
+#pragma unroll 1
+  for (int r = r0; r < r0 + kRows; r += kB) {
+    float z[kB];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < kB; ++i) {
       const int ry = rays[r + i];
       z[i] = ry >= 0 ? __ldg(hpe + int64_t(ry) * kW + n) : 0.f;
     }
 #pragma unroll
-    for (int b = 0; b < CQ; ++b)
+    for (int i = 0; i < kB; ++i)
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
+      for (int b = 0; b < CQ; ++b) {
         const float4 v = *reinterpret_cast<const float4*>(x + (r + i) * 4 * CQ + 4 * b);
         z[i] = fmaf(w[4 * b], v.x, z[i]);
         z[i] = fmaf(w[4 * b + 1], v.y, z[i]);
         z[i] = fmaf(w[4 * b + 2], v.z, z[i]);
         z[i] = fmaf(w[4 * b + 3], v.w, z[i]);
       }
-    *reinterpret_cast<float4*>(h0 + n * ld + r) =
-        make_float4(fmaxf(z[0], 0.f), fmaxf(z[1], 0.f), fmaxf(z[2], 0.f), fmaxf(z[3], 0.f));
+#pragma unroll
+    for (int i = 0; i < kB; i += 4)
+      *reinterpret_cast<float4*>(h0 + n * ld + r + i) =
+          make_float4(fmaxf(z[i], 0.f), fmaxf(z[i + 1], 0.f), fmaxf(z[i + 2], 0.f),
+                      fmaxf(z[i + 3], 0.f));
   }
 }
 
@@ -159,26 +183,29 @@ __device__ __forceinline__ void fwd_tile(FwdSmem<CQ>& S, FwdGroupSmem<CQ>& G, in
   bar_group(bar, kFwdGroup);
   layer0<TR, CQ, kFwdGroup>(G.h0, ld, S.w0k, G.x, G.rays, hpe, t);
   bar_group(bar, kFwdGroup);
-  float acc[4 * RT][4 * CT];
+  f32x2 acc2[2 * RT][4 * CT];  // row pairs
 #pragma unroll
-  for (int i = 0; i < 4 * RT; ++i)
+  for (int i = 0; i < 2 * RT; ++i)
 #pragma unroll
-    for (int j = 0; j < 4 * CT; ++j) acc[i][j] = 0.f;
+    for (int j = 0; j < 4 * CT; ++j) acc2[i][j] = 0;
 #pragma unroll 4
   for (int k = 0; k < kW; ++k) {
-    float av[4 * RT], bv[4 * CT];
+    f32x2 av[2 * RT];
+    float bv[4 * CT];
 #pragma unroll
     for (int i = 0; i < RT; ++i)
-      *reinterpret_cast<float4*>(av + 4 * i) =
-          *reinterpret_cast<const float4*>(G.h0 + k * ld + rb + 16 * i);
+      *reinterpret_cast<ulonglong2*>(av + 2 * i) =
+          *reinterpret_cast<const ulonglong2*>(G.h0 + k * ld + rb + 16 * i);
 #pragma unroll
     for (int j = 0; j < CT; ++j)
       *reinterpret_cast<float4*>(bv + 4 * j) =
           *reinterpret_cast<const float4*>(S.w1t + k * kW + cb + 32 * j);
 #pragma unroll
-    for (int i = 0; i < 4 * RT; ++i)
+    for (int j = 0; j < 4 * CT; ++j) {
+      const f32x2 d = dup2(bv[j]);
 #pragma unroll
-      for (int j = 0; j < 4 * CT; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+      for (int i = 0; i < 2 * RT; ++i) acc2[i][j] = fma2(av[i], d, acc2[i][j]);
+    }
   }
   // logits: this thread's columns, then the 8 lanes of its rows (a
   // reduce-scatter: lane tx ends with one row), then the column warps
@@ -191,10 +218,16 @@ __device__ __forceinline__ void fwd_tile(FwdSmem<CQ>& S, FwdGroupSmem<CQ>& G, in
     const float b1 = S.b1[n];
     const float w[3] = {S.w2[n], S.w2[kW + n], S.w2[2 * kW + n]};
 #pragma unroll
-    for (int i = 0; i < 4 * RT; ++i) {
-      const float h = fmaxf(acc[i][j] + b1, 0.f);
+    for (int i = 0; i < 2 * RT; ++i) {
+      float h[2];
+      unpack2(acc2[i][j], h[0], h[1]);
 #pragma unroll
-      for (int c = 0; c < 3; ++c) lg[3 * i + c] = fmaf(w[c], h, lg[3 * i + c]);
+      for (int e = 0; e < 2; ++e) {
+        h[e] = fmaxf(h[e] + b1, 0.f);
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+          lg[3 * (2 * i + e) + c] = fmaf(w[c], h[e], lg[3 * (2 * i + e) + c]);
+      }
     }
   }
   float* red = G.x;

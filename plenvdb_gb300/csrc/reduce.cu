@@ -534,9 +534,8 @@ __global__ void k_point_keys(GridView gv, const float* __restrict__ xs, const fl
 
 // The merge of the up to 8 point lists around one voxel: list c is the points
 // of the cell that has the voxel as corner c, at positions pos[c] .. end[c];
-// ids(pos) gives a point's id. Each kMergeBatch points are taken first and then
+// ids(pos) gives a point's id. A few points are taken first and then
 // loaded together: their loads do not wait for one another, only the sums do.
-constexpr int kMergeBatch = 4;
 
 // A point as the sums read it: cell-relative position, gradient of up to 12
 // channels (density: g[0]).
@@ -549,6 +548,7 @@ template <bool SCALAR, class Ids, class Load>
 __device__ __forceinline__ void merge_lists(const Ids& ids, const Load& load,
                                             const uint32_t first[8], const uint32_t end[8],
                                             float acc[12], bool& any) {
+  constexpr int kMergeBatch = SCALAR ? 4 : 2;
   uint32_t head[8], pos[8];
 #pragma unroll
   for (int c = 0; c < 8; ++c) {
