@@ -252,7 +252,8 @@ def stream_of(x=None) -> int | None:
     try:
         import torch
         if torch.cuda.is_initialized():
-            return torch.cuda.current_stream().cuda_stream
+            # the raw handle: building a Stream object for it costs more than a launch
+            return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
     except Exception:
         pass
     return None

@@ -112,18 +112,20 @@ class MarchWorkspace:
         base = known[1]
         return base.new_empty(0).set_(base.untyped_storage(), 0, shape)
 
-    def rows(self, M: int, C0: int):
-        """Torch tensors over the colour rows of the last forward."""
+    def rows(self, M: int, C0: int, stage_only: bool = False):
+        """Torch tensors over the colour rows of the last forward (stage_only: just
+        those the sample stage returns)."""
         v = self.views()
         R, cap = self.n_rays, v.rows_capacity
         out = {
             "alphainv_last": self._tensor("T", v.alphainv_last, self.max_rays, (R,), "float32"),
-            "n_color": self._tensor("n", v.n_color, self.max_rays, (R,), "int32"),
             "weight": self._tensor("w", v.weight, cap, (M,), "float32"),
-            "alpha": self._tensor("a", v.alpha, cap, (M,), "float32"),
             "ray_id": self._tensor("r", v.ray_id, cap, (M,), "int32"),
-            "step_id": self._tensor("s", v.step_id, cap, (M,), "int32"),
         }
+        if not stage_only:
+            out["n_color"] = self._tensor("n", v.n_color, self.max_rays, (R,), "int32")
+            out["alpha"] = self._tensor("a", v.alpha, cap, (M,), "float32")
+            out["step_id"] = self._tensor("s", v.step_id, cap, (M,), "int32")
         if C0:
             out["k0"] = self._tensor("k0", v.k0, cap * C0, (M, C0), "float32")
         return out
@@ -152,7 +154,7 @@ class MarchSample(torch.autograd.Function):
         C0 = k0.ndim if k0 is not None else 0
         ws.k0_channels = C0
         _, M = ws.totals()
-        rows = ws.rows(M, C0)
+        rows = ws.rows(M, C0, stage_only=True)
         ctx.ws, ctx.gen, ctx.density, ctx.k0 = ws, ws.generation, density, k0
         ctx.M, ctx.R, ctx.C0 = M, R, C0
         k0_rows = rows["k0"] if C0 else torch.zeros(M, 0, device=rays_o.device)
