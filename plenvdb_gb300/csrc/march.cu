@@ -470,8 +470,8 @@ __device__ __forceinline__ void k0_trilinear(const GridView& g, const float idx[
 }
 
 // The 12-channel trilinear from the grid's BF16 shadow (the BF16 train step):
-// one 32-byte record per corner in two 16-byte loads, FP32 interpolation in
-// the order of k0_trilinear.
+// one 32-byte record per corner in one load, four corners in flight, FP32
+// interpolation in the order of k0_trilinear.
 __device__ __forceinline__ void k0_trilinear_half(const GridView& g,
                                                   const __nv_bfloat16* __restrict__ half,
                                                   const float idx[3], float* out) {
@@ -480,36 +480,31 @@ __device__ __forceinline__ void k0_trilinear_half(const GridView& g,
   corner_scales(idx[0] - float(i), idx[1] - float(j), idx[2] - float(k), sc);
   int slots[8];
   corner_slots(g, i, j, k, slots);
-  uint4 lo[8];
-  uint2 hi[8];
-#pragma unroll
-  for (int c = 0; c < 8; ++c) {
-    if (slots[c] >= 0) {
-      const uint4* src = reinterpret_cast<const uint4*>(half + int64_t(slots[c]) * kHalfStride);
-      lo[c] = __ldg(src);
-      const uint4 h = __ldg(src + 1);
-      hi[c] = make_uint2(h.x, h.y);
-    }
-  }
   float acc[12];
 #pragma unroll
   for (int q = 0; q < 12; ++q) acc[q] = 0.f;
 #pragma unroll
-  for (int c = 0; c < 8; ++c) {
-    float v[12];
-    if (slots[c] >= 0) {
-      const uint32_t w[6] = {lo[c].x, lo[c].y, lo[c].z, lo[c].w, hi[c].x, hi[c].y};
+  for (int c0 = 0; c0 < 8; c0 += 4) {
+    uint32_t w[4][8];
 #pragma unroll
-      for (int b = 0; b < 6; ++b) {
-        v[2 * b] = __uint_as_float(w[b] << 16);
-        v[2 * b + 1] = __uint_as_float(w[b] & 0xFFFF0000u);
+    for (int c = 0; c < 4; ++c)
+      if (slots[c0 + c] >= 0) ld_nc32(half + int64_t(slots[c0 + c]) * kHalfStride, w[c]);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      float v[12];
+      if (slots[c0 + c] >= 0) {
+#pragma unroll
+        for (int b = 0; b < 6; ++b) {
+          v[2 * b] = __uint_as_float(w[c][b] << 16);
+          v[2 * b + 1] = __uint_as_float(w[c][b] & 0xFFFF0000u);
+        }
+      } else {
+#pragma unroll
+        for (int q = 0; q < 12; ++q) v[q] = g.background;
       }
-    } else {
 #pragma unroll
-      for (int q = 0; q < 12; ++q) v[q] = g.background;
+      for (int q = 0; q < 12; ++q) acc[q] = __fadd_rn(acc[q], __fmul_rn(v[q], sc[c0 + c]));
     }
-#pragma unroll
-    for (int q = 0; q < 12; ++q) acc[q] = __fadd_rn(acc[q], __fmul_rn(v[q], sc[c]));
   }
 #pragma unroll
   for (int q = 0; q < 12; ++q) out[q] = acc[q];
@@ -941,9 +936,18 @@ __global__ void __launch_bounds__(256)
     float4 q[NB];
     if (NQ) gather_row<NQ>(gk0, __ldg(brow + sv), C, vec, q);
     float4* dst = rec_g + j * (1 + NQ);
-    dst[0] = p;
+    if constexpr (NQ == 3) {
+      const auto bits = [](const float4& f) {
+        return make_uint4(__float_as_uint(f.x), __float_as_uint(f.y), __float_as_uint(f.z),
+                          __float_as_uint(f.w));
+      };
+      st_32(dst, bits(p), bits(q[0]));
+      st_32(dst + 2, bits(q[1]), bits(q[2]));
+    } else {
+      dst[0] = p;
 #pragma unroll
-    for (int b = 0; b < NQ; ++b) dst[1 + b] = q[b];
+      for (int b = 0; b < NQ; ++b) dst[1 + b] = q[b];
+    }
   }
 }
 
@@ -1019,11 +1023,16 @@ __global__ void __launch_bounds__(256, 4)
       const uint32_t h = __ldg(off + key[c]);
       for (uint32_t j = h; j < h + len[c]; ++j) {
         const float4* r = rec_g + int64_t(j) * (1 + NQ);
-        const float4 p0 = __ldg(r);
-        float4 q0[NB];
-        if (want_c) {
+        float4 p0, q0[NB];
+        if constexpr (NQ == 3) {
+          ld_nc32(r, p0, q0[0]);
+          if (want_c) ld_nc32(r + 2, q0[1], q0[2]);
+        } else {
+          p0 = __ldg(r);
+          if (want_c) {
 #pragma unroll
-          for (int b = 0; b < NQ; ++b) q0[b] = __ldg(r + 1 + b);
+            for (int b = 0; b < NQ; ++b) q0[b] = __ldg(r + 1 + b);
+          }
         }
         gather_add<NQ>(p0, q0, want_c, want_d, c, pd, pk);
       }

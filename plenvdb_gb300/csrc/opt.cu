@@ -238,10 +238,10 @@ __global__ void k_vdb_adam_c12(GridView g, float* __restrict__ m, float* __restr
       if (zero_after) g4[b] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
     if (half) {  // the voxel's 32-byte shadow record: channels 0..11, then zeros
-      uint4* h4 = reinterpret_cast<uint4*>(half + slot * kHalfStride);
-      h4[0] = make_uint4(tc::pack_bf16(dd[0], dd[1]), tc::pack_bf16(dd[2], dd[3]),
-                         tc::pack_bf16(dd[4], dd[5]), tc::pack_bf16(dd[6], dd[7]));
-      h4[1] = make_uint4(tc::pack_bf16(dd[8], dd[9]), tc::pack_bf16(dd[10], dd[11]), 0u, 0u);
+      st_32(half + slot * kHalfStride,
+            make_uint4(tc::pack_bf16(dd[0], dd[1]), tc::pack_bf16(dd[2], dd[3]),
+                       tc::pack_bf16(dd[4], dd[5]), tc::pack_bf16(dd[6], dd[7])),
+            make_uint4(tc::pack_bf16(dd[8], dd[9]), tc::pack_bf16(dd[10], dd[11]), 0u, 0u));
     }
   }
   if (counts) count_add(counts, n_act, n_upd);

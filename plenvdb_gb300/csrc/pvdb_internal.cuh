@@ -336,6 +336,29 @@ __device__ __forceinline__ void bmax_raise(const GridView& g, int x, int y, int 
         atomicMax(g.bmax + (int64_t(bx) * g.bdim[1] + by) * g.bdim[2] + bz, key);
 }
 
+// 32 bytes from a 32-byte boundary in one load (read-only data) or store: half
+// the requests of two 16-byte ones for records that are gathered a whole
+// sector at a time.
+__device__ __forceinline__ void ld_nc32(const void* p, uint32_t v[8]) {
+  asm("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
+        "=r"(v[7])
+      : "l"(p));
+}
+__device__ __forceinline__ void ld_nc32(const float4* p, float4& a, float4& b) {
+  uint32_t v[8];
+  ld_nc32(static_cast<const void*>(p), v);
+  a = make_float4(__uint_as_float(v[0]), __uint_as_float(v[1]), __uint_as_float(v[2]),
+                  __uint_as_float(v[3]));
+  b = make_float4(__uint_as_float(v[4]), __uint_as_float(v[5]), __uint_as_float(v[6]),
+                  __uint_as_float(v[7]));
+}
+__device__ __forceinline__ void st_32(void* p, const uint4& a, const uint4& b) {
+  asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(a.x), "r"(a.y),
+               "r"(a.z), "r"(a.w), "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w)
+               : "memory");
+}
+
 __device__ __forceinline__ unsigned lanemask_lt() {
   unsigned m;
   asm volatile("mov.u32 %0, %%lanemask_lt;" : "=r"(m));

@@ -797,14 +797,21 @@ struct RecLoad {
   int ch0, nch;
   __device__ __forceinline__ void operator()(uint32_t s, uint32_t at, PointTerm& t) const {
     const float4* r = rec + int64_t(at) * (VEC ? 4 : 1);
-    const float4 p = __ldg(r);
+    float4 p;
+    if (VEC) {
+      float4 g[3];
+      ld_nc32(r, p, g[0]);
+      ld_nc32(r + 2, g[1], g[2]);
+#pragma unroll
+      for (int b = 0; b < 3; ++b) *reinterpret_cast<float4*>(t.g + 4 * b) = g[b];
+    } else {
+      p = __ldg(r);
+    }
     t.u = p.x;
     t.v = p.y;
     t.w = p.z;
-    if (VEC) {
-#pragma unroll
-      for (int b = 0; b < 3; ++b) *reinterpret_cast<float4*>(t.g + 4 * b) = __ldg(r + 1 + b);
-    } else if (src.C == 1) {
+    if (VEC) return;
+    if (src.C == 1) {
       t.g[0] = p.w;
     } else {
       const float* gs = src.g + int64_t(s) * src.C + ch0;
