@@ -87,33 +87,51 @@ __device__ __forceinline__ void slot_coord(const GridView& g, int leaf, int vox,
   z = __ldg(g.origin + leaf * 3 + 2) + (vox & 7);
 }
 
-// The leaves next to `leaf` in the order -z, +z, -y, +y, -x, +x (-1: none), the
-// same in every lane. A whole warp calls it with one leaf: six lanes look a
-// leaf up each. (A lookup per voxel on a leaf face, which more than half of the
-// voxels are, had every warp walk six divergent lookups.)
-__device__ __forceinline__ void face_leaves(const GridView& g, int leaf, int fl[6]) {
+// A quarter of a leaf, 128 voxels, as a warp of the TV kernels takes it: what
+// its voxels share is looked up once, by lanes side by side. (With a voxel a
+// thread, every warp repeated it for 32 voxels and spent two thirds of its
+// instructions there, and a voxel on a leaf face walked up to six divergent
+// lookups.)
+struct LeafQuarter {
+  int leaf, q;
+  int x, y, z;       // origin of the leaf
+  uint64_t m0, m1;   // active bits of the voxels
+  int fl[6];         // the leaves next to it: -z, +z, -y, +y, -x, +x (-1: none)
+  // voxel of slice s (0..3) and this lane, its coordinates and whether it is active
+  __device__ __forceinline__ int vox(int s) const { return q * 128 + s * 32 + int(threadIdx.x & 31); }
+  __device__ __forceinline__ bool active(int s) const {
+    return ((s & 2 ? m1 : m0) >> ((s & 1) * 32 + (threadIdx.x & 31))) & 1ull;
+  }
+};
+__device__ __forceinline__ LeafQuarter leaf_quarter(const GridView& g, int leaf, int q) {
+  LeafQuarter L;
+  L.leaf = leaf;
+  L.q = q;
+  L.x = __ldg(g.origin + leaf * 3);
+  L.y = __ldg(g.origin + leaf * 3 + 1);
+  L.z = __ldg(g.origin + leaf * 3 + 2);
+  L.m0 = __ldg(g.mask + leaf * 8 + 2 * q);
+  L.m1 = __ldg(g.mask + leaf * 8 + 2 * q + 1);
   const int lane = threadIdx.x & 31;
   int v = -1;
   if (lane < 6) {
     const int ax = 2 - (lane >> 1), d = lane & 1 ? 8 : -8;
-    const int x = __ldg(g.origin + leaf * 3) + (ax == 0 ? d : 0),
-              y = __ldg(g.origin + leaf * 3 + 1) + (ax == 1 ? d : 0),
-              z = __ldg(g.origin + leaf * 3 + 2) + (ax == 2 ? d : 0);
-    v = leaf_of(g, x, y, z);
+    v = leaf_of(g, L.x + (ax == 0 ? d : 0), L.y + (ax == 1 ? d : 0), L.z + (ax == 2 ? d : 0));
   }
 #pragma unroll
-  for (int q = 0; q < 6; ++q) fl[q] = __shfl_sync(0xffffffffu, v, q);
+  for (int e = 0; e < 6; ++e) L.fl[e] = __shfl_sync(0xffffffffu, v, e);
+  return L;
 }
 
 // Slots of the 6 face neighbours of voxel (x, y, z) = (leaf, vox), in the order
 // -z, +z, -y, +y, -x, +x: -2 outside [0, reso) (no TV term), -1 in no
 // allocated leaf (background). Offsets follow from the layout (+64 x, +8 y,
-// +1 z); across a face they wrap into the neighbour leaf fl[q].
-__device__ __forceinline__ void face_neighbours(const GridView& g, int leaf, int vox, int x, int y,
-                                                int z, const int fl[6], int nb[6]) {
+// +1 z); across a face they wrap into the neighbour leaf.
+__device__ __forceinline__ void face_neighbours(const GridView& g, const LeafQuarter& L, int vox,
+                                                int x, int y, int z, int nb[6]) {
   const int lx = vox >> 6, ly = (vox >> 3) & 7, lz = vox & 7;
   auto at = [&](bool edge, bool inner, int q, int step) {
-    const int l = inner ? leaf : fl[q];
+    const int l = inner ? L.leaf : L.fl[q];
     return edge ? -2 : l < 0 ? -1 : (l << 9) + vox + (inner ? step : -7 * step);
   };
   nb[0] = at(z == 0, lz > 0, 0, -1);
@@ -287,46 +305,70 @@ __device__ __forceinline__ float value_c(const GridView& g, int i, int j, int k,
 }
 
 // TV gradient (total_variation_kernel.cu:13-35) on the leaf store, for the
-// voxels of the listed leaves (list = NULL: all leaves). One thread per voxel:
-// the six neighbour slots are looked up once and shared by the channels;
-// neighbours inside [0,reso) only, values through the leaf table (background
-// outside allocated leaves). Per channel the sum is formed in the reference's
-// order z-, z+, y-, y+, x-, x+.
-__global__ void k_tv(GridView g, float wx, float wy, float wz, int dense_mode,
-                     const int32_t* __restrict__ list, const uint32_t* __restrict__ count) {
+// voxels of the listed leaves (list = NULL: all leaves), a warp per quarter of
+// a leaf: neighbours inside [0,reso) only, values through the leaf table
+// (background outside allocated leaves). Per channel the sum is formed in the
+// reference's order z-, z+, y-, y+, x-, x+, each term rounded, then added (the
+// reference's conditional terms are not fused, total_variation_kernel.cu:27-32).
+// TERMS: the sums alone, into out, for every active voxel (0 outside
+// [0, reso)); else they are added to the gradient (sparse: where it is not
+// zero).
+template <bool TERMS>
+__global__ void __launch_bounds__(256)
+    k_tv(GridView g, float wx, float wy, float wz, int dense_mode, const int32_t* __restrict__ list,
+         const uint32_t* __restrict__ count, float* __restrict__ out) {
   grid_dep_sync();
-  const int64_t nl = list ? int64_t(*count) : int64_t(g.nleaf);
-  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < nl * kLeafVox;
-       i += int64_t(gridDim.x) * blockDim.x) {
-    const int leaf = list ? list[i >> 9] : int(i >> 9);
-    const int vox = int(i & 511);
-    int fl[6];
-    face_leaves(g, leaf, fl);
-    if (!is_active(g, leaf, vox)) continue;
-    int x, y, z;
-    slot_coord(g, leaf, vox, x, y, z);
-    if (x >= g.reso[0] || y >= g.reso[1] || z >= g.reso[2]) continue;
-    int nb[6];
-    face_neighbours(g, leaf, vox, x, y, z, fl, nb);
-    const float wt[6] = {wz, wz, wy, wy, wx, wx};
-    const int64_t t0 = (int64_t(leaf) * kLeafVox + vox) * g.C;
+  const int64_t nq = 4 * (list ? int64_t(*count) : int64_t(g.nleaf));
+  const float wt[6] = {wz, wz, wy, wy, wx, wx};
+  for (int64_t u = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5; u < nq;
+       u += (int64_t(gridDim.x) * blockDim.x) >> 5) {
+    const LeafQuarter L = leaf_quarter(g, list ? list[u >> 2] : int(u >> 2), int(u & 3));
     for (int ch = 0; ch < g.C; ++ch) {
-      const float gcur = g.grad[t0 + ch];
-      if (!dense_mode && gcur == 0.f) continue;
-      const float p = g.data[t0 + ch];
-      float add = 0.f;
+      // two slices' values and neighbours are loaded together
+#pragma unroll 1
+      for (int s0 = 0; s0 < 4; s0 += 2) {
+        float gc[2], p[2], vn[2][6];
+        bool take[2];
+        uint32_t skip[2];  // bit q: no term for neighbour q
 #pragma unroll
-      for (int q = 0; q < 6; ++q) {
-        if (nb[q] == -2) {
-          add += 0.f;
-        } else {
-          const float vn = nb[q] < 0 ? g.background : g.data[int64_t(nb[q]) * g.C + ch];
-          // each term rounded, then added (the reference's conditional terms
-          // are not fused, total_variation_kernel.cu:27-32)
-          add = __fadd_rn(add, __fmul_rn(wt[q], tv_clamp(p - vn)));
+        for (int e = 0; e < 2; ++e) {
+          const int64_t t = (int64_t(L.leaf) * kLeafVox + L.vox(s0 + e)) * g.C + ch;
+          take[e] = L.active(s0 + e);
+          gc[e] = !TERMS && take[e] ? g.grad[t] : 0.f;
+          if (!TERMS && !dense_mode && gc[e] == 0.f) take[e] = false;
+          p[e] = take[e] ? g.data[t] : 0.f;
+        }
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int vox = L.vox(s0 + e);
+          const int x = L.x + (vox >> 6), y = L.y + ((vox >> 3) & 7), z = L.z + (vox & 7);
+          const bool in = x < g.reso[0] && y < g.reso[1] && z < g.reso[2];
+          if (!TERMS) take[e] = take[e] && in;
+          int nb[6];
+          face_neighbours(g, L, vox, x, y, z, nb);
+          skip[e] = in ? 0u : 0x3Fu;
+#pragma unroll
+          for (int q = 0; q < 6; ++q) {
+            if (nb[q] == -2) skip[e] |= 1u << q;
+            vn[e][q] = g.background;
+            if (take[e] && nb[q] >= 0) vn[e][q] = g.data[int64_t(nb[q]) * g.C + ch];
+          }
+        }
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          if (!take[e]) continue;
+          float add = 0.f;
+#pragma unroll
+          for (int q = 0; q < 6; ++q)
+            if (!((skip[e] >> q) & 1u))
+              add = __fadd_rn(add, __fmul_rn(wt[q], tv_clamp(p[e] - vn[e][q])));
+          const int64_t t = (int64_t(L.leaf) * kLeafVox + L.vox(s0 + e)) * g.C + ch;
+          if (TERMS)
+            out[t] = add;
+          else
+            g.grad[t] = gc[e] + add;
         }
       }
-      g.grad[t0 + ch] = gcur + add;
     }
   }
 }
@@ -351,37 +393,46 @@ __global__ void k_bmax_init(GridView g, uint32_t* bmax) {
   }
 }
 
-// k_tv for 12-channel grids: the voxel's and its neighbours' channels in
-// float4 loads; per-channel arithmetic and order as k_tv.
-__global__ void k_tv_c12(GridView g, float wx, float wy, float wz, int dense_mode,
-                         const int32_t* __restrict__ list, const uint32_t* __restrict__ count) {
+// k_tv for 12-channel grids, channels in 16-byte loads, a thread per voxel (a
+// warp walking its quarter's four slices took 275 against 235 us at 320^3);
+// per-channel arithmetic and order as k_tv. The sums alone (TERMS) need only the values, so the fused
+// step runs them beside the gradient sums and its voxel Adam adds them to the
+// channels with a nonzero gradient, which is what the sparse mode does.
+template <bool TERMS>
+__global__ void __launch_bounds__(256)
+    k_tv_c12(GridView g, float wx, float wy, float wz, int dense_mode,
+             const int32_t* __restrict__ list, const uint32_t* __restrict__ count,
+             float* __restrict__ out) {
   grid_dep_sync();
   const int64_t nl = list ? int64_t(*count) : int64_t(g.nleaf);
+  const float wt[6] = {wz, wz, wy, wy, wx, wx};
   for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < nl * kLeafVox;
        i += int64_t(gridDim.x) * blockDim.x) {
-    const int leaf = list ? list[i >> 9] : int(i >> 9);
     const int vox = int(i & 511);
-    int fl[6];
-    face_leaves(g, leaf, fl);
-    if (!is_active(g, leaf, vox)) continue;
-    const int64_t t0 = (int64_t(leaf) * kLeafVox + vox) * 12;
-    float4* g4 = reinterpret_cast<float4*>(g.grad + t0);
+    const LeafQuarter L = leaf_quarter(g, list ? list[i >> 9] : int(i >> 9), vox >> 7);
+    if (!L.active((vox >> 5) & 3)) continue;
+    const int64_t t0 = (int64_t(L.leaf) * kLeafVox + vox) * 12;
+    float4* o4 = reinterpret_cast<float4*>((TERMS ? out : g.grad) + t0);
+    const int x = L.x + (vox >> 6), y = L.y + ((vox >> 3) & 7), z = L.z + (vox & 7);
+    const bool in = x < g.reso[0] && y < g.reso[1] && z < g.reso[2];
     float gc[12];
+    if (!TERMS) {
 #pragma unroll
-    for (int b = 0; b < 3; ++b) {
-      const float4 x = g4[b];
-      gc[4 * b] = x.x; gc[4 * b + 1] = x.y; gc[4 * b + 2] = x.z; gc[4 * b + 3] = x.w;
+      for (int b = 0; b < 3; ++b) {
+        const float4 v = o4[b];
+        gc[4 * b] = v.x; gc[4 * b + 1] = v.y; gc[4 * b + 2] = v.z; gc[4 * b + 3] = v.w;
+      }
+      bool any = dense_mode != 0;
+#pragma unroll
+      for (int ch = 0; ch < 12; ++ch) any = any || gc[ch] != 0.f;
+      if (!any || !in) continue;
+    } else if (!in) {
+#pragma unroll
+      for (int b = 0; b < 3; ++b) o4[b] = make_float4(0.f, 0.f, 0.f, 0.f);
+      continue;
     }
-    bool any = dense_mode != 0;
-#pragma unroll
-    for (int ch = 0; ch < 12; ++ch) any = any || gc[ch] != 0.f;
-    if (!any) continue;
-    int x, y, z;
-    slot_coord(g, leaf, vox, x, y, z);
-    if (x >= g.reso[0] || y >= g.reso[1] || z >= g.reso[2]) continue;
     int nb[6];
-    face_neighbours(g, leaf, vox, x, y, z, fl, nb);
-    const float wt[6] = {wz, wz, wy, wy, wx, wx};
+    face_neighbours(g, L, vox, x, y, z, nb);
     float p[12], add[12];
     const float4* d4 = reinterpret_cast<const float4*>(g.data + t0);
 #pragma unroll
@@ -416,110 +467,10 @@ __global__ void k_tv_c12(GridView g, float wx, float wy, float wz, int dense_mod
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const int ch = 4 * b + e;
-        o[e] = (!dense_mode && gc[ch] == 0.f) ? gc[ch] : gc[ch] + add[ch];
+        o[e] = TERMS ? add[ch] : (!dense_mode && gc[ch] == 0.f) ? gc[ch] : gc[ch] + add[ch];
       }
-      g4[b] = make_float4(o[0], o[1], o[2], o[3]);
+      o4[b] = make_float4(o[0], o[1], o[2], o[3]);
     }
-  }
-}
-
-// The TV sums of k_tv / k_tv_c12 (same neighbours, order and rounding)
-// without the gradient: tv[slot*C + ch] for every active voxel of the listed
-// leaves (0 outside [0, reso)). In sparse mode k_tv adds them to the channels
-// whose gradient is nonzero; the fused step's voxel Adam does that addition
-// instead, so this pass needs only the values and can run beside the
-// gradient sums.
-__global__ void k_tv_terms(GridView g, float wx, float wy, float wz,
-                           const int32_t* __restrict__ list, const uint32_t* __restrict__ count,
-                           float* __restrict__ tv) {
-  grid_dep_sync();
-  const int64_t nl = *count;
-  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < nl * kLeafVox;
-       i += int64_t(gridDim.x) * blockDim.x) {
-    const int leaf = list[i >> 9];
-    const int vox = int(i & 511);
-    int fl[6];
-    face_leaves(g, leaf, fl);
-    if (!is_active(g, leaf, vox)) continue;
-    const int64_t t0 = (int64_t(leaf) * kLeafVox + vox) * g.C;
-    int x, y, z;
-    slot_coord(g, leaf, vox, x, y, z);
-    if (x >= g.reso[0] || y >= g.reso[1] || z >= g.reso[2]) {
-      for (int ch = 0; ch < g.C; ++ch) tv[t0 + ch] = 0.f;
-      continue;
-    }
-    int nb[6];
-    face_neighbours(g, leaf, vox, x, y, z, fl, nb);
-    const float wt[6] = {wz, wz, wy, wy, wx, wx};
-    for (int ch = 0; ch < g.C; ++ch) {
-      const float p = g.data[t0 + ch];
-      float add = 0.f;
-#pragma unroll
-      for (int q = 0; q < 6; ++q) {
-        if (nb[q] == -2) continue;
-        const float vn = nb[q] < 0 ? g.background : g.data[int64_t(nb[q]) * g.C + ch];
-        add = __fadd_rn(add, __fmul_rn(wt[q], tv_clamp(p - vn)));
-      }
-      tv[t0 + ch] = add;
-    }
-  }
-}
-
-__global__ void k_tv_terms_c12(GridView g, float wx, float wy, float wz,
-                               const int32_t* __restrict__ list,
-                               const uint32_t* __restrict__ count, float* __restrict__ tv) {
-  grid_dep_sync();
-  const int64_t nl = *count;
-  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < nl * kLeafVox;
-       i += int64_t(gridDim.x) * blockDim.x) {
-    const int leaf = list[i >> 9];
-    const int vox = int(i & 511);
-    int fl[6];
-    face_leaves(g, leaf, fl);
-    if (!is_active(g, leaf, vox)) continue;
-    const int64_t t0 = (int64_t(leaf) * kLeafVox + vox) * 12;
-    float4* o4 = reinterpret_cast<float4*>(tv + t0);
-    int x, y, z;
-    slot_coord(g, leaf, vox, x, y, z);
-    if (x >= g.reso[0] || y >= g.reso[1] || z >= g.reso[2]) {
-#pragma unroll
-      for (int b = 0; b < 3; ++b) o4[b] = make_float4(0.f, 0.f, 0.f, 0.f);
-      continue;
-    }
-    int nb[6];
-    face_neighbours(g, leaf, vox, x, y, z, fl, nb);
-    const float wt[6] = {wz, wz, wy, wy, wx, wx};
-    float p[12], add[12];
-    const float4* d4 = reinterpret_cast<const float4*>(g.data + t0);
-#pragma unroll
-    for (int b = 0; b < 3; ++b) {
-      const float4 v = d4[b];
-      p[4 * b] = v.x; p[4 * b + 1] = v.y; p[4 * b + 2] = v.z; p[4 * b + 3] = v.w;
-    }
-#pragma unroll
-    for (int ch = 0; ch < 12; ++ch) add[ch] = 0.f;
-#pragma unroll
-    for (int q = 0; q < 6; ++q) {
-      if (nb[q] == -2) continue;
-      float vn[12];
-      if (nb[q] < 0) {
-#pragma unroll
-        for (int ch = 0; ch < 12; ++ch) vn[ch] = g.background;
-      } else {
-        const float4* n4 = reinterpret_cast<const float4*>(g.data + int64_t(nb[q]) * 12);
-#pragma unroll
-        for (int b = 0; b < 3; ++b) {
-          const float4 v = n4[b];
-          vn[4 * b] = v.x; vn[4 * b + 1] = v.y; vn[4 * b + 2] = v.z; vn[4 * b + 3] = v.w;
-        }
-      }
-#pragma unroll
-      for (int ch = 0; ch < 12; ++ch)
-        add[ch] = __fadd_rn(add[ch], __fmul_rn(wt[q], tv_clamp(p[ch] - vn[ch])));
-    }
-#pragma unroll
-    for (int b = 0; b < 3; ++b)
-      o4[b] = make_float4(add[4 * b], add[4 * b + 1], add[4 * b + 2], add[4 * b + 3]);
   }
 }
 
@@ -673,12 +624,8 @@ int tv_terms_launch(pvdb_grid_s* g, float wx, float wy, float wz, cudaStream_t s
   wx /= 6.f;
   wy /= 6.f;
   wz /= 6.f;
-  if (g->C == 12)
-    launch_k(k_tv_terms_c12, stride_grid(), 256, 0, st, g->view(), wx, wy, wz, g->d_tlist,
-             g->d_tcount, g->d_tv);
-  else
-    launch_k(k_tv_terms, stride_grid(), 256, 0, st, g->view(), wx, wy, wz, g->d_tlist, g->d_tcount,
-             g->d_tv);
+  launch_k(g->C == 12 ? k_tv_c12<true> : k_tv<true>, stride_grid(), 256, 0, st, g->view(), wx, wy,
+           wz, 0, g->d_tlist, g->d_tcount, g->d_tv);
   PVDB_CHECK_LAUNCH("k_tv_terms");
   return PVDB_OK;
 }
@@ -1023,12 +970,8 @@ int pvdb_grid_tv_add_grad(pvdb_grid g, float wx, float wy, float wz, int32_t den
     int rc = touched_list(g, st);
     if (rc) return rc;
   }
-  if (g->C == 12)
-    launch_k(k_tv_c12, stride_grid(), 256, 0, st, g->view(), wx, wy, wz, dense_mode ? 1 : 0,
-             use_list ? g->d_tlist : nullptr, g->d_tcount);
-  else
-    launch_k(k_tv, stride_grid(), 256, 0, st, g->view(), wx, wy, wz, dense_mode ? 1 : 0,
-             use_list ? g->d_tlist : nullptr, g->d_tcount);
+  launch_k(g->C == 12 ? k_tv_c12<false> : k_tv<false>, stride_grid(), 256, 0, st, g->view(), wx, wy,
+           wz, dense_mode ? 1 : 0, use_list ? g->d_tlist : nullptr, g->d_tcount, nullptr);
   PVDB_CHECK_LAUNCH("k_tv");
   if (dense_mode) g->all_touched = true;
   return PVDB_OK;

@@ -285,11 +285,13 @@ constexpr uint32_t kChainSpinMax = 1u << 24;
 __global__ void __launch_bounds__(kMarchThreads)
     k_march_chain(int R, MarchP P, MarchW W, uint32_t spin_max, int hold_first) {
   grid_dep_sync();
+  __shared__ __align__(16) float kept_alpha[kMarchWarps][36];
   const int lane = threadIdx.x & 31;
   uint32_t ticket = 0;
   if (lane == 0) ticket = atomicAdd(W.totals + 6, 1u);
   const int r = int(__shfl_sync(0xffffffffu, ticket, 0));
   if (r >= R) return;
+  float* buf = kept_alpha[threadIdx.x >> 5];
   const unsigned lt = lanemask_lt();
   const int64_t sbase = int64_t(r) * P.cap;
   int nk = 0, nc = 0;
@@ -311,21 +313,36 @@ __global__ void __launch_bounds__(kMarchThreads)
         if (stop) continue;
         const int k = b0 + 32 * j + lane;
         unsigned km = __ballot_sync(0xffffffffu, al[j] > P.thr);
-        // alpha2weight over the kept lanes, in sample order (uniform across the warp)
-        float w = 0.f;
-        unsigned rem = km;
-        while (rem) {
-          const int l = __ffs(rem) - 1;
-          rem &= rem - 1;
-          const float a = __shfl_sync(0xffffffffu, al[j], l);
-          const float wl = T * a;
-          if (lane == l) w = wl;
-          T = trans_step(T, a);
-          if (T < P.t_stop) {
-            km &= (l == 31) ? 0xffffffffu : ((2u << l) - 1u);
-            stop = true;
-            break;
+        if (!km) continue;  // uniform: most chunks of a ray hold no kept sample
+        // alpha2weight over the kept samples in order. Their alphas are packed
+        // and read back by every lane, so that the chain is one dependent FMA a
+        // sample (fetching each from its lane cost some 60 cycles a sample);
+        // entries behind the last are zero and leave T as it is. A lane keeps
+        // the T before its own sample.
+        const int rank = __popc(km & lt), nkc = __popc(km);
+        const bool in = (km >> lane) & 1u;
+        if (in) buf[rank] = al[j];
+        if (lane >= nkc && lane < nkc + 4) buf[lane] = 0.f;
+        __syncwarp();
+        float before = 0.f;
+        for (int i = 0; i < nkc; i += 4) {
+          const float4 a4 = *reinterpret_cast<const float4*>(buf + i);
+          const float a[4] = {a4.x, a4.y, a4.z, a4.w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            if (rank == i + e) before = T;
+            T = trans_step(T, a[e]);
           }
+        }
+        __syncwarp();  // the alphas are read: the next chunk's may be written
+        const float w = in ? before * al[j] : 0.f;
+        const float after = trans_step(before, al[j]);
+        const unsigned sm = __ballot_sync(0xffffffffu, in && after < P.t_stop);
+        if (sm) {  // the chain ends behind the first such sample
+          const int l = __ffs(sm) - 1;
+          km &= (l == 31) ? 0xffffffffu : ((2u << l) - 1u);
+          T = __shfl_sync(0xffffffffu, after, l);
+          stop = true;
         }
         const bool kept = (km >> lane) & 1u;
         const bool col = kept && (w > P.thr);

@@ -102,11 +102,14 @@ static int pe_launch(const float* viewdirs, int R, const MlpArgs& a, float* pe, 
 // Sum of the per-CTA partials: eight interleaved running sums (partials c,
 // c+8, ...) combined in a fixed order, so the loads of eight partials are in
 // flight together and the result is the same on every run.
+// Only the CTAs that had a tile wrote one (a batch smaller than the grid).
 // 256 threads per 32 parameters: warp u sums the partials c = u, u+8, ... in
 // increasing c, then the 8 warp sums combine as ((s0+s1)+(s2+s3))+((s4+s5)+(s6+s7)).
 __global__ void __launch_bounds__(256)
-    k_wgrad_reduce(const float* __restrict__ wpart, int nparts, int64_t P, float* out) {
+    k_wgrad_reduce(const float* __restrict__ wpart, int grid, int tensor_cores,
+                   const uint32_t* __restrict__ totals, int64_t P, float* out) {
   grid_dep_sync();
+  const int nparts = active_parts(totals[1], grid, tensor_cores);
   __shared__ float part[8][33];
   const int u = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t i = blockIdx.x * 32ll + lane;
@@ -260,14 +263,16 @@ int mlp_backward_impl(pvdb_march_s* m, const MlpArgs& a, const float* k0rows, co
                               &m->mlp_packed_cap, &m->mlp_xt, &m->mlp_xt_cap, m->w.totals + 3, st,
                               prepared ? 1 : 0, prepared ? 1 : 0);
     if (rc) return rc;
-    launch_k(k_wgrad_reduce, ceil_div(P, 32), 256, 0, st, m->wpart, G, P, grad_flat);
+    launch_k(k_wgrad_reduce, ceil_div(P, 32), 256, 0, st, m->wpart, G, precision, m->w.totals,
+             P, grad_flat);
     PVDB_CHECK_LAUNCH("k_wgrad_reduce");
     return PVDB_OK;
   }
   rc = mlp_f32_backward(a, k0rows, m->w.r_ray, m->hpe, m->hpe + size_t(m->max_rays) * kW,
                         m->w.totals, rgb, grad_rgb, grad_k0, m->wpart, G, st);
   if (rc) return rc;
-  launch_k(k_wgrad_reduce, ceil_div(P, 32), 256, 0, st, m->wpart, G, P, grad_flat);
+  launch_k(k_wgrad_reduce, ceil_div(P, 32), 256, 0, st, m->wpart, G, precision, m->w.totals,
+             P, grad_flat);
   PVDB_CHECK_LAUNCH("k_wgrad_reduce");
   return PVDB_OK;
 }

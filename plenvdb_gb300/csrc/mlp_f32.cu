@@ -27,23 +27,6 @@ constexpr int kW = 128;        // hidden width
 constexpr int kLd = kW + 4;    // row stride of a 128-wide tile (4 mod 32 words)
 constexpr int kPeStride = 32;  // PE floats per ray
 
-// Row tiles of one CTA (or group): `full` rounds of 128-row tiles over all
-// units, then 32-row tiles. The remainder takes a further round of 128-row
-// tiles when it would need more than three rounds of 32-row tiles.
-struct TilePlan {
-  int64_t full;   // 128-row tiles, tile t to unit t % units
-  int64_t row32;  // first row of the 32-row tiles
-};
-__device__ __forceinline__ TilePlan tile_plan(int64_t M, int64_t units) {
-  TilePlan p;
-  const int64_t rounds = M / (128 * units);
-  p.full = rounds * units;
-  const int64_t rem = M - p.full * 128;
-  if (rem > 3 * 32 * units) p.full += (rem + 127) / 128;
-  p.row32 = p.full * 128;
-  return p;
-}
-
 __device__ __forceinline__ void bar_group(int id, int threads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
@@ -612,7 +595,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
   for (int e = 0; e < 8; ++e) A.m128[e] = 0.f;
   A.m32[0] = A.m32[1] = 0.f;
   A.b2 = 0.f;
-  if (int64_t(blockIdx.x) < P.full || P.row32 + 32ll * blockIdx.x < M) {
+  if (blockIdx.x >= active_parts(M, gridDim.x, false)) return;
+  {
     for (int i = tid; i < kW * kW / 4; i += kBwdThreads) {
       const int n = i / (kW / 4), k = 4 * (i % (kW / 4));
       *reinterpret_cast<float4*>(B.w1 + n * kLd + k) =
@@ -627,7 +611,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
     bwd_tile<128, CQ>(B, A, a, in, i * 128, M);
   for (int64_t r = P.row32 + 32ll * blockIdx.x; r < M; r += 32ll * gridDim.x)
     bwd_tile<32, CQ>(B, A, a, in, r, M);
-  // this CTA's partials (zeros if it had no tile)
+  // this CTA's partials
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll

@@ -450,10 +450,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
   float* pb1 = pw1 + kW * kW;
   float* pw2 = pb1 + kW;
   float* pb2 = pw2 + 3 * kW;
-  if (blockIdx.x >= ntiles) {
-    for (int64_t i = tid; i < P; i += kBwdThreads) pw0[i] = 0.f;
-    return;
-  }
+  if (blockIdx.x >= ntiles) return;  // no partial either (active_parts)
   // this CTA's tiles: t_j = blockIdx.x + j * gridDim.x, j < nj; tile j goes to slot j & 1
   const int nj = int((ntiles - blockIdx.x + gridDim.x - 1) / gridDim.x);
   uint64_t* mbar = reinterpret_cast<uint64_t*>(sm + kBBar);  // [2] MMA stage done
