@@ -214,7 +214,9 @@ def check(rc: int):
 
 
 def call(name: str, *args):
-    check(getattr(load(), name)(*args))
+    rc = getattr(_lib or load(), name)(*args)
+    if rc != PVDB_OK:
+        check(rc)
 
 
 # ---------------------------------------------------------------- pointers

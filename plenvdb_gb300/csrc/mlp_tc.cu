@@ -10,7 +10,10 @@
 //   L0  Z0 = X . W0f^T            3 MMAs (K=48)        H0 = relu(Z0)
 //   L1  Z1 = H0 . W1^T            8 MMAs (K=128)       H1 = relu(Z1 + b1)
 //   L2  Z2 = H1 . W2p^T           8 MMAs, N=16         rgb = sigmoid(Z2 + b2)
-// X tiles are built beforehand and fetched with bulk copies. A tile is a chain
+// X tiles are built beforehand and fetched with bulk copies, or (GATHER, the
+// renderer's BF16 features) formed by the slot's own threads, a row a thread,
+// while the tensor cores run the previous tile's layer 1: the rows are then
+// never written out. A tile is a chain
 // of three MMA batches and three epilogues, so the kernel is bound by that
 // chain's latency and by how many chains an SM keeps going: one persistent CTA
 // per SM shares the 48 KB of weights between four independent warpgroups, each
@@ -21,6 +24,7 @@
 #include <algorithm>
 
 #include "march.cuh"
+#include "render_rows.cuh"
 #include "tc.cuh"
 
 namespace pvdb {
@@ -181,10 +185,11 @@ __device__ __forceinline__ void slot_sync(int slot) {
 
 // out [M, 3]: sigmoid(Z2 + b2), times rw [M] when given (a row's contribution to
 // its pixel).
+template <bool GATHER>
 __global__ void __launch_bounds__(kFwdThreads, 1)
     k_mlp_fwd_tc(MlpArgsTc a, const uint8_t* __restrict__ blob, const uint8_t* __restrict__ xt,
-                 const uint32_t* __restrict__ totals, float* out, const float* __restrict__ rw,
-                 uint32_t* err) {
+                 RowSource src, const uint32_t* __restrict__ totals, float* out,
+                 const float* __restrict__ rw, uint32_t* err) {
   grid_dep_sync();
   extern __shared__ __align__(1024) uint8_t sm[];
   const int64_t M = totals[1];
@@ -216,7 +221,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
     *flag = 0;
     tc::mbar_init(bar, 1);
     tc::mbar_init(xbar, 1);
-    if (u < ntiles) x_fetch(sx, xt, u, xbar);
+    if (!GATHER && u < ntiles) x_fetch(sx, xt, u, xbar);
   }
   if (tid < 32) {
     tc::tmem_alloc(tmem_slot, kTmemCols);
@@ -247,9 +252,13 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
     slot_sync(slot);
     return *((volatile uint32_t*)flag) == 0;
   };
-  for (int64_t t = u; t < ntiles; t += stride) {
+  if (GATHER && u < ntiles) {
+    write_x_row(src, u * 128 + row, M, row, sx);
+    ok = slot_ok();
+  }
+  for (int64_t t = u; ok && t < ntiles; t += stride) {
     if (row == 0) {
-      wait(xbar, xph);
+      if (!GATHER) wait(xbar, xph);
       if (t == u) wait(wbar, 0);
       tc::fence_after();
 #pragma unroll
@@ -263,7 +272,8 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
     phase ^= 1u;
     tc::fence_after();
     // the X tile is read: the next one travels from here
-    x_out = t + stride < ntiles;
+    const bool more = t + stride < ntiles;
+    x_out = !GATHER && more;
     if (row == 0 && x_out) x_fetch(sx, xt, t + stride, xbar);
     // ---- H0 = relu(Z0)
     epilogue_relu(t_lane, sh, row, nullptr);
@@ -276,6 +286,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
                      tc::make_desc(sbase + kOffW1 + 256 * s, 128, 2048), id_n128, s > 0);
       tc::mma_commit(bar);
     }
+    if (GATHER && more) write_x_row(src, (t + stride) * 128 + row, M, row, sx);
     wait(bar, phase);
     phase ^= 1u;
     tc::fence_after();
@@ -876,11 +887,27 @@ int mlp_tc_forward_rows(const float* w0, const float* b0, const float* w1, const
                                        xt_cap, st)))
     return rc;
   MlpArgsTc a{w0, b0, w1, b1, w2, b2, c0, dpe, c0 + dpe};
-  PVDB_SMEM_ATTR(k_mlp_fwd_tc, int(kSmFwdBytes));
-  launch_k(k_mlp_fwd_tc, num_sms(), kFwdThreads, kSmFwdBytes, st, a,
-           static_cast<const uint8_t*>(*blob), static_cast<const uint8_t*>(*xt), totals, out,
-           rw, err);
+  PVDB_SMEM_ATTR(k_mlp_fwd_tc<false>, int(kSmFwdBytes));
+  launch_k(k_mlp_fwd_tc<false>, num_sms(), kFwdThreads, kSmFwdBytes, st, a,
+           static_cast<const uint8_t*>(*blob), static_cast<const uint8_t*>(*xt), RowSource{}, totals,
+           out, rw, err);
   PVDB_CHECK_LAUNCH("k_mlp_fwd_tc");
+  return PVDB_OK;
+}
+
+// The forward over the renderer's rows (12 BF16 feature channels, 27 PE
+// values), X rows formed from src by the kernel itself.
+int mlp_tc_forward_gather(const float* w0, const float* b0, const float* w1, const float* b1,
+                          const float* w2, const float* b2, int c0, int dpe, const RowSource& src,
+                          const uint32_t* totals, float* out, const float* rw, void** blob,
+                          size_t* blob_cap, uint32_t* err, cudaStream_t st) {
+  const int rc = mlp_tc_pack(w0, b0, w1, b1, w2, b2, c0, dpe, blob, blob_cap, st);
+  if (rc) return rc;
+  MlpArgsTc a{w0, b0, w1, b1, w2, b2, c0, dpe, c0 + dpe};
+  PVDB_SMEM_ATTR(k_mlp_fwd_tc<true>, int(kSmFwdBytes));
+  launch_k(k_mlp_fwd_tc<true>, num_sms(), kFwdThreads, kSmFwdBytes, st, a,
+           static_cast<const uint8_t*>(*blob), nullptr, src, totals, out, rw, err);
+  PVDB_CHECK_LAUNCH("k_mlp_fwd_tc<gather>");
   return PVDB_OK;
 }
 

@@ -18,7 +18,8 @@
 //                          position, weight and pixel to the frame's rows
 //   k_render_pe / k_render_x (BF16), k_render_k0 (FP32)
 //                          per row: the trilinear features (renderer.cu:303-310)
-//                          into the rgbnet's X tiles or k0 rows
+//                          into the rgbnet's X tiles or k0 rows; with BF16
+//                          features the BF16 rgbnet gathers them itself
 //   rgbnet                 the MLP on all rows (PE part once per pixel), each
 //                          row's w/(1+exp(-logit))
 //   k_render_composite     per pixel: T*bg + the sum of its rows in sample
@@ -37,6 +38,7 @@
 #include <vector>
 
 #include "pvdb_internal.cuh"
+#include "render_rows.cuh"
 #include "tc.cuh"
 
 namespace pvdb {
@@ -52,6 +54,10 @@ int mlp_forward_rows(const MlpArgs& a, const float* k0rows, const int32_t* ray,
                      int64_t max_rows, const float* rw, float* out, float* hpe_buf, int precision,
                      void** blob, size_t* blob_cap, void** xt, size_t* xt_cap, uint32_t* err,
                      cudaStream_t st);
+int mlp_tc_forward_gather(const float* w0, const float* b0, const float* w1, const float* b1,
+                          const float* w2, const float* b2, int c0, int dpe, const RowSource& src,
+                          const uint32_t* totals, float* out, const float* rw, void** blob,
+                          size_t* blob_cap, uint32_t* err, cudaStream_t st);
 
 struct RenderP {
   int H, W, inverse_y;
@@ -66,7 +72,7 @@ struct RenderP {
   // (the leaf table holds -d for a block with no leaf, d the Chebyshev distance
   // in blocks to the nearest leaf)
   GridView idx;               // topology; values unused
-  int64_t nslots;
+  int nslots;
   const float* vden;          // [nslots + 1]
   const float* vcol;          // [nslots + 1][12] (12 channels, storage 0)
   const __nv_bfloat16* vcolh; // [nslots + 1][kHalfStride] (12 channels, storage 1)
@@ -125,19 +131,6 @@ __device__ __forceinline__ void pixel_ray(const RenderP& P, int n, PixelRay& r) 
     r.o[a] = __fdiv_rn(P.c2w[4 * a + 3] - P.mn[a], ext);
     r.d[a] = __fdiv_rn(r.rd[a], ext);
   }
-}
-
-// Slots of the 8 corners of the sample's cell (int() truncation,
-// renderer.cu:271-300), P.nslots where a corner lies in no allocated leaf, and
-// their scales.
-__device__ __forceinline__ void cell_corners(const RenderP& P, const float xyz[3], int64_t s[8],
-                                             float sc[8]) {
-  const int i = int(xyz[0]), j = int(xyz[1]), k = int(xyz[2]);
-  int s8[8];
-  corner_slots(P.idx, i, j, k, s8);
-#pragma unroll
-  for (int c = 0; c < 8; ++c) s[c] = s8[c] < 0 ? P.nslots : int64_t(s8[c]);
-  corner_scales(xyz[0] - float(i), xyz[1] - float(j), xyz[2] - float(k), sc);
 }
 
 // advance: t after n additions of step, each rounded. While t stays between
@@ -297,9 +290,9 @@ __global__ void __launch_bounds__(128)
       const float xyz[3] = {__fmul_rn(__fmaf_rn(te, dx, r.o[0]), P.wsm1[0]),
                             __fmul_rn(__fmaf_rn(te, dy, r.o[1]), P.wsm1[1]),
                             __fmul_rn(__fmaf_rn(te, dz, r.o[2]), P.wsm1[2])};
-      int64_t slot[8];
+      int slot[8];
       float sc[8];
-      cell_corners(P, xyz, slot, sc);
+      cell_corners(P.idx, P.nslots, xyz, slot, sc);
       float val[8];
 #pragma unroll
       for (int q = 0; q < 8; ++q) val[q] = __ldg(P.vden + slot[q]);
@@ -397,35 +390,24 @@ __device__ __forceinline__ void row_features(const RenderP& P, const RenderW& Wk
                                              float* acc) {
   const float xyz[3] = {__ldg(Wk.rxyz + m * 3), __ldg(Wk.rxyz + m * 3 + 1),
                         __ldg(Wk.rxyz + m * 3 + 2)};
-  int64_t slot[8];
+  if (CT == 12 && P.storage == 1) {
+    features12_bf16(P.idx, P.nslots, P.vcolh, xyz, acc);
+    return;
+  }
+  int slot[8];
   float sc[8];
-  cell_corners(P, xyz, slot, sc);
+  cell_corners(P.idx, P.nslots, xyz, slot, sc);
   if (CT == 12) {
-    if (P.storage == 0) {
+    {
 #pragma unroll
       for (int c = 0; c < 8; ++c) {
-        const float4* src = reinterpret_cast<const float4*>(P.vcol + slot[c] * 12);
+        const float4* src = reinterpret_cast<const float4*>(P.vcol + int64_t(slot[c]) * 12);
         float v[12];
 #pragma unroll
         for (int b = 0; b < 3; ++b) *reinterpret_cast<float4*>(v + 4 * b) = __ldg(src + b);
 #pragma unroll
         for (int q = 0; q < 12; ++q)
           acc[q] = c == 0 ? __fmul_rn(v[q], sc[0]) : __fmaf_rn(v[q], sc[c], acc[q]);
-      }
-    } else {
-#pragma unroll
-      for (int c0 = 0; c0 < 8; c0 += 4) {
-        uint32_t w[4][8];
-#pragma unroll
-        for (int c = 0; c < 4; ++c) ld_nc32(P.vcolh + slot[c0 + c] * kHalfStride, w[c]);
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-#pragma unroll
-          for (int q = 0; q < 12; ++q) {
-            const float v =
-                __uint_as_float(q & 1 ? w[c][q >> 1] & 0xFFFF0000u : w[c][q >> 1] << 16);
-            acc[q] = c0 + c == 0 ? __fmul_rn(v, sc[0]) : __fmaf_rn(v, sc[c0 + c], acc[q]);
-          }
       }
     }
     return;
@@ -979,7 +961,7 @@ int pvdb_renderer_render(pvdb_renderer r, int32_t precision, pvdb_stream s) {
   P.t_stop = r->t_stop;
   P.dcol = r->dcol;
   P.idx = r->topo->view();
-  P.nslots = r->topo->nslots();
+  P.nslots = int(r->topo->nslots());
   P.vden = r->d_vden;
   P.rows = r->d_rows;
   P.vcol = P.col = r->d_col;
@@ -1031,21 +1013,25 @@ int pvdb_renderer_render(pvdb_renderer r, int32_t precision, pvdb_stream s) {
   a.c0 = r->dcol;
   a.dpe = r->dpe;
   a.din = din;
+  // 12 BF16 channels and the BF16 rgbnet: the rgbnet gathers the features itself
+  const bool gather = precision == 1 && r->dcol == 12 && r->storage == 1;
+  uint4* pex = reinterpret_cast<uint4*>(r->d_hpe);  // 96 of the 640 bytes a pixel
   if (total) {
     const int64_t M = total;
     const int rgrid = ceil_div((M + 127) / 128 * 128, 256);
     if (precision == 1) {
-      const int64_t ntiles = (r->rows_cap + 127) / 128;
-      if ((rc = dev_reserve(&r->d_xt, &r->xt_cap, size_t(ntiles) * kRgbXTile))) return rc;
-      uint4* pex = reinterpret_cast<uint4*>(r->d_hpe);  // 96 of the 640 bytes a pixel
-      uint8_t* xt = static_cast<uint8_t*>(r->d_xt);
       k_render_pe<<<ceil_div(int64_t(HW) * 6, 192), 192, 0, st>>>(P, Wk, (r->dpe - 3) / 6, pex);
       PVDB_CHECK_LAUNCH("k_render_pe");
-      if (r->dcol == 12)
-        k_render_x<12><<<rgrid, 256, 0, st>>>(P, Wk, M, pex, xt);
-      else
-        k_render_x<0><<<rgrid, 256, 0, st>>>(P, Wk, M, pex, xt);
-      PVDB_CHECK_LAUNCH("k_render_x");
+      if (!gather) {
+        const int64_t ntiles = (r->rows_cap + 127) / 128;
+        if ((rc = dev_reserve(&r->d_xt, &r->xt_cap, size_t(ntiles) * kRgbXTile))) return rc;
+        uint8_t* xt = static_cast<uint8_t*>(r->d_xt);
+        if (r->dcol == 12)
+          k_render_x<12><<<rgrid, 256, 0, st>>>(P, Wk, M, pex, xt);
+        else
+          k_render_x<0><<<rgrid, 256, 0, st>>>(P, Wk, M, pex, xt);
+        PVDB_CHECK_LAUNCH("k_render_x");
+      }
     } else {
       if (r->dcol == 12)
         k_render_k0<12><<<rgrid, 256, 0, st>>>(P, Wk, M);
@@ -1055,7 +1041,13 @@ int pvdb_renderer_render(pvdb_renderer r, int32_t precision, pvdb_stream s) {
     }
   }
   prof_mark(st, 3);
-  if (total) {
+  if (total && gather) {
+    const RowSource src{P.idx, P.nslots, P.vcolh, r->d_rxyz, r->d_rpix, pex};
+    rc = mlp_tc_forward_gather(a.w0, a.b0, a.w1, a.b1, a.w2, a.b2, a.c0, a.dpe, src, r->d_totals,
+                               r->d_part, r->d_rw, &r->d_packed, &r->packed_cap, r->d_totals + 3,
+                               st);
+    if (rc) return rc;
+  } else if (total) {
     rc = mlp_forward_rows(a, r->d_rk0, r->d_rpix, r->d_viewdirs, HW, r->d_n, r->d_totals,
                           r->rows_cap, r->d_rw, r->d_part, r->d_hpe, precision, &r->d_packed,
                           &r->packed_cap, &r->d_xt, &r->xt_cap, r->d_totals + 3, st);

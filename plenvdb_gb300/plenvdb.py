@@ -51,6 +51,14 @@ def _dev_f32(t):
     return t.contiguous()
 
 
+def _dev_flat(t):
+    """_dev_f32 as a flat tensor; t itself where it is one already."""
+    import torch
+    if t.dim() == 1 and t.dtype == torch.float32 and t.is_contiguous():
+        return t
+    return _dev_f32(t).reshape(-1)
+
+
 class _CudaArray:
     """Minimal __cuda_array_interface__ holder to view library memory in torch."""
 
@@ -195,7 +203,7 @@ class BaseVDB:
         t0 = time.perf_counter()
         if L.is_cuda(x):
             import torch
-            xs, ys, zs = _dev_f32(x).reshape(-1), _dev_f32(y).reshape(-1), _dev_f32(z).reshape(-1)
+            xs, ys, zs = _dev_flat(x), _dev_flat(y), _dev_flat(z)
             n = xs.numel()
             if ys.numel() != n or zs.numel() != n:
                 raise ValueError("x, y, z must have the same length")
@@ -216,8 +224,8 @@ class BaseVDB:
 
     def backward(self, x, y, z, g):
         if L.is_cuda(x):
-            xs, ys, zs = _dev_f32(x).reshape(-1), _dev_f32(y).reshape(-1), _dev_f32(z).reshape(-1)
-            gg = _dev_f32(g).reshape(-1)
+            xs, ys, zs = _dev_flat(x), _dev_flat(y), _dev_flat(z)
+            gg = _dev_flat(g)
             n = xs.numel()
             if gg.numel() != n * self.ndim:
                 raise ValueError("grad must have len(x) * ndim entries")
@@ -245,7 +253,7 @@ class BaseVDB:
 
     def copyFromDense(self, arr, which: int = L.WHICH_DATA):
         if L.is_cuda(arr):
-            a = _dev_f32(arr).reshape(-1)
+            a = _dev_flat(arr)
             L.call("pvdb_grid_copy_from_dense", self.handle, which, L.ptr(a), a.numel(),
                    L.MEM_DEVICE, L.stream_of())
         else:
@@ -380,7 +388,7 @@ class _BaseOpt:
 
     def set_grad(self, arr):
         if L.is_cuda(arr):
-            a = _dev_f32(arr).reshape(-1)
+            a = _dev_flat(arr)
             L.call("pvdb_opt_set_grad", self.h, L.ptr(a), a.numel(), L.MEM_DEVICE, L.stream_of())
         else:
             a = _as_host_f32(arr).reshape(-1)
@@ -388,7 +396,7 @@ class _BaseOpt:
 
     def set_pervoxel_lr(self, count):
         if L.is_cuda(count):
-            a = _dev_f32(count).reshape(-1)
+            a = _dev_flat(count)
             L.call("pvdb_opt_set_pervoxel_lr", self.h, L.ptr(a), a.numel(), L.MEM_DEVICE,
                    L.stream_of())
         else:
