@@ -253,10 +253,13 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
     return *((volatile uint32_t*)flag) == 0;
   };
   if (GATHER && u < ntiles) {
-    write_x_row(src, u * 128 + row, M, row, sx);
+    write_x_row(src, load_row_pos(src, u * 128 + row, M), row, sx);
     ok = slot_ok();
   }
   for (int64_t t = u; ok && t < ntiles; t += stride) {
+    const bool more = t + stride < ntiles;
+    RowPos next;
+    if (GATHER) next = load_row_pos(src, (t + stride) * 128 + row, M);
     if (row == 0) {
       if (!GATHER) wait(xbar, xph);
       if (t == u) wait(wbar, 0);
@@ -272,7 +275,6 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
     phase ^= 1u;
     tc::fence_after();
     // the X tile is read: the next one travels from here
-    const bool more = t + stride < ntiles;
     x_out = !GATHER && more;
     if (row == 0 && x_out) x_fetch(sx, xt, t + stride, xbar);
     // ---- H0 = relu(Z0)
@@ -286,7 +288,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
                      tc::make_desc(sbase + kOffW1 + 256 * s, 128, 2048), id_n128, s > 0);
       tc::mma_commit(bar);
     }
-    if (GATHER && more) write_x_row(src, (t + stride) * 128 + row, M, row, sx);
+    if (GATHER && more) write_x_row(src, next, row, sx);
     wait(bar, phase);
     phase ^= 1u;
     tc::fence_after();
