@@ -17,10 +17,13 @@
 // of three MMA batches and three epilogues, so the kernel is bound by that
 // chain's latency and by how many chains an SM keeps going: one persistent CTA
 // per SM shares the 48 KB of weights between four independent warpgroups, each
-// with its own tile, 128 TMEM columns (Z0, Z1 and Z2 in turn), barriers and
-// issuing thread. Epilogues read TMEM with tcgen05.ld (thread = tile row),
-// apply bias/activation in FP32 and store BF16 into shared memory in the
-// canonical layout the next MMA reads.
+// with its own tile, 128 TMEM columns (Z0 and Z1 in turn, then H1 and Z2),
+// barriers and issuing thread. Epilogues read TMEM with tcgen05.ld (thread =
+// tile row), apply bias/activation in FP32 and store BF16: H0 into shared memory
+// in the canonical layout the next MMA reads, H1 back into TMEM, from where L2
+// takes its A operand (512 cycles a tile of shared-memory traffic less; 800x800
+// frame 1496 -> 1480 us, 320^3 step 4831 -> 4807 us). Both in TMEM would take 192
+// columns a tile, so two tiles in flight instead of four.
 #include <algorithm>
 
 #include "march.cuh"
@@ -159,7 +162,9 @@ __device__ __forceinline__ void store_relu32(uint8_t* tile, int row, int col0, i
 }
 
 // relu(Z [+ bias]) of this thread's row, 128 columns, as BF16 into the K-major
-// tile; the TMEM load of a chunk travels while the previous one is packed.
+// tile, or (TO_TMEM) packed in pairs over the first 64 of the columns they were
+// read from; the TMEM load of a chunk travels while the previous one is packed.
+template <bool TO_TMEM>
 __device__ __forceinline__ void epilogue_relu(uint32_t taddr, uint8_t* tile, int row,
                                               const float* bias) {
   uint32_t r[2][32];
@@ -175,8 +180,21 @@ __device__ __forceinline__ void epilogue_relu(uint32_t taddr, uint8_t* tile, int
     float v[32];
 #pragma unroll
     for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[j & 1][i]);
-    store_relu32(tile, row, 32 * j, 128, v, bias);
+    if (TO_TMEM) {
+      // (columns 16 j .. 16 j + 15 were read before: the loads in flight are
+      // those of columns 32 (j + 1) and up)
+      uint32_t h[16];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const uint4 p = relu_pack8(v + 8 * c, bias, 32 * j + 8 * c);
+        h[4 * c] = p.x; h[4 * c + 1] = p.y; h[4 * c + 2] = p.z; h[4 * c + 3] = p.w;
+      }
+      tc::tmem_st16_issue(taddr + 16 * j, h);
+    } else {
+      store_relu32(tile, row, 32 * j, 128, v, bias);
+    }
   }
+  if (TO_TMEM) tc::tmem_wait_st();
 }
 
 __device__ __forceinline__ void slot_sync(int slot) {
@@ -278,7 +296,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
     x_out = !GATHER && more;
     if (row == 0 && x_out) x_fetch(sx, xt, t + stride, xbar);
     // ---- H0 = relu(Z0)
-    epilogue_relu(t_lane, sh, row, nullptr);
+    epilogue_relu<false>(t_lane, sh, row, nullptr);
     if (!(ok = slot_ok())) break;
     if (row == 0) {
       tc::fence_after();
@@ -292,15 +310,15 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
     wait(bar, phase);
     phase ^= 1u;
     tc::fence_after();
-    // ---- H1 = relu(Z1 + b1), over H0
-    epilogue_relu(t_lane, sh, row, b1s);
+    // ---- H1 = relu(Z1 + b1), over Z1's first 64 columns
+    epilogue_relu<true>(t_lane, nullptr, row, b1s);
     if (!(ok = slot_ok())) break;
     if (row == 0) {
       tc::fence_after();
 #pragma unroll
       for (int s = 0; s < 8; ++s)
-        tc::mma_bf16(d, tc::make_desc(hb + 256 * s, 128, 2048),
-                     tc::make_desc(sbase + kOffW2 + 256 * s, 128, 2048), id_n16, s > 0);
+        tc::mma_bf16_ta(d + 64, d + 8 * s, tc::make_desc(sbase + kOffW2 + 256 * s, 128, 2048),
+                        id_n16, s > 0);
       tc::mma_commit(bar);
     }
     wait(bar, phase);
@@ -308,7 +326,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
     tc::fence_after();
     // ---- logits
     float v[16];
-    tc::tmem_ld16(t_lane, v);
+    tc::tmem_ld16(t_lane + 64, v);
     const int64_t m = t * 128 + row;
     if (m < M) {
       const float w = rw ? __ldg(rw + m) : 1.f;
