@@ -213,7 +213,9 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
   const int64_t M = totals[1];
   const int64_t ntiles = (M + 127) / 128;
   if (blockIdx.x >= ntiles) return;
-  const int tid = threadIdx.x, slot = tid >> 7, row = tid & 127;
+  const int tid = threadIdx.x, row = tid & 127;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0), slot = warp >> 2;
+  const bool issuer = (warp & 3) == 0;  // the slot's warp that issues its MMAs
   uint64_t* bars = reinterpret_cast<uint64_t*>(sm + kSmBar);
   uint64_t* bar = bars + 2 * slot;       // this slot's MMAs
   uint64_t* xbar = bars + 2 * slot + 1;  // this slot's X tile
@@ -278,15 +280,18 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
     const bool more = t + stride < ntiles;
     RowPos next;
     if (GATHER) next = load_row_pos(src, (t + stride) * 128 + row, M);
-    if (row == 0) {
+    if (issuer) {
       if (!GATHER) wait(xbar, xph);
       if (t == u) wait(wbar, 0);
       tc::fence_after();
+      if (tc::elect_one()) {
 #pragma unroll
-      for (int s = 0; s < 3; ++s)
-        tc::mma_bf16(d, tc::make_desc(xb + 256 * s, 128, 768),
-                     tc::make_desc(sbase + kOffW0 + 256 * s, 128, 768), id_n128, s > 0);
-      tc::mma_commit(bar);
+        for (int s = 0; s < 3; ++s)
+          tc::mma_bf16(d, tc::make_desc(xb + 256 * s, 128, 768),
+                       tc::make_desc(sbase + kOffW0 + 256 * s, 128, 768), id_n128, s > 0);
+        tc::mma_commit(bar);
+      }
+      __syncwarp();
     }
     xph ^= 1u;
     wait(bar, phase);
@@ -298,13 +303,16 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
     // ---- H0 = relu(Z0)
     epilogue_relu<false>(t_lane, sh, row, nullptr);
     if (!(ok = slot_ok())) break;
-    if (row == 0) {
+    if (issuer) {
       tc::fence_after();
+      if (tc::elect_one()) {
 #pragma unroll
-      for (int s = 0; s < 8; ++s)
-        tc::mma_bf16(d, tc::make_desc(hb + 256 * s, 128, 2048),
-                     tc::make_desc(sbase + kOffW1 + 256 * s, 128, 2048), id_n128, s > 0);
-      tc::mma_commit(bar);
+        for (int s = 0; s < 8; ++s)
+          tc::mma_bf16(d, tc::make_desc(hb + 256 * s, 128, 2048),
+                       tc::make_desc(sbase + kOffW1 + 256 * s, 128, 2048), id_n128, s > 0);
+        tc::mma_commit(bar);
+      }
+      __syncwarp();
     }
     if (GATHER && more) write_x_row(src, next, row, sx);
     wait(bar, phase);
@@ -313,13 +321,16 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
     // ---- H1 = relu(Z1 + b1), over Z1's first 64 columns
     epilogue_relu<true>(t_lane, nullptr, row, b1s);
     if (!(ok = slot_ok())) break;
-    if (row == 0) {
+    if (issuer) {
       tc::fence_after();
+      if (tc::elect_one()) {
 #pragma unroll
-      for (int s = 0; s < 8; ++s)
-        tc::mma_bf16_ta(d + 64, d + 8 * s, tc::make_desc(sbase + kOffW2 + 256 * s, 128, 2048),
-                        id_n16, s > 0);
-      tc::mma_commit(bar);
+        for (int s = 0; s < 8; ++s)
+          tc::mma_bf16_ta(d + 64, d + 8 * s, tc::make_desc(sbase + kOffW2 + 256 * s, 128, 2048),
+                          id_n16, s > 0);
+        tc::mma_commit(bar);
+      }
+      __syncwarp();
     }
     wait(bar, phase);
     phase ^= 1u;
@@ -473,7 +484,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
   extern __shared__ __align__(1024) uint8_t sm[];
   const int64_t M = totals[1];
   const int64_t ntiles = (M + 127) / 128;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // (uniform for the compiler too)
   const int64_t P = int64_t(kW) * a.din + kW + kW * kW + kW + 3 * kW + 3;
   float* pw0 = wpart + int64_t(blockIdx.x) * P;
   float* pb0 = pw0 + kW * a.din;
@@ -531,90 +543,92 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
   const uint32_t tmem = *tmem_slot;
   const uint32_t sb = tc::smem_addr(sm);
   float db2[3] = {0.f, 0.f, 0.f};
-  uint32_t xwaits[kBwdXBufs] = {0u, 0u, 0u};  // X arrivals the issuer consumed, per buffer
+  int xdone = 0;  // X tiles the issuer saw land, in order: tile j in buffer j % kBwdXBufs
   bool wdone = false;             // the issuer saw the weight copy land
 
   if (warp == kBwdIssuer) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0 && !hold) {
+    // the whole warp waits, and goes on or leaves together; one elected lane issues
+    if (!hold) {
       const uint32_t id_kk = tc::idesc_bf16(128, 128);               // A, B K-major
       const uint32_t id_kn = tc::idesc_bf16(128, 128, false, true);  // B MN-major
       const uint32_t id_g = tc::idesc_bf16(128, 16, false, true);    // grad k0
       const uint32_t id_w2 = tc::idesc_bf16(128, 16, true, true);    // H1^T . dl
       const uint32_t id_w1 = tc::idesc_bf16(128, 144, true, true);   // dZ1^T . [H0|1]
       const uint32_t id_w0 = tc::idesc_bf16(128, 48, true, true);    // dZ0^T . X
-      uint32_t eph[2] = {0u, 0u};
+      uint32_t eph = 0u;  // bit s: parity of slot s's epilogue barrier
       bool w2_on = false, w1_on = false, w0_on = false;
-      bool ok = wdone = bwait(wbar, 0, flag, err, spin_max);
+      auto all_wait = [&](uint64_t* b, uint32_t parity) {
+        return bool(__all_sync(0xffffffffu, bwait(b, parity, flag, err, spin_max)));
+      };
+      bool ok = wdone = all_wait(wbar, 0);
       for (int pair = 0; ok && 2 * pair < nj; ++pair) {
-        for (int k = 0; ok && k < 5; ++k) {
+#pragma unroll
+        for (int k = 0; k < 5; ++k) {
+#pragma unroll 1
           for (int s = 0; ok && s < 2; ++s) {
             const int j = 2 * pair + s;
             if (j >= nj) continue;
             const int xb = j % kBwdXBufs;
             if (k == 0) {
-              ok = bwait(xbar + xb, xwaits[xb] & 1u, flag, err, spin_max);
-              if (ok) xwaits[xb]++;
+              ok = all_wait(xbar + xb, (j / kBwdXBufs) & 1u);
+              xdone += ok;
             } else {
-              ok = bwait(ebar + s, eph[s], flag, err, spin_max);
-              eph[s] ^= 1u;
+              ok = all_wait(ebar + s, (eph >> s) & 1u);
+              eph ^= 1u << s;
             }
             if (!ok) break;
             tc::fence_after();
-            // descriptors advance by (byte step >> 4) in their address field;
-            // the loops stay rolled so the single issuing thread keeps few
-            // registers live
             const uint32_t sl = sb + uint32_t(s) * kSlot;
             const uint32_t sx = sb + kBX + uint32_t(xb) * kXTile;
             const uint32_t tA = tmem + kTA0 + 128u * uint32_t(s);
-            if (k == 0) {  // Z0 = X . W0f^T
-              uint64_t da = tc::make_desc(sx, 128, 768);
-              uint64_t db = tc::make_desc(sb + kBW0f, 128, 768);
-#pragma unroll 1
-              for (int q = 0; q < 3; ++q, da += 256 >> 4, db += 256 >> 4)
-                tc::mma_bf16(tA, da, db, id_kk, q > 0);
-            } else if (k == 1) {  // Z1 = H0 . W1^T
-              uint64_t da = tc::make_desc(sl + kSlH0, 128, 2304);
-              uint64_t db = tc::make_desc(sb + kBW1, 128, 2048);
-#pragma unroll 1
-              for (int q = 0; q < 8; ++q, da += 256 >> 4, db += 256 >> 4)
-                tc::mma_bf16(tA, da, db, id_kk, q > 0);
-            } else if (k == 2) {  // dZ1' = dl . W2 -> A;  dW2 += H1^T . dl
-              tc::mma_bf16(tA, tc::make_desc(sl + kSlDl, 128, 256),
-                           tc::make_desc(sb + kBW2, 2048, 128), id_kn, 0u);
-              uint64_t da = tc::make_desc(sl + kSlH1, 2048, 128);
-              uint64_t db = tc::make_desc(sl + kSlDl, 256, 128);
-#pragma unroll 1
-              for (int q = 0; q < 8; ++q, da += 4096 >> 4, db += 512 >> 4)
-                tc::mma_bf16(tmem + kTW2, da, db, id_w2, (w2_on || q > 0) ? 1u : 0u);
-              w2_on = true;
-            } else if (k == 3) {  // dH0 = dZ1 . W1;  dW1|db1 += dZ1^T . [H0|1]
-              uint64_t da = tc::make_desc(sl + kSlH1, 128, 2048);
-              uint64_t db = tc::make_desc(sb + kBW1, 2048, 128);
-#pragma unroll 1
-              for (int q = 0; q < 8; ++q, da += 256 >> 4, db += 4096 >> 4)
-                tc::mma_bf16(tA, da, db, id_kn, q > 0);
-              da = tc::make_desc(sl + kSlH1, 2048, 128);
-              db = tc::make_desc(sl + kSlH0, 2304, 128);
-#pragma unroll 1
-              for (int q = 0; q < 8; ++q, da += 4096 >> 4, db += 4608 >> 4)
-                tc::mma_bf16(tmem + kTW1, da, db, id_w1, (w1_on || q > 0) ? 1u : 0u);
-              w1_on = true;
-            } else {  // grad k0 = dZ0 . W0k;  dW0|db0 += dZ0^T . X
-              const uint32_t tG = tmem + kTG0 + 16u * uint32_t(s);
-              uint64_t da = tc::make_desc(sl + kSlH1, 128, 2048);
-              uint64_t db = tc::make_desc(sb + kBW0f, 768, 128);
-#pragma unroll 1
-              for (int q = 0; q < 8; ++q, da += 256 >> 4, db += 1536 >> 4)
-                tc::mma_bf16(tG, da, db, id_g, q > 0);
-              da = tc::make_desc(sl + kSlH1, 2048, 128);
-              db = tc::make_desc(sx, 768, 128);
-#pragma unroll 1
-              for (int q = 0; q < 8; ++q, da += 4096 >> 4, db += 1536 >> 4)
-                tc::mma_bf16(tmem + kTW0, da, db, id_w0, (w0_on || q > 0) ? 1u : 0u);
-              w0_on = true;
+            if (tc::elect_one()) {
+              if (k == 0) {  // Z0 = X . W0f^T
+#pragma unroll
+                for (uint32_t q = 0; q < 3; ++q)
+                  tc::mma_bf16(tA, tc::make_desc(sx + 256 * q, 128, 768),
+                               tc::make_desc(sb + kBW0f + 256 * q, 128, 768), id_kk, q > 0);
+              } else if (k == 1) {  // Z1 = H0 . W1^T
+#pragma unroll
+                for (uint32_t q = 0; q < 8; ++q)
+                  tc::mma_bf16(tA, tc::make_desc(sl + kSlH0 + 256 * q, 128, 2304),
+                               tc::make_desc(sb + kBW1 + 256 * q, 128, 2048), id_kk, q > 0);
+              } else if (k == 2) {  // dZ1' = dl . W2 -> A;  dW2 += H1^T . dl
+                tc::mma_bf16(tA, tc::make_desc(sl + kSlDl, 128, 256),
+                             tc::make_desc(sb + kBW2, 2048, 128), id_kn, 0u);
+#pragma unroll
+                for (uint32_t q = 0; q < 8; ++q)
+                  tc::mma_bf16(tmem + kTW2, tc::make_desc(sl + kSlH1 + 4096 * q, 2048, 128),
+                               tc::make_desc(sl + kSlDl + 512 * q, 256, 128), id_w2,
+                               (w2_on || q > 0) ? 1u : 0u);
+              } else if (k == 3) {  // dH0 = dZ1 . W1;  dW1|db1 += dZ1^T . [H0|1]
+#pragma unroll
+                for (uint32_t q = 0; q < 8; ++q)
+                  tc::mma_bf16(tA, tc::make_desc(sl + kSlH1 + 256 * q, 128, 2048),
+                               tc::make_desc(sb + kBW1 + 4096 * q, 2048, 128), id_kn, q > 0);
+#pragma unroll
+                for (uint32_t q = 0; q < 8; ++q)
+                  tc::mma_bf16(tmem + kTW1, tc::make_desc(sl + kSlH1 + 4096 * q, 2048, 128),
+                               tc::make_desc(sl + kSlH0 + 4608 * q, 2304, 128), id_w1,
+                               (w1_on || q > 0) ? 1u : 0u);
+              } else {  // grad k0 = dZ0 . W0k;  dW0|db0 += dZ0^T . X
+                const uint32_t tG = tmem + kTG0 + 16u * uint32_t(s);
+#pragma unroll
+                for (uint32_t q = 0; q < 8; ++q)
+                  tc::mma_bf16(tG, tc::make_desc(sl + kSlH1 + 256 * q, 128, 2048),
+                               tc::make_desc(sb + kBW0f + 1536 * q, 768, 128), id_g, q > 0);
+#pragma unroll
+                for (uint32_t q = 0; q < 8; ++q)
+                  tc::mma_bf16(tmem + kTW0, tc::make_desc(sl + kSlH1 + 4096 * q, 2048, 128),
+                               tc::make_desc(sx + 1536 * q, 768, 128), id_w0,
+                               (w0_on || q > 0) ? 1u : 0u);
+              }
+              tc::mma_commit(mbar + s);
             }
-            tc::mma_commit(mbar + s);
+            __syncwarp();
+            w2_on = w2_on || k == 2;
+            w1_on = w1_on || k == 3;
+            w0_on = w0_on || k == 4;
           }
         }
       }
@@ -764,7 +778,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
   // ---------------------------------------------------------------- teardown
   __syncthreads();
   const bool failed = *((volatile uint32_t*)flag) != 0;
-  if (warp == kBwdIssuer && lane == 0) {
+  if (warp == kBwdIssuer && tc::elect_one()) {
     // every MMA this thread issued completes before TMEM is released; copies
     // still in flight (a wait gave up) land before shared memory is released
     if (!hold) {
@@ -772,8 +786,10 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
       tc::mbar_wait(dbar, 0, spin_max);
     }
     if (!wdone) tc::mbar_wait(wbar, 0, spin_max);
-    for (int b = 0; b < kBwdXBufs; ++b)  // at most one copy per buffer is outstanding
-      if (xissued[b] > xwaits[b]) tc::mbar_wait(xbar + b, xwaits[b] & 1u, spin_max);
+    for (int b = 0; b < kBwdXBufs; ++b) {  // at most one copy per buffer is outstanding
+      const uint32_t waits = uint32_t(xdone + kBwdXBufs - 1 - b) / kBwdXBufs;
+      if (xissued[b] > waits) tc::mbar_wait(xbar + b, waits & 1u, spin_max);
+    }
   }
   __syncthreads();
   // The dW1 and dW0|db0 rows are staged in shared memory (the slots' space,
