@@ -995,7 +995,7 @@ __device__ __forceinline__ void gather_add(const float4 p, const float4* q, bool
 // sum to grad_d and/or the k0 sums to grad_c (C channels). NQ = the number of
 // float4 chunks of the k0 gradient in a grouped record (0 = density only).
 template <int NQ>
-__global__ void __launch_bounds__(256, 4)
+__global__ void __launch_bounds__(kVoxelThreads, 1024 / kVoxelThreads)
     k_voxel_gather(GridView g, const int32_t* __restrict__ list, const uint32_t* __restrict__ count,
                    const uint32_t* __restrict__ cnt, const uint32_t* __restrict__ off,
                    const float4* __restrict__ rec_g, float* grad_d, float* grad_c, int C) {
@@ -1066,6 +1066,16 @@ __global__ void __launch_bounds__(256, 4)
     if (want_d) grad_d[slot] = __fadd_rn(grad_d[slot], sum_d);
     if (want_c) {
       float* dst = grad_c + slot * C;
+      if (NQ == 3 && C == 12) {
+        float4* d4 = reinterpret_cast<float4*>(dst);
+#pragma unroll
+        for (int b = 0; b < NQ; ++b) {
+          const float4 v = d4[b];
+          d4[b] = make_float4(__fadd_rn(v.x, acc[b].x), __fadd_rn(v.y, acc[b].y),
+                              __fadd_rn(v.z, acc[b].z), __fadd_rn(v.w, acc[b].w));
+        }
+        continue;
+      }
 #pragma unroll
       for (int b = 0; b < NQ; ++b) {
         const float a4[4] = {acc[b].x, acc[b].y, acc[b].z, acc[b].w};
@@ -1099,12 +1109,12 @@ static int cell_reduce_launch(pvdb_march_s* m, pvdb_grid_s* density, pvdb_grid_s
     PVDB_CHECK_LAUNCH("k_group_records");
   }
   const float4* rec_g = m->b_rec_s;
-  launch_k(k_voxel_gather<NQ>, grid, 256, 0, st, gv, density->d_tlist, density->d_tcount,
+  launch_k(k_voxel_gather<NQ>, voxel_grid(density), kVoxelThreads, 0, st, gv, density->d_tlist, density->d_tcount,
            m->cell_cnt, m->cell_off, rec_g, density->d_grad, same ? k0->d_grad : nullptr, C);
   PVDB_CHECK_LAUNCH("k_voxel_gather");
   if (NQ && !same) {
     if ((rc = touched_list(k0, st))) return rc;
-    launch_k(k_voxel_gather<NQ>, grid, 256, 0, st, kv, k0->d_tlist, k0->d_tcount, m->cell_cnt,
+    launch_k(k_voxel_gather<NQ>, voxel_grid(k0), kVoxelThreads, 0, st, kv, k0->d_tlist, k0->d_tcount, m->cell_cnt,
              m->cell_off, rec_g, nullptr, k0->d_grad, C);
     PVDB_CHECK_LAUNCH("k_voxel_gather(k0)");
   }

@@ -445,6 +445,17 @@ int touched_list(pvdb_grid_s* g, cudaStream_t st);
 // Fixed grid for grid-stride kernels whose work size lives on the device.
 inline int stride_grid() { return num_sms() * 8; }
 
+// Kernels with a thread per voxel of the touched leaves whose work differs much
+// from voxel to voxel: small blocks, one for every 128 voxels of the grid's
+// leaves, so that an SM takes the next voxels when some are done (against a grid
+// of 8 blocks of 256 threads an SM that walk the voxels, gradient rows in 4-byte
+// accesses: 320^3 step 4332 -> 4280 us, 160^3 247.5 -> 241.6 us, 149 k colour
+// points 196 -> 175 us); blocks beyond the touched leaves return at once.
+constexpr int kVoxelThreads = 128;
+inline int voxel_grid(const pvdb_grid_s* g) {
+  return int(std::min<int64_t>(std::max<int64_t>(g->nslots() / kVoxelThreads, 1), 1 << 20));
+}
+
 // Programmatic dependent launch. Kernels launched by launch_k on a stream
 // that is not being captured may be scheduled while the kernel before them
 // in the stream is still running, so that a dependent kernel's launch

@@ -824,7 +824,7 @@ struct RecLoad {
 // Thread per voxel of the touched leaves; neighbouring threads read
 // neighbouring table entries and records.
 template <bool SCALAR, bool VEC>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kVoxelThreads, SCALAR ? 7 : VEC ? 6 : 4)
     k_point_gather(GridView g, CellLattice L, const int32_t* __restrict__ list,
                    const uint32_t* __restrict__ count, const uint32_t* __restrict__ svals,
                    const uint2* __restrict__ cells, const float4* __restrict__ rec, PointSrc src,
@@ -1034,7 +1034,7 @@ static int point_backward_cells(pvdb_grid_s* g, const CellLattice& L, int64_t nc
   launch_k(g->C == 1 ? k_point_gather<true, false>
            : src.vec ? k_point_gather<false, true>
                      : k_point_gather<false, false>,
-           stride_grid(), 256, 0, st, g->view(), L, g->d_tlist, g->d_tcount, svals, rs.cells,
+           voxel_grid(g), kVoxelThreads, 0, st, g->view(), L, g->d_tlist, g->d_tcount, svals, rs.cells,
            rs.rec, src, *status);
   PVDB_CHECK_LAUNCH("k_point_gather");
   launch_k(k_point_clear, sgrid, 256, 0, st, skeys, n, n_dev, rs.cells, *status);
