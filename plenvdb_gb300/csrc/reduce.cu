@@ -544,11 +544,10 @@ struct PointTerm {
   float g[12];
 };
 
-template <bool SCALAR, class Ids, class Load>
+template <bool SCALAR, int BATCH, class Ids, class Load>
 __device__ __forceinline__ void merge_lists(const Ids& ids, const Load& load,
                                             const uint32_t first[8], const uint32_t end[8],
                                             float acc[12], bool& any) {
-  constexpr int kMergeBatch = SCALAR ? 4 : 2;
   uint32_t head[8], pos[8];
 #pragma unroll
   for (int c = 0; c < 8; ++c) {
@@ -559,10 +558,10 @@ __device__ __forceinline__ void merge_lists(const Ids& ids, const Load& load,
   for (int q = 0; q < 12; ++q) acc[q] = 0.f;
   any = false;
   for (;;) {
-    uint32_t s[kMergeBatch], at[kMergeBatch];
-    int corner[kMergeBatch];
+    uint32_t s[BATCH], at[BATCH];
+    int corner[BATCH];
 #pragma unroll
-    for (int b = 0; b < kMergeBatch; ++b) {
+    for (int b = 0; b < BATCH; ++b) {
       s[b] = head[0];
 #pragma unroll
       for (int c = 1; c < 8; ++c) s[b] = min(s[b], head[c]);
@@ -580,12 +579,12 @@ __device__ __forceinline__ void merge_lists(const Ids& ids, const Load& load,
       }
     }
     if (s[0] == kInvalidKey) return;
-    PointTerm t[kMergeBatch];
+    PointTerm t[BATCH];
 #pragma unroll
-    for (int b = 0; b < kMergeBatch; ++b)
+    for (int b = 0; b < BATCH; ++b)
       if (s[b] != kInvalidKey) load(s[b], at[b], t[b]);
 #pragma unroll
-    for (int b = 0; b < kMergeBatch; ++b) {
+    for (int b = 0; b < BATCH; ++b) {
       if (s[b] == kInvalidKey) break;
       if (SCALAR) {
         if (t[b].g[0] == 0.f) continue;
@@ -607,20 +606,21 @@ __device__ __forceinline__ void merge_lists(const Ids& ids, const Load& load,
 // ((g*a)*b)*c per point with a nonzero gradient; features g*scale, channels in
 // chunks of 12, the lists walked again per chunk. make_load(ch0, nch): the
 // loader of that chunk.
-template <bool SCALAR, class Ids, class MakeLoad>
+// BATCH points are loaded together.
+template <bool SCALAR, int BATCH, class Ids, class MakeLoad>
 __device__ __forceinline__ void merge_voxel(int C, const Ids& ids, const MakeLoad& make_load,
                                             const uint32_t first[8], const uint32_t end[8],
                                             int64_t slot, float* grad, uint8_t* touched) {
   float acc[12];
   bool any;
   if (SCALAR) {
-    merge_lists<true>(ids, make_load(0, 1), first, end, acc, any);
+    merge_lists<true, BATCH>(ids, make_load(0, 1), first, end, acc, any);
     if (!any) return;
     grad[slot] = __fadd_rn(grad[slot], acc[0]);
   } else {
     for (int ch0 = 0; ch0 < C; ch0 += 12) {
       const int nch = min(12, C - ch0);
-      merge_lists<false>(ids, make_load(ch0, nch), first, end, acc, any);
+      merge_lists<false, BATCH>(ids, make_load(ch0, nch), first, end, acc, any);
       if (!any) return;
       float* dst = grad + slot * C + ch0;
 #pragma unroll
@@ -849,7 +849,7 @@ __global__ void __launch_bounds__(kVoxelThreads, SCALAR ? 7 : VEC ? 6 : 4)
       some |= e.y;
     }
     if (!some) continue;
-    merge_voxel<SCALAR>(
+    merge_voxel<SCALAR, SCALAR ? 4 : 2>(
         src.C, [&](uint32_t pos) { return __ldg(svals + pos); },
         [&](int ch0, int nch) { return RecLoad<VEC>{rec, src, ch0, nch}; }, first, end,
         int64_t(leaf) * kLeafVox + vox, g.grad, nullptr);
@@ -859,9 +859,13 @@ __global__ void __launch_bounds__(kVoxelThreads, SCALAR ? 7 : VEC ? 6 : 4)
 // Up to kSmallPoints points: one block sorts (cell, point) words in shared
 // memory, and a second kernel, eight threads per sorted point, takes a voxel at
 // the first point of its first cell and finds its cells by binary search; two
-// launches in place of the sort's seven and no table.
+// launches in place of the sort's seven and no table. The eight searches run
+// side by side and four points are loaded at a time: a thread is alone with its
+// latencies (203 rays' colour points 67 -> 59 us a call).
 constexpr int kSmallPoints = 2048;
 constexpr int kSmallBits = 11;
+// points a thread loads together: the few threads leave the registers free
+constexpr int kSmallBatch = 4;
 constexpr uint64_t kNoPoint = ~0ull;
 // 14 bits per coordinate (resolutions are at most 8192)
 __device__ __forceinline__ uint64_t small_cell(const CellLattice& L, int i, int j, int k) {
@@ -908,8 +912,13 @@ __global__ void __launch_bounds__(128)
     k_point_small_gather(GridView g, CellLattice L, const uint64_t* __restrict__ sorted, int n,
                          PointSrc src, uint8_t* touched) {
   grid_dep_sync();
-  __shared__ uint64_t w[kSmallPoints];
-  for (int p = threadIdx.x; p < n; p += 128) w[p] = sorted[p];
+  __shared__ __align__(16) uint64_t w[kSmallPoints];
+  const ulonglong2* s2 = reinterpret_cast<const ulonglong2*>(sorted);
+#pragma unroll
+  for (int b = 0; b < kSmallPoints / 256; ++b) {  // (the words behind n are not used)
+    const int p = b * 128 + threadIdx.x;
+    if (2 * p < n) reinterpret_cast<ulonglong2*>(w)[p] = __ldg(s2 + p);
+  }
   __syncthreads();
   const int t = blockIdx.x * 128 + threadIdx.x, i = t >> 3, c = t & 7;
   if (i >= n) return;
@@ -921,33 +930,41 @@ __global__ void __launch_bounds__(128)
             vk = int(cell & 0x3FFFu) - 1 + dk;
   const int slot = slot_of(g, vi, vj, vk);
   if (slot < 0) return;
+  // the eight cells' lists: their binary searches, then the walks to their ends,
+  // side by side
+  uint64_t want[8];
   uint32_t first[8], end[8];
-  bool owner = true;
 #pragma unroll
   for (int q = 0; q < 8; ++q) {
     int ei, ej, ek;
     corner_delta(q, ei, ej, ek);
-    const uint64_t want = small_cell(L, vi - ei, vj - ej, vk - ek);
-    int lo = 0, hi = n;
-    if (q == c) {
-      lo = i;
-    } else {
-      while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if ((w[mid] >> kSmallBits) < want)
-          lo = mid + 1;
-        else
-          hi = mid;
-      }
-    }
-    first[q] = uint32_t(lo);
-    hi = lo;
-    while (hi < n && (w[hi] >> kSmallBits) == want) ++hi;
-    end[q] = uint32_t(hi);
-    owner = owner && (q >= c || hi == lo);
+    want[q] = small_cell(L, vi - ei, vj - ej, vk - ek);
+    first[q] = 0;
   }
+#pragma unroll 1
+  for (int step = kSmallPoints; step > 0; step >>= 1) {
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const uint32_t at = first[q] + step;
+      if (at <= uint32_t(n) && (w[at - 1] >> kSmallBits) < want[q]) first[q] = at;
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < 8; ++q) end[q] = first[q];
+  for (bool more = true; more;) {
+    more = false;
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      if (end[q] < uint32_t(n) && (w[end[q]] >> kSmallBits) == want[q]) {
+        ++end[q];
+        more = true;
+      }
+  }
+  bool owner = true;  // (another thread takes the voxel at its first cell with points)
+#pragma unroll
+  for (int q = 0; q < 8; ++q) owner = owner && (q >= c || end[q] == first[q]);
   if (!owner) return;
-  merge_voxel<SCALAR>(
+  merge_voxel<SCALAR, kSmallBatch>(
       src.C, [&](uint32_t pos) { return uint32_t(w[pos]) & (kSmallPoints - 1); },
       [&](int ch0, int nch) { return ArrayLoad{src, ch0, nch}; }, first, end, slot, g.grad,
       touched);
