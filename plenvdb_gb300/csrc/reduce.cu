@@ -971,7 +971,8 @@ __global__ void __launch_bounds__(128)
 }
 
 // Largest cell table the point backward keeps per grid (1 GiB, about 500^3
-// voxels); grids beyond it sort the (slot, corner) pairs.
+// voxels); grids beyond it, or with no memory left for it, sort the (slot,
+// corner) pairs.
 constexpr int64_t kMaxCells = int64_t(1) << 27;
 
 static int point_backward_pairs(pvdb_grid_s* g, const PointSrc& src, int64_t n, cudaStream_t st,
@@ -1008,16 +1009,22 @@ static int point_backward_small(pvdb_grid_s* g, const CellLattice& L, const Poin
   return PVDB_OK;
 }
 
+// The cell table, zeroed when it is new.
+static int cell_table(pvdb_grid_s* g, int64_t ncells, cudaStream_t st) {
+  ReduceScratch& rs = g->red;
+  if (rs.cells_cap >= size_t(ncells) * 8) return PVDB_OK;
+  int rc = dev_reserve((void**)&rs.cells, &rs.cells_cap, size_t(ncells) * 8);
+  if (rc) return rc;
+  PVDB_CHECK_CUDA(cudaMemsetAsync(rs.cells, 0, rs.cells_cap, st));
+  return PVDB_OK;
+}
+
 static int point_backward_cells(pvdb_grid_s* g, const CellLattice& L, int64_t ncells,
                                 const PointSrc& src, int64_t n, cudaStream_t st,
                                 uint32_t** status) {
   ReduceScratch& rs = g->red;
   int rc = reduce_reserve(g, n);
   if (rc) return rc;
-  if (rs.cells_cap < size_t(ncells) * 8) {
-    if ((rc = dev_reserve((void**)&rs.cells, &rs.cells_cap, size_t(ncells) * 8))) return rc;
-    PVDB_CHECK_CUDA(cudaMemsetAsync(rs.cells, 0, rs.cells_cap, st));
-  }
   if ((rc = dev_reserve((void**)&rs.rec, &rs.rec_cap, size_t(n) * (src.vec ? 64 : 16)))) return rc;
   if (!rs.npts && (rc = dev_alloc((void**)&rs.npts, 16))) return rc;
   const int bits = slot_key_bits(ncells);
@@ -1096,12 +1103,18 @@ extern "C" int pvdb_grid_sample_backward(pvdb_grid g, const float* xs, const flo
   const int64_t ncells = int64_t(L.ext[0]) * L.ext[1] * L.ext[2] * kLeafVox;
   uint32_t* status = nullptr;
   int rc = PVDB_OK;
-  if (n <= kSmallPoints)
+  if (n <= kSmallPoints) {
     rc = point_backward_small(g, L, src, int(n), st);
-  else if (ncells <= kMaxCells)
-    rc = point_backward_cells(g, L, ncells, src, n, st, &status);
-  else
-    rc = point_backward_pairs(g, src, n, st, &status);
+  } else {
+    rc = ncells <= kMaxCells ? cell_table(g, ncells, st) : int(PVDB_ERR_NOMEM);
+    if (rc == PVDB_OK) {
+      rc = point_backward_cells(g, L, ncells, src, n, st, &status);
+    } else if (rc == PVDB_ERR_NOMEM) {
+      cudaGetLastError();  // a failed allocation is answered here
+      clear_error();
+      rc = point_backward_pairs(g, src, n, st, &status);
+    }
+  }
   if (rc) return rc;
   g->tlist_valid = false;  // new touched leaves
   // the call waits for its stream (as the reference's backward does) so that a

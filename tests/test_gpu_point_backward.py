@@ -61,6 +61,31 @@ def test_matches_the_pair_sort(lib, channels, kind, n):
         assert not np.any(left[act > 0])
 
 
+@pytest.mark.parametrize("channels", [1, 12])
+def test_without_memory_for_the_cell_table(lib, channels):
+    import torch
+    from plenvdb_gb300 import ColorVDB, DensityVDB
+    from plenvdb_gb300 import _lib as L
+    rng = np.random.default_rng(channels)
+    reso, n = [24, 17, 33], 3000
+    act = (rng.random(reso) < 0.05).astype(np.uint8)
+    cls = DensityVDB if channels == 1 else ColorVDB
+    a, b = (cls.from_mask(reso, act, background=-1.0, n=channels) for _ in range(2))
+    xyz = torch.from_numpy(_points("spread", n, reso, rng).astype(np.float32)).cuda()
+    xs, ys, zs = (xyz[:, q].contiguous() for q in range(3))
+    g = torch.from_numpy(rng.normal(0, 1, n * channels).astype(np.float32)).cuda()
+    for it in range(2):  # the second call gets its table
+        if it == 0:
+            L.load().pvdb_debug_fail_next_allocs(1)
+        try:
+            a.backward(xs, ys, zs, g)
+        finally:
+            L.load().pvdb_debug_fail_next_allocs(0)
+        b.backward(xs, ys, zs, g)
+        ga, gb = (v.get_dense_grid(which=L.WHICH_GRAD).view(np.uint32) for v in (a, b))
+        np.testing.assert_array_equal(ga, gb)
+
+
 @pytest.mark.parametrize("n", [1, 255, 257])
 def test_color_forward_12_matches_general(lib, n):
     import torch
