@@ -635,7 +635,7 @@ NCU_TRAFFIC = {
     "rgbnet_bwd": 18.388e6,            # k_mlp_bwd_tc
     "march_bwd": 7.145e6,              # k_march_bwd
     "voxel_gather": 11.030e6 + 26.148e6,  # k_group_records + k_voxel_gather
-    "tv": 12.608e6,                    # k_tv_terms_c12 (the density grid's k_tv_terms not captured)
+    "tv": 12.608e6,                    # k_tv_c12<true> (the density grid's k_tv<true> not captured)
     "voxel_adam": 52.651e6 + 3.142e6 + 6.055e6,  # k_vdb_adam_c12 + k_vdb_adam1
 }
 
