@@ -129,6 +129,13 @@ __device__ __forceinline__ void load_w0k(float* w0k, const MlpArgs& a, int t, in
 // each takes its own tiles (named barriers), so one group's loads and layer 0
 // run under the other's FMAs. Layer 1 per thread: 8 rows x 8 columns (128-row
 // tiles), 4 x 4 (32-row tiles), each sum in k order.
+// A row's logits are the same bits in either kind of tile (the renderer's rows
+// lie anywhere): of each 64 columns the chain over columns 4 x .. 4 x + 3 and
+// 32 + 4 x .. 32 + 4 x + 3 for x = 0..7, the chains' sum as a tree over bits 2, 1,
+// 0 of x, then the two 64-column sums. In a 128-row tile a thread has the whole
+// chain; in a 32-row tile lane x has its first half and lane x + 8 goes on from
+// there. (Two chains of four instead, added in the thread, cost a 397x301 FP32
+// frame 2237 -> 2304 us.)
 constexpr int kFwdGroup = 256;
 constexpr int kFwdThreads = 2 * kFwdGroup;
 
@@ -157,11 +164,13 @@ __device__ __forceinline__ void fwd_tile(FwdSmem<CQ>& S, FwdGroupSmem<CQ>& G, in
                                          float* out, const float* rw) {
   constexpr int TR = RT == 2 ? 128 : 32;
   constexpr int ld = TR + 4;
-  constexpr int kColWarps = RT == 2 ? 2 : 4;
-  const int lane = t & 31, warp = t >> 5, tx = lane & 7, ty = lane >> 3;
-  const int rb = (warp / kColWarps) * (16 * RT) + 4 * ty;  // rows rb + 16 i + e
+  constexpr int kColWarps = 2;                // 64 columns each
+  constexpr int kColLanes = RT == 2 ? 8 : 16;
+  const int lane = t & 31, warp = t >> 5, tx = lane % kColLanes, ty = lane / kColLanes;
   const int cw = warp % kColWarps;
-  const int cb = cw * (32 * CT) + 4 * tx;  // columns cb + 32 j + e
+  // rows rb + 16 i + e, columns cb + 32 j + e
+  const int rb = (warp / kColWarps) * (RT == 2 ? 32 : 8) + 4 * ty;
+  const int cb = cw * 64 + 4 * tx;
   load_rows<TR, CQ>(G.x, G.rays, t, kFwdGroup, a.c0, k0, ray, row0, M);
   bar_group(bar, kFwdGroup);
   layer0<TR, CQ, kFwdGroup>(G.h0, ld, S.w0k, G.x, G.rays, hpe, t);
@@ -190,43 +199,53 @@ __device__ __forceinline__ void fwd_tile(FwdSmem<CQ>& S, FwdGroupSmem<CQ>& G, in
       for (int i = 0; i < 2 * RT; ++i) acc2[i][j] = fma2(av[i], d, acc2[i][j]);
     }
   }
-  // logits: this thread's columns, then the 8 lanes of its rows (a
-  // reduce-scatter: lane tx ends with one row), then the column warps
+  // logits: this thread's columns, then the lanes of its rows (a reduce-scatter),
+  // then the column warps
   float lg[12 * RT];
 #pragma unroll
   for (int i = 0; i < 12 * RT; ++i) lg[i] = 0.f;
+  auto add_columns = [&](float* l) {
 #pragma unroll
-  for (int j = 0; j < 4 * CT; ++j) {
-    const int n = cb + 32 * (j >> 2) + (j & 3);
-    const float b1 = S.b1[n];
-    const float w[3] = {S.w2[n], S.w2[kW + n], S.w2[2 * kW + n]};
+    for (int j = 0; j < 4 * CT; ++j) {
+      const int n = cb + 32 * (j >> 2) + (j & 3);
+      const float b1 = S.b1[n];
+      const float w[3] = {S.w2[n], S.w2[kW + n], S.w2[2 * kW + n]};
 #pragma unroll
-    for (int i = 0; i < 2 * RT; ++i) {
-      float h[2];
-      unpack2(acc2[i][j], h[0], h[1]);
+      for (int i = 0; i < 2 * RT; ++i) {
+        float h[2];
+        unpack2(acc2[i][j], h[0], h[1]);
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        h[e] = fmaxf(h[e] + b1, 0.f);
+        for (int e = 0; e < 2; ++e) {
+          h[e] = fmaxf(h[e] + b1, 0.f);
 #pragma unroll
-        for (int c = 0; c < 3; ++c)
-          lg[3 * (2 * i + e) + c] = fmaf(w[c], h[e], lg[3 * (2 * i + e) + c]);
+          for (int c = 0; c < 3; ++c)
+            l[3 * (2 * i + e) + c] = fmaf(w[c], h[e], l[3 * (2 * i + e) + c]);
+        }
       }
     }
-  }
+  };
+  add_columns(lg);
   float* red = G.x;
   int row = rb;
+  bool mine = true;
   if (RT == 2) {
     scatter_step<24>(lg, 4, tx & 4);
-    row += tx & 4 ? 16 : 0;
-  }
-  scatter_step<12>(lg, 2, tx & 2);
-  scatter_step<6>(lg, 1, tx & 1);
-  row += (tx & 2) + (tx & 1);
-  if (RT == 1) {
+    scatter_step<12>(lg, 2, tx & 2);
+    scatter_step<6>(lg, 1, tx & 1);
+    row += (tx & 4 ? 16 : 0) + (tx & 2) + (tx & 1);
+  } else {
+    // the chain goes on from the lane of the lower half
 #pragma unroll
-    for (int c = 0; c < 3; ++c) lg[c] += __shfl_xor_sync(0xffffffffu, lg[c], 4);
+    for (int i = 0; i < 12; ++i) lg[i] = __shfl_xor_sync(0xffffffffu, lg[i], 8);
+    add_columns(lg);
+    scatter_step<12>(lg, 4, tx & 4);
+    scatter_step<6>(lg, 2, tx & 2);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) lg[c] += __shfl_xor_sync(0xffffffffu, lg[c], 1);
+    row += (tx & 4 ? 2 : 0) + (tx & 2 ? 1 : 0);
+    mine = (tx & 9) == 8;
   }
-  if (RT == 2 || tx < 4) {
+  if (mine) {
 #pragma unroll
     for (int c = 0; c < 3; ++c) red[(cw * TR + row) * 3 + c] = lg[c];
   }
