@@ -124,6 +124,15 @@ __device__ __forceinline__ void load_w0k(float* w0k, const MlpArgs& a, int t, in
   }
 }
 
+// Four floats of W1, which may be a view into a parameter buffer at any offset: in
+// one load (VEC) only where it lies on a 16-byte boundary, which the launch looks
+// at. (A choice in the kernel moved its schedule: 160^3 FP32 step 741 -> 747 us.)
+template <bool VEC>
+__device__ __forceinline__ float4 w1_quad(const float* w1) {
+  if constexpr (VEC) return __ldg(reinterpret_cast<const float4*>(w1));
+  return make_float4(__ldg(w1), __ldg(w1 + 1), __ldg(w1 + 2), __ldg(w1 + 3));
+}
+
 // ----------------------------------------------------------------- forward
 // One CTA of 512 threads per SM: two groups of 256 share the transposed W1 and
 // each takes its own tiles (named barriers), so one group's loads and layer 0
@@ -261,7 +270,7 @@ __device__ __forceinline__ void fwd_tile(FwdSmem<CQ>& S, FwdGroupSmem<CQ>& G, in
   bar_group(bar, kFwdGroup);  // the partials are read: the next tile's rows may land
 }
 
-template <int CQ>
+template <int CQ, bool VEC>
 __global__ void __launch_bounds__(kFwdThreads, 1)
     k_mlp_fwd_f32(MlpArgs a, const float* __restrict__ k0, const int32_t* __restrict__ ray,
                   const float* __restrict__ hpe, const uint32_t* __restrict__ totals, float* out,
@@ -277,7 +286,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
   const int tid = threadIdx.x;
   for (int i = tid; i < kW * kW / 4; i += kFwdThreads) {
     const int n = i % kW, k = 4 * (i / kW);  // lanes along n: conflict-free stores
-    const float4 v = __ldg(reinterpret_cast<const float4*>(a.w1 + n * kW + k));
+    const float4 v = w1_quad<VEC>(a.w1 + n * kW + k);
     S.w1t[k * kW + n] = v.x;
     S.w1t[(k + 1) * kW + n] = v.y;
     S.w1t[(k + 2) * kW + n] = v.z;
@@ -585,7 +594,7 @@ __device__ __forceinline__ void bwd_tile(BwdSmem<CQ>& B, BwdAcc<CQ>& A, const Ml
   __syncthreads();
 }
 
-template <int CQ>
+template <int CQ, bool VEC>
 __global__ void __launch_bounds__(kBwdThreads, 1)
     k_mlp_bwd_f32(MlpArgs a, BwdIn in, const uint32_t* __restrict__ totals, float* wpart) {
   grid_dep_sync();
@@ -618,8 +627,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
   {
     for (int i = tid; i < kW * kW / 4; i += kBwdThreads) {
       const int n = i / (kW / 4), k = 4 * (i % (kW / 4));
-      *reinterpret_cast<float4*>(B.w1 + n * kLd + k) =
-          __ldg(reinterpret_cast<const float4*>(a.w1 + n * kW + k));
+      *reinterpret_cast<float4*>(B.w1 + n * kLd + k) = w1_quad<VEC>(a.w1 + n * kW + k);
     }
     load_w0k<CQ>(B.w0k, a, tid, kBwdThreads);
     for (int i = tid; i < 3 * kW; i += kBwdThreads) B.w2[i] = a.w2[i];
@@ -690,24 +698,28 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
 static_assert(sizeof(FwdSmem<4>) <= 227 * 1024 && sizeof(BwdSmem<4>) <= 227 * 1024,
               "one CTA's shared memory");
 
-template <int CQ>
+template <int CQ, bool VEC>
 int fwd_launch(const MlpArgs& a, const float* k0, const int32_t* ray, const float* hpe,
                const uint32_t* totals, float* out, const float* rw, cudaStream_t st) {
-  PVDB_SMEM_ATTR(k_mlp_fwd_f32<CQ>, int(sizeof(FwdSmem<CQ>)));
-  launch_k(k_mlp_fwd_f32<CQ>, num_sms(), kFwdThreads, sizeof(FwdSmem<CQ>), st, a, k0, ray, hpe,
-           totals, out, rw);
+  const auto kernel = k_mlp_fwd_f32<CQ, VEC>;
+  PVDB_SMEM_ATTR(kernel, int(sizeof(FwdSmem<CQ>)));
+  launch_k(kernel, num_sms(), kFwdThreads, sizeof(FwdSmem<CQ>), st, a, k0, ray, hpe, totals, out,
+           rw);
   PVDB_CHECK_LAUNCH("k_mlp_fwd_f32");
   return PVDB_OK;
 }
 
-template <int CQ>
+template <int CQ, bool VEC>
 int bwd_launch(const MlpArgs& a, const BwdIn& in, const uint32_t* totals, float* wpart, int grid,
                cudaStream_t st) {
-  PVDB_SMEM_ATTR(k_mlp_bwd_f32<CQ>, int(sizeof(BwdSmem<CQ>)));
-  launch_k(k_mlp_bwd_f32<CQ>, grid, kBwdThreads, sizeof(BwdSmem<CQ>), st, a, in, totals, wpart);
+  const auto kernel = k_mlp_bwd_f32<CQ, VEC>;
+  PVDB_SMEM_ATTR(kernel, int(sizeof(BwdSmem<CQ>)));
+  launch_k(kernel, grid, kBwdThreads, sizeof(BwdSmem<CQ>), st, a, in, totals, wpart);
   PVDB_CHECK_LAUNCH("k_mlp_bwd_f32");
   return PVDB_OK;
 }
+
+bool on_16_bytes(const float* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 }  // namespace
 
@@ -715,8 +727,10 @@ int bwd_launch(const MlpArgs& a, const BwdIn& in, const uint32_t* totals, float*
 // channel count padded to 12 or 16 with zeros.
 int mlp_f32_forward(const MlpArgs& a, const float* k0, const int32_t* ray, const float* hpe,
                     const uint32_t* totals, float* out, const float* rw, cudaStream_t st) {
-  return a.c0 <= 12 ? fwd_launch<3>(a, k0, ray, hpe, totals, out, rw, st)
-                    : fwd_launch<4>(a, k0, ray, hpe, totals, out, rw, st);
+  const bool vec = on_16_bytes(a.w1);
+  const auto launch = a.c0 <= 12 ? (vec ? fwd_launch<3, true> : fwd_launch<3, false>)
+                                 : (vec ? fwd_launch<4, true> : fwd_launch<4, false>);
+  return launch(a, k0, ray, hpe, totals, out, rw, st);
 }
 
 int mlp_f32_backward(const MlpArgs& a, const float* k0, const int32_t* ray, const float* hpe,
@@ -724,8 +738,10 @@ int mlp_f32_backward(const MlpArgs& a, const float* k0, const int32_t* ray, cons
                      const float* grad_rgb, float* grad_k0, float* wpart, int grid,
                      cudaStream_t st) {
   const BwdIn in{k0, ray, hpe, pe, rgb, grad_rgb, grad_k0};
-  return a.c0 <= 12 ? bwd_launch<3>(a, in, totals, wpart, grid, st)
-                    : bwd_launch<4>(a, in, totals, wpart, grid, st);
+  const bool vec = on_16_bytes(a.w1);
+  const auto launch = a.c0 <= 12 ? (vec ? bwd_launch<3, true> : bwd_launch<3, false>)
+                                 : (vec ? bwd_launch<4, true> : bwd_launch<4, false>);
+  return launch(a, in, totals, wpart, grid, st);
 }
 
 }  // namespace pvdb
