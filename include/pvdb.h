@@ -525,7 +525,10 @@ int pvdb_renderer_set_kwargs(pvdb_renderer r, float near_, float far_, float ste
 int pvdb_renderer_input_c2w(pvdb_renderer r, const float* c2w, int32_t mem, pvdb_stream s);
 /* render_an_image (plenvdb.h:1027-1037) into the renderer's device image. */
 int pvdb_renderer_render(pvdb_renderer r, int32_t precision, pvdb_stream s);
-/* output_an_image (plenvdb.h:1038-1046): [H*W*3]. */
+/* output_an_image (plenvdb.h:1038-1046): [H*W*3]. A frame in which a bounded wait
+ * of the BF16 rgbnet gave up is reported as PVDB_ERR_TIMEOUT by the host form, or,
+ * when it was taken to device memory (no wait for the stream), by the next
+ * pvdb_renderer_render, which then renders nothing; it is reported once. */
 int pvdb_renderer_output(pvdb_renderer r, float* out, int32_t mem, pvdb_stream s);
 /* Device pointer of the image [H*W*3] and the sample count of the last frame
  * (device scalar). */

@@ -92,7 +92,7 @@ struct RenderBatch {
 struct RenderW {
   uint32_t* n;       // [HW] colour samples per pixel
   float* T;          // [HW]
-  uint32_t* totals;  // [1] rows, [2] batches
+  uint32_t* totals;  // [1] rows, [2] batches, [3] the rgbnet's given-up waits
   int32_t* head;     // [warps] first batch of each warp, -1: none
   RenderBatch* batch;  // [bcap]
   int64_t bcap;
@@ -723,6 +723,14 @@ static int renderer_grow_rows(pvdb_renderer_s* r, int64_t need) {
   return PVDB_OK;
 }
 
+// The status word of the rgbnet's bounded waits was set: some rows of that frame
+// were not written. Cleared once it is reported.
+static int wait_gave_up(pvdb_renderer_s* r, cudaStream_t st) {
+  PVDB_CHECK_CUDA(cudaMemsetAsync(r->d_totals + 3, 0, 4, st));
+  return set_error(PVDB_ERR_TIMEOUT,
+                   "a tensor-core MMA wait timed out: the last rendered image is incomplete");
+}
+
 extern "C" {
 
 int pvdb_renderer_create(int32_t dcol, int32_t dpe, int32_t dhid, int32_t dout,
@@ -742,6 +750,10 @@ int pvdb_renderer_create(int32_t dcol, int32_t dpe, int32_t dhid, int32_t dout,
   const size_t P = size_t(dhid) * (dcol + dpe) + dhid + size_t(dhid) * dhid + dhid + 3 * dhid + 3;
   int rc = dev_alloc((void**)&r->d_params, P * 4);
   if (!rc) rc = dev_alloc((void**)&r->d_totals, 64);
+  if (!rc) {
+    const cudaError_t e = cudaMemset(r->d_totals, 0, 64);
+    if (e != cudaSuccess) rc = cuda_error(e, "renderer create");
+  }
   if (rc) {
     pvdb_renderer_destroy(r);
     return rc;
@@ -999,12 +1011,14 @@ int pvdb_renderer_render(pvdb_renderer r, int32_t precision, pvdb_stream s) {
     Wk.cap = r->rows_cap;
     Wk.batch = r->d_batch;
     Wk.bcap = r->batch_cap;
-    PVDB_CHECK_CUDA(cudaMemsetAsync(r->d_totals, 0, 16, st));
+    PVDB_CHECK_CUDA(cudaMemsetAsync(r->d_totals, 0, 12, st));
     k_render_march<<<ceil_div(tiles, kTileWarps), 32 * kTileWarps, 0, st>>>(P, Wk);
     PVDB_CHECK_LAUNCH("k_render_march");
-    uint32_t tot[2] = {0, 0};
-    PVDB_CHECK_CUDA(cudaMemcpyAsync(tot, r->d_totals + 1, 8, cudaMemcpyDeviceToHost, st));
+    uint32_t tot[3] = {0, 0, 0};
+    PVDB_CHECK_CUDA(cudaMemcpyAsync(tot, r->d_totals + 1, 12, cudaMemcpyDeviceToHost, st));
     PVDB_CHECK_CUDA(cudaStreamSynchronize(st));
+    // (this frame's rgbnet has not run: the word is an earlier frame's)
+    if (tot[2]) return wait_gave_up(r, st);
     total = tot[0];
     if (int64_t(tot[0]) <= r->rows_cap && int64_t(tot[1]) <= r->batch_cap) break;
     // the counts do not depend on the buffers: one more march holds them
@@ -1082,7 +1096,12 @@ int pvdb_renderer_output(pvdb_renderer r, float* out, int32_t mem, pvdb_stream s
                                   mem == PVDB_MEM_DEVICE ? cudaMemcpyDeviceToDevice
                                                          : cudaMemcpyDeviceToHost,
                                   st));
-  if (mem == PVDB_MEM_HOST) PVDB_CHECK_CUDA(cudaStreamSynchronize(st));
+  if (mem == PVDB_MEM_HOST) {
+    uint32_t status = 0;
+    PVDB_CHECK_CUDA(cudaMemcpyAsync(&status, r->d_totals + 3, 4, cudaMemcpyDeviceToHost, st));
+    PVDB_CHECK_CUDA(cudaStreamSynchronize(st));
+    if (status) return wait_gave_up(r, st);
+  }
   return PVDB_OK;
 }
 
