@@ -57,6 +57,8 @@ int pvdb_last_error(char* buf, size_t len);
 /* Test hook: makes the next `count` device allocations made by the library fail
  * with PVDB_ERR_NOMEM (host-side injection; no device call is made for them). */
 int pvdb_debug_fail_next_allocs(int count);
+/* The same after `skip` allocations that succeed. */
+int pvdb_debug_fail_allocs_after(int skip, int count);
 /* Test hook of the bounded device-side waits (no counterpart in the
  * reference): spins > 0 replaces the built-in spin limit of the device waits
  * (radix sort and march look-backs, tensor-core MMA waits, leaf-staging copy

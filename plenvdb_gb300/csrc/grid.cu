@@ -21,6 +21,7 @@ thread_local int g_err_code = PVDB_OK;
 thread_local std::string g_err_msg;
 std::mutex g_fail_mu;
 int g_fail_allocs = 0;
+int g_fail_skip = 0;  // allocations that succeed before those that fail
 }  // namespace
 
 int set_error(int code, const std::string& msg) {
@@ -40,7 +41,7 @@ void clear_error() {
 int dev_alloc(void** p, size_t bytes) {
   {
     std::lock_guard<std::mutex> lk(g_fail_mu);
-    if (g_fail_allocs > 0) {
+    if (g_fail_allocs > 0 && g_fail_skip-- <= 0) {
       --g_fail_allocs;
       *p = nullptr;
       return set_error(PVDB_ERR_NOMEM, "device allocation failed (injected)");
@@ -661,11 +662,14 @@ int pvdb_last_error(char* buf, size_t len) {
   return g_err_code;
 }
 
-int pvdb_debug_fail_next_allocs(int count) {
+int pvdb_debug_fail_allocs_after(int skip, int count) {
   std::lock_guard<std::mutex> lk(g_fail_mu);
+  g_fail_skip = std::max(0, skip);
   g_fail_allocs = std::max(0, count);
   return PVDB_OK;
 }
+
+int pvdb_debug_fail_next_allocs(int count) { return pvdb_debug_fail_allocs_after(0, count); }
 
 int pvdb_grid_create(const int32_t reso[3], int32_t channels, float background, pvdb_grid* out) {
   clear_error();

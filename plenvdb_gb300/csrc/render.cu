@@ -926,6 +926,8 @@ int pvdb_renderer_set_kwargs(pvdb_renderer r, float near_, float far_, float ste
     r->d_n = nullptr;
     r->d_head = nullptr;
     r->d_T = r->d_viewdirs = r->d_hpe = r->d_image = nullptr;
+    r->flags[3] = false;  // no frame, and no size that a later call could keep,
+    r->H = r->W = 0;      // until all of them are there again
     int rc;
     if ((rc = dev_alloc((void**)&r->d_n, HW * 4)) || (rc = dev_alloc((void**)&r->d_head,
                         size_t(ceil_div(w, kTileW)) * ceil_div(h, kTileH) * 4)) ||
