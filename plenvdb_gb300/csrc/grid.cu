@@ -51,6 +51,7 @@ int dev_alloc(void** p, size_t bytes) {
   cudaError_t e = cudaMalloc(p, bytes);
   if (e != cudaSuccess) {
     *p = nullptr;
+    cudaGetLastError();  // reported here: the next launch check does not find it
     return cuda_error(e, "cudaMalloc");
   }
   return PVDB_OK;

@@ -666,16 +666,6 @@ __device__ __forceinline__ uint32_t lattice_key(const CellLattice& L, int i, int
   return (((x >> 3) * L.ext[1] + (y >> 3)) * L.ext[2] + (z >> 3)) << 9 |
          unsigned(vox_offset(x, y, z));
 }
-__device__ __forceinline__ void lattice_cell(const CellLattice& L, uint32_t key, int& i, int& j,
-                                             int& k) {
-  const uint32_t leaf = key >> 9, v = key & 511u;
-  const uint32_t lz = leaf % L.ext[2], ly = (leaf / L.ext[2]) % L.ext[1],
-                 lx = leaf / (L.ext[2] * L.ext[1]);
-  i = int(lx * 8 + (v >> 6)) - 8;
-  j = int(ly * 8 + ((v >> 3) & 7)) - 8;
-  k = int(lz * 8 + (v & 7)) - 8;
-}
-
 __global__ void k_point_cells(CellLattice L, PointSrc src, int64_t n, uint32_t* keys) {
   grid_dep_sync();
   const int64_t p = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
@@ -1009,22 +999,35 @@ static int point_backward_small(pvdb_grid_s* g, const CellLattice& L, const Poin
   return PVDB_OK;
 }
 
+// What the cell form keeps with the grid beyond the sort's scratch: given back when
+// memory for the rest is missing, or when a call ends between the kernels that
+// fill and clear the table.
+static void free_cells(ReduceScratch& rs) {
+  dev_free(rs.cells);
+  dev_free(rs.rec);
+  rs.cells = nullptr;
+  rs.rec = nullptr;
+  rs.cells_cap = rs.rec_cap = 0;
+}
+
 // The cell table, zeroed when it is new.
 static int cell_table(pvdb_grid_s* g, int64_t ncells, cudaStream_t st) {
   ReduceScratch& rs = g->red;
   if (rs.cells_cap >= size_t(ncells) * 8) return PVDB_OK;
   int rc = dev_reserve((void**)&rs.cells, &rs.cells_cap, size_t(ncells) * 8);
   if (rc) return rc;
-  PVDB_CHECK_CUDA(cudaMemsetAsync(rs.cells, 0, rs.cells_cap, st));
-  return PVDB_OK;
+  const cudaError_t e = cudaMemsetAsync(rs.cells, 0, rs.cells_cap, st);
+  if (e == cudaSuccess) return PVDB_OK;
+  free_cells(rs);
+  return cuda_error(e, "cell table");
 }
 
 static int point_backward_cells(pvdb_grid_s* g, const CellLattice& L, int64_t ncells,
                                 const PointSrc& src, int64_t n, cudaStream_t st,
                                 uint32_t** status) {
   ReduceScratch& rs = g->red;
-  int rc = reduce_reserve(g, n);
-  if (rc) return rc;
+  int rc = cell_table(g, ncells, st);
+  if (rc || (rc = reduce_reserve(g, n))) return rc;
   if ((rc = dev_reserve((void**)&rs.rec, &rs.rec_cap, size_t(n) * (src.vec ? 64 : 16)))) return rc;
   if (!rs.npts && (rc = dev_alloc((void**)&rs.npts, 16))) return rc;
   const int bits = slot_key_bits(ncells);
@@ -1050,6 +1053,12 @@ static int point_backward_cells(pvdb_grid_s* g, const CellLattice& L, int64_t nc
   if (rc) return rc;
   const uint32_t *skeys = rs.keys[buf], *svals = rs.vals[buf];
   const int sgrid = int(std::min<int64_t>(ceil_div(n, 256), stride_grid()));
+  struct Filled {  // the table, until k_point_clear is launched
+    ReduceScratch* rs;
+    ~Filled() {
+      if (rs) free_cells(*rs);
+    }
+  } filled{&rs};
   launch_k(src.vec ? k_point_group<true> : k_point_group<false>, sgrid, 256, 0, st, g->view(), L,
            src, skeys, svals, n, n_dev, rs.cells, rs.rec, g->d_touched, *status);
   PVDB_CHECK_LAUNCH("k_point_group");
@@ -1063,6 +1072,7 @@ static int point_backward_cells(pvdb_grid_s* g, const CellLattice& L, int64_t nc
   PVDB_CHECK_LAUNCH("k_point_gather");
   launch_k(k_point_clear, sgrid, 256, 0, st, skeys, n, n_dev, rs.cells, *status);
   PVDB_CHECK_LAUNCH("k_point_clear");
+  filled.rs = nullptr;
   return PVDB_OK;
 }
 
@@ -1106,12 +1116,11 @@ extern "C" int pvdb_grid_sample_backward(pvdb_grid g, const float* xs, const flo
   if (n <= kSmallPoints) {
     rc = point_backward_small(g, L, src, int(n), st);
   } else {
-    rc = ncells <= kMaxCells ? cell_table(g, ncells, st) : int(PVDB_ERR_NOMEM);
-    if (rc == PVDB_OK) {
-      rc = point_backward_cells(g, L, ncells, src, n, st, &status);
-    } else if (rc == PVDB_ERR_NOMEM) {
-      cudaGetLastError();  // a failed allocation is answered here
+    rc = ncells <= kMaxCells ? point_backward_cells(g, L, ncells, src, n, st, &status)
+                             : int(PVDB_ERR_NOMEM);
+    if (rc == PVDB_ERR_NOMEM) {  // (nothing is added yet: all memory is reserved before)
       clear_error();
+      free_cells(g->red);
       rc = point_backward_pairs(g, src, n, st, &status);
     }
   }
