@@ -112,6 +112,9 @@ struct ReduceScratch {
   float4* rec = nullptr;
   size_t rec_cap = 0;
   uint32_t* npts = nullptr;
+  // per leaf the point backward that listed it last, the number of the last one
+  uint32_t* mark = nullptr;
+  uint32_t epoch = 0;
 };
 
 }  // namespace pvdb

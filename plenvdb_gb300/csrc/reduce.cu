@@ -470,10 +470,12 @@ void free_scratch(ReduceScratch& rs) {
   dev_free(rs.cells);
   dev_free(rs.rec);
   dev_free(rs.npts);
-  rs.hist = rs.partial = rs.npts = nullptr;
+  dev_free(rs.mark);
+  rs.hist = rs.partial = rs.npts = rs.mark = nullptr;
   rs.cells = nullptr;
   rs.rec = nullptr;
   rs.cap = rs.hist_cap = rs.partial_cap = rs.cells_cap = rs.rec_cap = 0;
+  rs.epoch = 0;
 }
 
 // ------------------------------------------------- generic point backward
@@ -727,13 +729,15 @@ __global__ void __launch_bounds__(256)
 // Thread per sorted point, set: the point's record (u, v, w and the density
 // gradient; with VEC the 12 feature gradients behind it) in sorted order, its
 // cell's entry of the table from the first and the last point of the cell, and
-// the leaves holding the cell's corners flagged. Not set: clears the entries.
+// the leaves holding the cell's corners flagged and listed, once each (mark: the
+// call that listed a leaf last). The sums walk the leaves of this call, not all
+// that were touched since the gradient was zeroed.
 template <bool VEC>
 __global__ void __launch_bounds__(256)
     k_point_group(GridView g, CellLattice L, PointSrc src, const uint32_t* __restrict__ skeys,
                   const uint32_t* __restrict__ svals, int64_t n_max, const uint32_t* n_dev,
-                  uint2* cells, float4* rec, uint8_t* touched,
-                  const uint32_t* __restrict__ status) {
+                  uint2* cells, float4* rec, uint8_t* touched, uint32_t* mark, uint32_t epoch,
+                  int32_t* list, uint32_t* count, const uint32_t* __restrict__ status) {
   grid_dep_sync();
   if (*status) return;  // the sort gave up a wait: its order is wrong
   const int64_t n = eff_size(n_max, n_dev);
@@ -759,9 +763,16 @@ __global__ void __launch_bounds__(256)
     cells[key].x = uint32_t(i);
     int slots[8];
     corner_slots(g, ci, cj, ck, slots);
+    int before = -1;  // (most cells lie in one leaf)
 #pragma unroll
-    for (int c = 0; c < 8; ++c)
-      if (slots[c] >= 0) touched[slots[c] >> 9] = 1;
+    for (int c = 0; c < 8; ++c) {
+      const int l = slots[c] < 0 ? -1 : slots[c] >> 9;
+      if (l != before && l >= 0 && mark[l] != epoch && atomicExch(mark + l, epoch) != epoch) {
+        touched[l] = 1;
+        list[atomicAdd(count, 1u)] = l;
+      }
+      before = l;
+    }
   }
 }
 
@@ -1030,6 +1041,17 @@ static int point_backward_cells(pvdb_grid_s* g, const CellLattice& L, int64_t nc
   if (rc || (rc = reduce_reserve(g, n))) return rc;
   if ((rc = dev_reserve((void**)&rs.rec, &rs.rec_cap, size_t(n) * (src.vec ? 64 : 16)))) return rc;
   if (!rs.npts && (rc = dev_alloc((void**)&rs.npts, 16))) return rc;
+  if (!rs.mark) {
+    rs.epoch = 0;
+    if ((rc = dev_alloc((void**)&rs.mark, size_t(g->nleaf) * 4))) return rc;
+  }
+  if (rs.epoch + 1 <= 1) {  // new marks, or the last number is given out
+    rs.epoch = 0;
+    PVDB_CHECK_CUDA(cudaMemsetAsync(rs.mark, 0, size_t(g->nleaf) * 4, st));
+  }
+  ++rs.epoch;
+  PVDB_CHECK_CUDA(cudaMemsetAsync(g->d_tcount, 0, 4, st));
+  g->tlist_valid = false;  // d_tlist takes this call's leaves
   const int bits = slot_key_bits(ncells);
   const uint32_t* n_dev = nullptr;
   int buf = 0;
@@ -1060,10 +1082,9 @@ static int point_backward_cells(pvdb_grid_s* g, const CellLattice& L, int64_t nc
     }
   } filled{&rs};
   launch_k(src.vec ? k_point_group<true> : k_point_group<false>, sgrid, 256, 0, st, g->view(), L,
-           src, skeys, svals, n, n_dev, rs.cells, rs.rec, g->d_touched, *status);
+           src, skeys, svals, n, n_dev, rs.cells, rs.rec, g->d_touched, rs.mark, rs.epoch, g->d_tlist,
+           g->d_tcount, *status);
   PVDB_CHECK_LAUNCH("k_point_group");
-  g->tlist_valid = false;
-  if ((rc = touched_list(g, st))) return rc;
   launch_k(g->C == 1 ? k_point_gather<true, false>
            : src.vec ? k_point_gather<false, true>
                      : k_point_gather<false, false>,
