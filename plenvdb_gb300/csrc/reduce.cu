@@ -546,6 +546,12 @@ struct PointTerm {
   float g[12];
 };
 
+__device__ __forceinline__ float corner_scale(const PointTerm& t, int corner) {
+  int di, dj, dk;
+  corner_delta(corner, di, dj, dk);
+  return __fmul_rn(__fmul_rn(di ? t.u : 1.f - t.u, dj ? t.v : 1.f - t.v), dk ? t.w : 1.f - t.w);
+}
+
 template <bool SCALAR, int BATCH, class Ids, class Load>
 __device__ __forceinline__ void merge_lists(const Ids& ids, const Load& load,
                                             const uint32_t first[8], const uint32_t end[8],
@@ -592,10 +598,7 @@ __device__ __forceinline__ void merge_lists(const Ids& ids, const Load& load,
         if (t[b].g[0] == 0.f) continue;
         acc[0] = __fadd_rn(acc[0], density_corner_term(t[b].g[0], t[b].u, t[b].v, t[b].w, corner[b]));
       } else {
-        int di, dj, dk;
-        corner_delta(corner[b], di, dj, dk);
-        const float scale = __fmul_rn(__fmul_rn(di ? t[b].u : 1.f - t[b].u, dj ? t[b].v : 1.f - t[b].v),
-                                      dk ? t[b].w : 1.f - t[b].w);
+        const float scale = corner_scale(t[b], corner[b]);
 #pragma unroll
         for (int q = 0; q < 12; ++q) acc[q] = __fadd_rn(acc[q], __fmul_rn(t[b].g[q], scale));
       }
@@ -633,6 +636,131 @@ __device__ __forceinline__ void merge_voxel(int C, const Ids& ids, const MakeLoa
   if (touched) touched[slot >> 9] = 1;
 }
 
+// A voxel with more points than long_from is summed by a warp (merge_long): its
+// thread would take them one after another, some 0.6 us each, twice what the pair
+// sort's walk takes. A warp takes a voxel's points 12 times as fast but is a warp:
+// where many voxels are long, their threads together are faster, and their one
+// longest voxel does not count. So 32 points up to 64 k points in the call, 128
+// from 256 k. (160^3, 30 k points at 600 voxels: 152 us from 128 up, 101 from 64 or
+// 32, 384 without; 1.8 M points over the scene: 519, 900, 1053, 522 us.)
+__device__ __forceinline__ uint32_t long_from(int64_t n) {
+  return uint32_t(min(max(n >> 11, int64_t(32)), int64_t(128)));
+}
+constexpr uint32_t kLongLeast = 32;
+struct LongVoxel {
+  uint32_t first[8], end[8];
+  uint32_t slot;
+  __device__ __forceinline__ void set(const uint32_t f[8], const uint32_t e[8], int64_t s) {
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      first[c] = f[c];
+      end[c] = e[c];
+    }
+    slot = uint32_t(s);
+  }
+};
+// The most that n points have of them.
+inline int64_t most_long_voxels(int64_t n) { return n * 8 / (kLongLeast + 1); }
+// A warp's space to sum one.
+struct LongWarp {
+  uint32_t ids[8][32];   // the next points of each list
+  uint32_t order[256];   // their merge: position | list << 29
+  float term[12 * 33];   // [channel][point]
+};
+
+// merge_voxel by a warp, the same sums in the same order. A round takes the next
+// 32 points of every list. What lies up to the smallest of the lists' last ids is
+// complete, and ranked by counting the smaller ids of each list; then 32 points
+// at a time are loaded and multiplied by the lanes side by side, and a lane per
+// channel adds them in order.
+template <bool SCALAR, class Ids, class MakeLoad>
+__device__ __forceinline__ void merge_long(LongWarp& S, const LongVoxel& V, int C, const Ids& ids,
+                                           const MakeLoad& make_load, float* grad,
+                                           uint8_t* touched) {
+  const int lane = threadIdx.x & 31;
+  for (int ch0 = 0; ch0 < (SCALAR ? 1 : C); ch0 += 12) {
+    const int nch = SCALAR ? 1 : min(12, C - ch0);
+    const auto load = make_load(ch0, nch);
+    uint32_t pos[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) pos[c] = V.first[c];
+    float acc = 0.f;
+    for (;;) {
+      uint32_t id[8], rank[8], bound = kInvalidKey - 1u, live = 0;
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        const uint32_t left = V.end[c] - pos[c];
+        id[c] = uint32_t(lane) < left ? ids(pos[c] + lane) : kInvalidKey;
+        S.ids[c][lane] = id[c];
+        const uint32_t last = __shfl_sync(0xffffffffu, id[c], 31);
+        if (left > 32) bound = min(bound, last);
+        live |= uint32_t(left > 0) << c;
+        rank[c] = 0;
+      }
+      if (!live) break;
+      __syncwarp();
+      for (uint32_t rest = live; rest; rest &= rest - 1) {
+        const uint32_t* w = S.ids[__ffs(rest) - 1];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {  // (the own list: the lane)
+          uint32_t lo = 0;
+#pragma unroll
+          for (int step = 16; step > 0; step >>= 1) lo += w[lo + step - 1] < id[c] ? step : 0;
+          rank[c] += lo + (w[lo] < id[c]);
+        }
+      }
+      uint32_t m = 0;
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        const bool take = id[c] <= bound;
+        if (take) S.order[rank[c]] = (pos[c] + lane) | uint32_t(c) << 29;
+        const uint32_t taken = __popc(__ballot_sync(0xffffffffu, take));
+        pos[c] += taken;
+        m += taken;
+      }
+      __syncwarp();  // (the ids are read too: the next round may write them)
+      PointTerm t;
+      int corner = 0;
+      const auto fetch = [&](uint32_t e) {
+        if (e >= m) return;
+        const uint32_t o = S.order[e], at = o & 0x1FFFFFFFu;
+        corner = int(o >> 29);
+        load(ids(at), at, t);
+      };
+      fetch(lane);
+      for (uint32_t b = 0; b < m; b += 32) {
+        if (b + lane < m) {
+          if (SCALAR) {
+            // (a zero gradient is left out of the sum: x + -0 = x for every x)
+            S.term[lane] = t.g[0] == 0.f ? -0.f : density_corner_term(t.g[0], t.u, t.v, t.w, corner);
+          } else {
+            const float scale = corner_scale(t, corner);
+#pragma unroll
+            for (int q = 0; q < 12; ++q) S.term[q * 33 + lane] = __fmul_rn(t.g[q], scale);
+          }
+        }
+        __syncwarp();
+        fetch(b + 32 + lane);  // these travel while the lanes add
+        if (lane < nch) {
+          const float* row = S.term + lane * 33;
+          if (m - b >= 32) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) acc = __fadd_rn(acc, row[j]);
+          } else {
+            for (uint32_t j = 0; j < m - b; ++j) acc = __fadd_rn(acc, row[j]);
+          }
+        }
+        __syncwarp();
+      }
+    }
+    if (lane < nch) {
+      float* dst = grad + int64_t(V.slot) * C + ch0 + lane;
+      *dst = __fadd_rn(*dst, acc);
+    }
+  }
+  if (touched && lane == 0) touched[V.slot >> 9] = 1;
+}
+
 // A point's term from the call's arrays.
 struct ArrayLoad {
   const PointSrc& src;
@@ -668,8 +796,12 @@ __device__ __forceinline__ uint32_t lattice_key(const CellLattice& L, int i, int
   return (((x >> 3) * L.ext[1] + (y >> 3)) * L.ext[2] + (z >> 3)) << 9 |
          unsigned(vox_offset(x, y, z));
 }
-__global__ void k_point_cells(CellLattice L, PointSrc src, int64_t n, uint32_t* keys) {
+// (also clears the count of the call's leaves, as k_point_compact does: a memset
+// between the launches would hold up the ones behind it)
+__global__ void k_point_cells(CellLattice L, PointSrc src, int64_t n, uint32_t* keys,
+                              uint32_t* nleaves) {
   grid_dep_sync();
+  if (blockIdx.x == 0 && threadIdx.x == 0) *nleaves = 0;
   const int64_t p = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   if (p >= n) return;
   float x, y, z;
@@ -696,8 +828,9 @@ __global__ void __launch_bounds__(256)
 }
 __global__ void __launch_bounds__(256)
     k_point_compact(CellLattice L, PointSrc src, int64_t n, const uint32_t* __restrict__ offs,
-                    uint32_t* keys, uint32_t* ids) {
+                    uint32_t* keys, uint32_t* ids, uint32_t* nleaves) {
   grid_dep_sync();
+  if (blockIdx.x == 0 && threadIdx.x == 0) *nleaves = 0;
   __shared__ uint32_t wc[kPtItems][8];  // points of each 32-point group, then their offsets
   const int64_t b0 = int64_t(blockIdx.x) * kPtBlock;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -737,9 +870,11 @@ __global__ void __launch_bounds__(256)
     k_point_group(GridView g, CellLattice L, PointSrc src, const uint32_t* __restrict__ skeys,
                   const uint32_t* __restrict__ svals, int64_t n_max, const uint32_t* n_dev,
                   uint2* cells, float4* rec, uint8_t* touched, uint32_t* mark, uint32_t epoch,
-                  int32_t* list, uint32_t* count, const uint32_t* __restrict__ status) {
+                  int32_t* list, uint32_t* count, uint32_t* nlong,
+                  const uint32_t* __restrict__ status) {
   grid_dep_sync();
   if (*status) return;  // the sort gave up a wait: its order is wrong
+  if (blockIdx.x == 0 && threadIdx.x == 0) *nlong = 0;
   const int64_t n = eff_size(n_max, n_dev);
   for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n;
        i += int64_t(gridDim.x) * blockDim.x) {
@@ -776,19 +911,6 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-__global__ void __launch_bounds__(256)
-    k_point_clear(const uint32_t* __restrict__ skeys, int64_t n_max, const uint32_t* n_dev,
-                  uint2* cells, const uint32_t* __restrict__ status) {
-  grid_dep_sync();
-  if (*status) return;
-  const int64_t n = eff_size(n_max, n_dev);
-  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n;
-       i += int64_t(gridDim.x) * blockDim.x) {
-    const uint32_t key = skeys[i];
-    if (key != kInvalidKey && (i == 0 || skeys[i - 1] != key)) cells[key] = make_uint2(0u, 0u);
-  }
-}
-
 // A sorted point's term from its record, and (without grouped features) the
 // call's gradients.
 template <bool VEC>
@@ -822,24 +944,26 @@ struct RecLoad {
   }
 };
 
-// Thread per voxel of the touched leaves; neighbouring threads read
-// neighbouring table entries and records.
+// Thread per voxel of the listed leaves; neighbouring threads read neighbouring
+// table entries and records. Long voxels are listed.
 template <bool SCALAR, bool VEC>
 __global__ void __launch_bounds__(kVoxelThreads, SCALAR ? 7 : VEC ? 6 : 4)
     k_point_gather(GridView g, CellLattice L, const int32_t* __restrict__ list,
                    const uint32_t* __restrict__ count, const uint32_t* __restrict__ svals,
                    const uint2* __restrict__ cells, const float4* __restrict__ rec, PointSrc src,
+                   int64_t n_max, const uint32_t* n_dev, LongVoxel* longs, uint32_t* nlong,
                    const uint32_t* __restrict__ status) {
   grid_dep_sync();
   if (*status) return;
   const int64_t nv = int64_t(*count) * kLeafVox;
+  const uint32_t most = long_from(eff_size(n_max, n_dev));
   for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < nv;
        i += int64_t(gridDim.x) * blockDim.x) {
     const int leaf = __ldg(list + (i >> 9)), vox = int(i & 511);
     const int vi = __ldg(g.origin + leaf * 3) + (vox >> 6),
               vj = __ldg(g.origin + leaf * 3 + 1) + ((vox >> 3) & 7),
               vk = __ldg(g.origin + leaf * 3 + 2) + (vox & 7);
-    uint32_t first[8], end[8], some = 0;
+    uint32_t first[8], end[8], points = 0;
 #pragma unroll
     for (int c = 0; c < 8; ++c) {
       int di, dj, dk;
@@ -847,13 +971,43 @@ __global__ void __launch_bounds__(kVoxelThreads, SCALAR ? 7 : VEC ? 6 : 4)
       const uint2 e = __ldg(cells + lattice_key(L, vi - di, vj - dj, vk - dk));
       first[c] = e.x;
       end[c] = e.y;
-      some |= e.y;
+      points += e.y - e.x;
     }
-    if (!some) continue;
+    if (!points) continue;
+    const int64_t slot = int64_t(leaf) * kLeafVox + vox;
+    if (points > most) {
+      longs[atomicAdd(nlong, 1u)].set(first, end, slot);
+      continue;
+    }
     merge_voxel<SCALAR, SCALAR ? 4 : 2>(
         src.C, [&](uint32_t pos) { return __ldg(svals + pos); },
-        [&](int ch0, int nch) { return RecLoad<VEC>{rec, src, ch0, nch}; }, first, end,
-        int64_t(leaf) * kLeafVox + vox, g.grad, nullptr);
+        [&](int ch0, int nch) { return RecLoad<VEC>{rec, src, ch0, nch}; }, first, end, slot,
+        g.grad, nullptr);
+  }
+}
+
+// A warp per long voxel (they lie side by side: a block of the gather's would have
+// dozens, most blocks none); then the table's entries are cleared, thread per point.
+template <bool SCALAR, bool VEC>
+__global__ void __launch_bounds__(kVoxelThreads)
+    k_point_long(GridView g, const LongVoxel* __restrict__ longs,
+                 const uint32_t* __restrict__ nlong, const uint32_t* __restrict__ skeys,
+                 const uint32_t* __restrict__ svals, const float4* __restrict__ rec, PointSrc src,
+                 int64_t n_max, const uint32_t* n_dev, uint2* cells,
+                 const uint32_t* __restrict__ status) {
+  grid_dep_sync();
+  if (*status) return;
+  __shared__ LongWarp S[kVoxelThreads / 32];
+  const uint32_t nl = *nlong, w = threadIdx.x >> 5;
+  for (uint32_t k = w * gridDim.x + blockIdx.x; k < nl; k += gridDim.x * (kVoxelThreads / 32))
+    merge_long<SCALAR>(
+        S[w], longs[k], src.C, [&](uint32_t pos) { return __ldg(svals + pos); },
+        [&](int ch0, int nch) { return RecLoad<VEC>{rec, src, ch0, nch}; }, g.grad, nullptr);
+  const int64_t n = eff_size(n_max, n_dev);
+  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n;
+       i += int64_t(gridDim.x) * blockDim.x) {
+    const uint32_t key = skeys[i];
+    if (key != kInvalidKey && (i == 0 || skeys[i - 1] != key)) cells[key] = make_uint2(0u, 0u);
   }
 }
 
@@ -909,11 +1063,15 @@ __global__ void __launch_bounds__(1024)
 }
 
 template <bool SCALAR>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(kVoxelThreads)
     k_point_small_gather(GridView g, CellLattice L, const uint64_t* __restrict__ sorted, int n,
                          PointSrc src, uint8_t* touched) {
   grid_dep_sync();
   __shared__ __align__(16) uint64_t w[kSmallPoints];
+  __shared__ LongVoxel longs[kVoxelThreads];
+  __shared__ LongWarp S[kVoxelThreads / 32];
+  __shared__ int nlong;
+  if (threadIdx.x == 0) nlong = 0;
   const ulonglong2* s2 = reinterpret_cast<const ulonglong2*>(sorted);
 #pragma unroll
   for (int b = 0; b < kSmallPoints / 256; ++b) {  // (the words behind n are not used)
@@ -922,53 +1080,66 @@ __global__ void __launch_bounds__(128)
   }
   __syncthreads();
   const int t = blockIdx.x * 128 + threadIdx.x, i = t >> 3, c = t & 7;
-  if (i >= n) return;
-  const uint64_t cell = w[i] >> kSmallBits;
-  if (cell == kNoPoint >> kSmallBits || (i > 0 && (w[i - 1] >> kSmallBits) == cell)) return;
-  int di, dj, dk;
-  corner_delta(c, di, dj, dk);
-  const int vi = int(cell >> 28) - 1 + di, vj = int(cell >> 14 & 0x3FFFu) - 1 + dj,
-            vk = int(cell & 0x3FFFu) - 1 + dk;
-  const int slot = slot_of(g, vi, vj, vk);
-  if (slot < 0) return;
-  // the eight cells' lists: their binary searches, then the walks to their ends,
-  // side by side
-  uint64_t want[8];
-  uint32_t first[8], end[8];
-#pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    int ei, ej, ek;
-    corner_delta(q, ei, ej, ek);
-    want[q] = small_cell(L, vi - ei, vj - ej, vk - ek);
-    first[q] = 0;
-  }
-#pragma unroll 1
-  for (int step = kSmallPoints; step > 0; step >>= 1) {
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const uint32_t at = first[q] + step;
-      if (at <= uint32_t(n) && (w[at - 1] >> kSmallBits) < want[q]) first[q] = at;
+  // the voxel at corner c of point i's cell, if point i is the first of its cell
+  int slot = -1, vi = 0, vj = 0, vk = 0;
+  if (i < n) {
+    const uint64_t cell = w[i] >> kSmallBits;
+    if (cell != kNoPoint >> kSmallBits && (i == 0 || (w[i - 1] >> kSmallBits) != cell)) {
+      int di, dj, dk;
+      corner_delta(c, di, dj, dk);
+      vi = int(cell >> 28) - 1 + di;
+      vj = int(cell >> 14 & 0x3FFFu) - 1 + dj;
+      vk = int(cell & 0x3FFFu) - 1 + dk;
+      slot = slot_of(g, vi, vj, vk);
     }
   }
+  const auto ids = [&](uint32_t pos) { return uint32_t(w[pos]) & (kSmallPoints - 1); };
+  const auto make_load = [&](int ch0, int nch) { return ArrayLoad{src, ch0, nch}; };
+  if (slot >= 0) {
+    // the eight cells' lists: the binary searches of their first points, then of
+    // their ends, side by side
+    uint64_t want[8];
+    uint32_t first[8], end[8];
 #pragma unroll
-  for (int q = 0; q < 8; ++q) end[q] = first[q];
-  for (bool more = true; more;) {
-    more = false;
+    for (int q = 0; q < 8; ++q) {
+      int ei, ej, ek;
+      corner_delta(q, ei, ej, ek);
+      want[q] = small_cell(L, vi - ei, vj - ej, vk - ek);
+      first[q] = 0;
+    }
+#pragma unroll 1
+    for (int step = kSmallPoints; step > 0; step >>= 1) {
 #pragma unroll
-    for (int q = 0; q < 8; ++q)
-      if (end[q] < uint32_t(n) && (w[end[q]] >> kSmallBits) == want[q]) {
-        ++end[q];
-        more = true;
+      for (int q = 0; q < 8; ++q) {
+        const uint32_t at = first[q] + step;
+        if (at <= uint32_t(n) && (w[at - 1] >> kSmallBits) < want[q]) first[q] = at;
       }
-  }
-  bool owner = true;  // (another thread takes the voxel at its first cell with points)
+    }
 #pragma unroll
-  for (int q = 0; q < 8; ++q) owner = owner && (q >= c || end[q] == first[q]);
-  if (!owner) return;
-  merge_voxel<SCALAR, kSmallBatch>(
-      src.C, [&](uint32_t pos) { return uint32_t(w[pos]) & (kSmallPoints - 1); },
-      [&](int ch0, int nch) { return ArrayLoad{src, ch0, nch}; }, first, end, slot, g.grad,
-      touched);
+    for (int q = 0; q < 8; ++q) end[q] = first[q];
+#pragma unroll 1
+    for (int step = kSmallPoints; step > 0; step >>= 1) {
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const uint32_t at = end[q] + step;
+        if (at <= uint32_t(n) && (w[at - 1] >> kSmallBits) <= want[q]) end[q] = at;
+      }
+    }
+    bool owner = true;  // (another thread takes the voxel at its first cell with points)
+    uint32_t points = 0;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      owner = owner && (q >= c || end[q] == first[q]);
+      points += end[q] - first[q];
+    }
+    if (owner && points > kLongLeast)
+      longs[atomicAdd(&nlong, 1)].set(first, end, slot);
+    else if (owner)
+      merge_voxel<SCALAR, kSmallBatch>(src.C, ids, make_load, first, end, slot, g.grad, touched);
+  }
+  __syncthreads();
+  for (int k = threadIdx.x >> 5; k < nlong; k += kVoxelThreads / 32)
+    merge_long<SCALAR>(S[threadIdx.x >> 5], longs[k], src.C, ids, make_load, g.grad, touched);
 }
 
 // Largest cell table the point backward keeps per grid (1 GiB, about 500^3
@@ -1039,7 +1210,12 @@ static int point_backward_cells(pvdb_grid_s* g, const CellLattice& L, int64_t nc
   ReduceScratch& rs = g->red;
   int rc = cell_table(g, ncells, st);
   if (rc || (rc = reduce_reserve(g, n))) return rc;
-  if ((rc = dev_reserve((void**)&rs.rec, &rs.rec_cap, size_t(n) * (src.vec ? 64 : 16)))) return rc;
+  // the records, then the list of the long voxels
+  const size_t rec_bytes = size_t(n) * (src.vec ? 64 : 16);
+  if ((rc = dev_reserve((void**)&rs.rec, &rs.rec_cap,
+                        rec_bytes + size_t(most_long_voxels(n)) * sizeof(LongVoxel))))
+    return rc;
+  LongVoxel* longs = reinterpret_cast<LongVoxel*>(reinterpret_cast<char*>(rs.rec) + rec_bytes);
   if (!rs.npts && (rc = dev_alloc((void**)&rs.npts, 16))) return rc;
   if (!rs.mark) {
     rs.epoch = 0;
@@ -1050,7 +1226,6 @@ static int point_backward_cells(pvdb_grid_s* g, const CellLattice& L, int64_t nc
     PVDB_CHECK_CUDA(cudaMemsetAsync(rs.mark, 0, size_t(g->nleaf) * 4, st));
   }
   ++rs.epoch;
-  PVDB_CHECK_CUDA(cudaMemsetAsync(g->d_tcount, 0, 4, st));
   g->tlist_valid = false;  // d_tlist takes this call's leaves
   const int bits = slot_key_bits(ncells);
   const uint32_t* n_dev = nullptr;
@@ -1062,20 +1237,20 @@ static int point_backward_cells(pvdb_grid_s* g, const CellLattice& L, int64_t nc
     PVDB_CHECK_LAUNCH("k_point_count");
     if ((rc = scan_exclusive_u32(counts, offs, nb, rs.npts, &rs.partial, &rs.partial_cap, st)))
       return rc;
-    launch_k(k_point_compact, nb, 256, 0, st, L, src, n, offs, rs.keys[0],
-             rs.vals[0]);
+    launch_k(k_point_compact, nb, 256, 0, st, L, src, n, offs, rs.keys[0], rs.vals[0],
+             g->d_tcount);
     PVDB_CHECK_LAUNCH("k_point_compact");
     n_dev = rs.npts;
     rc = radix_sort_pairs_dev(rs, n, n_dev, bits, false, &buf, st, status);
   } else {
-    launch_k(k_point_cells, ceil_div(n, 256), 256, 0, st, L, src, n, rs.keys[0]);
+    launch_k(k_point_cells, ceil_div(n, 256), 256, 0, st, L, src, n, rs.keys[0], g->d_tcount);
     PVDB_CHECK_LAUNCH("k_point_cells");
     rc = radix_sort_pairs(rs, n, bits, true, &buf, st, status);
   }
   if (rc) return rc;
   const uint32_t *skeys = rs.keys[buf], *svals = rs.vals[buf];
   const int sgrid = int(std::min<int64_t>(ceil_div(n, 256), stride_grid()));
-  struct Filled {  // the table, until k_point_clear is launched
+  struct Filled {  // the table, until k_point_long is launched
     ReduceScratch* rs;
     ~Filled() {
       if (rs) free_cells(*rs);
@@ -1083,16 +1258,20 @@ static int point_backward_cells(pvdb_grid_s* g, const CellLattice& L, int64_t nc
   } filled{&rs};
   launch_k(src.vec ? k_point_group<true> : k_point_group<false>, sgrid, 256, 0, st, g->view(), L,
            src, skeys, svals, n, n_dev, rs.cells, rs.rec, g->d_touched, rs.mark, rs.epoch, g->d_tlist,
-           g->d_tcount, *status);
+           g->d_tcount, rs.npts + 1, *status);
   PVDB_CHECK_LAUNCH("k_point_group");
   launch_k(g->C == 1 ? k_point_gather<true, false>
            : src.vec ? k_point_gather<false, true>
                      : k_point_gather<false, false>,
            voxel_grid(g), kVoxelThreads, 0, st, g->view(), L, g->d_tlist, g->d_tcount, svals, rs.cells,
-           rs.rec, src, *status);
+           rs.rec, src, n, n_dev, longs, rs.npts + 1, *status);
   PVDB_CHECK_LAUNCH("k_point_gather");
-  launch_k(k_point_clear, sgrid, 256, 0, st, skeys, n, n_dev, rs.cells, *status);
-  PVDB_CHECK_LAUNCH("k_point_clear");
+  launch_k(g->C == 1 ? k_point_long<true, false>
+           : src.vec ? k_point_long<false, true>
+                     : k_point_long<false, false>,
+           stride_grid(), kVoxelThreads, 0, st, g->view(), longs, rs.npts + 1, skeys, svals, rs.rec,
+           src, n, n_dev, rs.cells, *status);
+  PVDB_CHECK_LAUNCH("k_point_long");
   filled.rs = nullptr;
   return PVDB_OK;
 }
