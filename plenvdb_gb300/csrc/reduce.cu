@@ -826,11 +826,18 @@ __global__ void __launch_bounds__(256)
   block_exclusive_scan(c, &tot);
   if (threadIdx.x == 0) counts[blockIdx.x] = tot;
 }
+// Their cell keys and ids; with PAIRS the slots of their corners and the ids of the
+// pairs, eight a point, and the number of those behind that of the points.
+template <bool PAIRS>
 __global__ void __launch_bounds__(256)
-    k_point_compact(CellLattice L, PointSrc src, int64_t n, const uint32_t* __restrict__ offs,
-                    uint32_t* keys, uint32_t* ids, uint32_t* nleaves) {
+    k_point_compact(GridView g, CellLattice L, PointSrc src, int64_t n,
+                    const uint32_t* __restrict__ offs, uint32_t* keys, uint32_t* ids,
+                    uint32_t* npts, uint32_t* nleaves) {
   grid_dep_sync();
-  if (blockIdx.x == 0 && threadIdx.x == 0) *nleaves = 0;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    *nleaves = 0;
+    if (PAIRS) npts[1] = npts[0] * 8;
+  }
   __shared__ uint32_t wc[kPtItems][8];  // points of each 32-point group, then their offsets
   const int64_t b0 = int64_t(blockIdx.x) * kPtBlock;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -854,8 +861,14 @@ __global__ void __launch_bounds__(256)
     const uint32_t o = base + wc[q][w] + __popc(bal[q] & lanemask_lt());
     float x, y, z;
     src.pos(p, x, y, z);
-    keys[o] = lattice_key(L, ifloor(x), ifloor(y), ifloor(z));
-    ids[o] = uint32_t(p);
+    if (PAIRS) {
+      emit_corner_keys(g, x, y, z, keys, o);
+#pragma unroll
+      for (int c = 0; c < 8; ++c) ids[int64_t(o) * 8 + c] = uint32_t(p) * 8 + c;
+    } else {
+      keys[o] = lattice_key(L, ifloor(x), ifloor(y), ifloor(z));
+      ids[o] = uint32_t(p);
+    }
   }
 }
 
@@ -1142,25 +1155,69 @@ __global__ void __launch_bounds__(kVoxelThreads)
     merge_long<SCALAR>(S[threadIdx.x >> 5], longs[k], src.C, ids, make_load, g.grad, touched);
 }
 
-// Largest cell table the point backward keeps per grid (1 GiB, about 500^3
-// voxels); grids beyond it, or with no memory left for it, sort the (slot,
-// corner) pairs.
+// The form of the backward for n points. Up to kSmallPoints: one block's sort.
+// Beyond, the sort by cell with a table over the lattice, where there are points
+// enough for the leaves that it walks, voxel by voxel, and for the table; else the
+// sort of the (slot, corner) pairs, whose cost is the points' alone. Points over
+// all voxels are as fast either way at n = nslots / 40 to nslots / 20 (pairs and
+// cells, us: 100^3 full 30 k points 100 and 99, 80 k 147 and 119; 256^3 full 600 k 610 and
+// 619, 150 k 215 and 386; a scene at 400^3 (4.5 M slots) 150 k 194 and 212, 300 k 304 and
+// 268), and below some 8192 points the fewer launches win (100^3 full, 5000: 77 and
+// 87). The table takes at most 2 KB a point and 1 GiB.
 constexpr int64_t kMaxCells = int64_t(1) << 27;
+static bool points_by_cell(const pvdb_grid_s* g, int64_t ncells, int64_t n) {
+  return n >= 8192 && n * 20 >= g->nslots() && n * 256 >= ncells && ncells <= kMaxCells;
+}
 
-static int point_backward_pairs(pvdb_grid_s* g, const PointSrc& src, int64_t n, cudaStream_t st,
-                                uint32_t** status) {
+// Scalar grids from this many points on: the pair sort, too, first drops the points
+// without a gradient. Of the samples of rays through a scene one in 16 carries one
+// (240^3, 58 k samples: 162 us without, 96 with it); where all do, the two more
+// passes cost some 5 us (400^3, 50 k points: 124 and 122, 160^3 full 119 and 123).
+constexpr int64_t kPairsCompact = 32768;
+
+// The points of a scalar grid that have a gradient, in order: keys[0], vals[0] and
+// npts of the grid's scratch (keys[1] and vals[1] are free until the sort's first pass).
+template <bool PAIRS>
+static int compact_points(pvdb_grid_s* g, const CellLattice& L, const PointSrc& src, int64_t n,
+                          cudaStream_t st) {
+  ReduceScratch& rs = g->red;
+  int rc;
+  if (!rs.npts && (rc = dev_alloc((void**)&rs.npts, 16))) return rc;
+  const int nb = ceil_div(n, kPtBlock);
+  uint32_t *counts = rs.vals[1], *offs = rs.keys[1];
+  launch_k(k_point_count, nb, 256, 0, st, src.g, n, counts);
+  PVDB_CHECK_LAUNCH("k_point_count");
+  if ((rc = scan_exclusive_u32(counts, offs, nb, rs.npts, &rs.partial, &rs.partial_cap, st)))
+    return rc;
+  launch_k(k_point_compact<PAIRS>, nb, 256, 0, st, g->view(), L, src, n, offs, rs.keys[0],
+           rs.vals[0], rs.npts, g->d_tcount);
+  PVDB_CHECK_LAUNCH("k_point_compact");
+  return PVDB_OK;
+}
+
+static int point_backward_pairs(pvdb_grid_s* g, const CellLattice& L, const PointSrc& src,
+                                int64_t n, cudaStream_t st, uint32_t** status) {
   const int64_t nc = n * 8;
   int rc = reduce_reserve(g, nc);
   if (rc) return rc;
-  launch_k(k_point_keys, ceil_div(n, 256), 256, 0, st, g->view(), src.xs, src.ys, src.zs, n,
-           g->red.keys[0]);
-  PVDB_CHECK_LAUNCH("k_point_keys");
+  g->tlist_valid = false;
+  const bool compact = g->C == 1 && n >= kPairsCompact;
+  const uint32_t* n_dev = nullptr;
+  if (compact) {
+    if ((rc = compact_points<true>(g, L, src, n, st))) return rc;
+    n_dev = g->red.npts + 1;
+  } else {
+    launch_k(k_point_keys, ceil_div(n, 256), 256, 0, st, g->view(), src.xs, src.ys, src.zs, n,
+             g->red.keys[0]);
+    PVDB_CHECK_LAUNCH("k_point_keys");
+  }
   int buf = 0;
-  rc = radix_sort_pairs(g->red, nc, slot_key_bits(g->nslots()), true, &buf, st, status);
+  rc = radix_sort_pairs_dev(g->red, nc, n_dev, slot_key_bits(g->nslots()), !compact, &buf, st,
+                            status);
   if (rc) return rc;
   const int grid = int(std::min<int64_t>(ceil_div(nc, 256), int64_t(num_sms()) * 16));
   launch_k(k_segment_reduce<PointSrc>, grid, 256, 0, st, g->red.keys[buf], g->red.vals[buf], nc,
-           nullptr, src, g->C == 1 ? g->d_grad : nullptr, g->C == 1 ? nullptr : g->d_grad, g->C,
+           n_dev, src, g->C == 1 ? g->d_grad : nullptr, g->C == 1 ? nullptr : g->d_grad, g->C,
            g->d_touched, g->d_touched, *status);
   PVDB_CHECK_LAUNCH("k_segment_reduce");
   return PVDB_OK;
@@ -1231,15 +1288,7 @@ static int point_backward_cells(pvdb_grid_s* g, const CellLattice& L, int64_t nc
   const uint32_t* n_dev = nullptr;
   int buf = 0;
   if (g->C == 1) {
-    const int nb = ceil_div(n, kPtBlock);
-    uint32_t *counts = rs.vals[1], *offs = rs.keys[1];  // free until the sort's first pass
-    launch_k(k_point_count, nb, 256, 0, st, src.g, n, counts);
-    PVDB_CHECK_LAUNCH("k_point_count");
-    if ((rc = scan_exclusive_u32(counts, offs, nb, rs.npts, &rs.partial, &rs.partial_cap, st)))
-      return rc;
-    launch_k(k_point_compact, nb, 256, 0, st, L, src, n, offs, rs.keys[0], rs.vals[0],
-             g->d_tcount);
-    PVDB_CHECK_LAUNCH("k_point_compact");
+    if ((rc = compact_points<false>(g, L, src, n, st))) return rc;
     n_dev = rs.npts;
     rc = radix_sort_pairs_dev(rs, n, n_dev, bits, false, &buf, st, status);
   } else {
@@ -1316,12 +1365,15 @@ extern "C" int pvdb_grid_sample_backward(pvdb_grid g, const float* xs, const flo
   if (n <= kSmallPoints) {
     rc = point_backward_small(g, L, src, int(n), st);
   } else {
-    rc = ncells <= kMaxCells ? point_backward_cells(g, L, ncells, src, n, st, &status)
-                             : int(PVDB_ERR_NOMEM);
-    if (rc == PVDB_ERR_NOMEM) {  // (nothing is added yet: all memory is reserved before)
+    // the form that the points are better off with, and the other one if memory is
+    // missing (all of it is reserved before anything is added)
+    bool cells = points_by_cell(g, ncells, n);
+    for (int attempt = 0;; ++attempt, cells = !cells) {
+      rc = cells ? point_backward_cells(g, L, ncells, src, n, st, &status)
+                 : point_backward_pairs(g, L, src, n, st, &status);
+      if (rc != PVDB_ERR_NOMEM || attempt || (!cells && ncells > kMaxCells)) break;
       clear_error();
-      free_cells(g->red);
-      rc = point_backward_pairs(g, src, n, st, &status);
+      if (cells) free_cells(g->red);
     }
   }
   if (rc) return rc;
