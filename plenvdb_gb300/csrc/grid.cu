@@ -303,14 +303,15 @@ __device__ __forceinline__ float value_c(const GridView& g, int i, int j, int k,
 }
 
 // TV gradient (total_variation_kernel.cu:13-35) on the leaf store, for the
-// voxels of the listed leaves (list = NULL: all leaves), a warp per quarter of
-// a leaf: neighbours inside [0,reso) only, values through the leaf table
-// (background outside allocated leaves). Per channel the sum is formed in the
-// reference's order z-, z+, y-, y+, x-, x+, each term rounded, then added (the
-// reference's conditional terms are not fused, total_variation_kernel.cu:27-32).
+// voxels of the listed leaves (list = NULL: all leaves): neighbours inside
+// [0,reso) only, values through the leaf table (background outside allocated
+// leaves). Per channel the sum is formed in the reference's order z-, z+, y-, y+,
+// x-, x+, each term rounded, then added (the reference's conditional terms are not
+// fused, total_variation_kernel.cu:27-32).
 // TERMS: the sums alone, into out, for every active voxel (0 outside
 // [0, reso)); else they are added to the gradient (sparse: where it is not
-// zero).
+// zero). Three forms: scalar grids (this one) a warp per quarter of a leaf, 12
+// channels in 16-byte loads, any other number of channels a voxel a thread.
 template <bool TERMS>
 __global__ void __launch_bounds__(256)
     k_tv(GridView g, float wx, float wy, float wz, int dense_mode, const int32_t* __restrict__ list,
@@ -321,51 +322,104 @@ __global__ void __launch_bounds__(256)
   for (int64_t u = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5; u < nq;
        u += (int64_t(gridDim.x) * blockDim.x) >> 5) {
     const LeafQuarter L = leaf_quarter(g, list ? list[u >> 2] : int(u >> 2), int(u & 3));
-    for (int ch = 0; ch < g.C; ++ch) {
-      // two slices' values and neighbours are loaded together
+    // two slices' values and neighbours are loaded together
 #pragma unroll 1
-      for (int s0 = 0; s0 < 4; s0 += 2) {
-        float gc[2], p[2], vn[2][6];
-        bool take[2];
-        uint32_t skip[2];  // bit q: no term for neighbour q
+    for (int s0 = 0; s0 < 4; s0 += 2) {
+      float gc[2], p[2], vn[2][6];
+      bool take[2];
+      uint32_t skip[2];  // bit q: no term for neighbour q
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int64_t t = (int64_t(L.leaf) * kLeafVox + L.vox(s0 + e)) * g.C + ch;
-          take[e] = L.active(s0 + e);
-          gc[e] = !TERMS && take[e] ? g.grad[t] : 0.f;
-          if (!TERMS && !dense_mode && gc[e] == 0.f) take[e] = false;
-          p[e] = take[e] ? g.data[t] : 0.f;
+      for (int e = 0; e < 2; ++e) {
+        const int64_t t = int64_t(L.leaf) * kLeafVox + L.vox(s0 + e);
+        take[e] = L.active(s0 + e);
+        gc[e] = !TERMS && take[e] ? g.grad[t] : 0.f;
+        if (!TERMS && !dense_mode && gc[e] == 0.f) take[e] = false;
+        p[e] = take[e] ? g.data[t] : 0.f;
+      }
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int vox = L.vox(s0 + e);
+        const int x = L.x + (vox >> 6), y = L.y + ((vox >> 3) & 7), z = L.z + (vox & 7);
+        const bool in = x < g.reso[0] && y < g.reso[1] && z < g.reso[2];
+        if (!TERMS) take[e] = take[e] && in;
+        int nb[6];
+        face_neighbours(g, L, vox, x, y, z, nb);
+        skip[e] = in ? 0u : 0x3Fu;
+#pragma unroll
+        for (int q = 0; q < 6; ++q) {
+          if (nb[q] == -2) skip[e] |= 1u << q;
+          vn[e][q] = g.background;
+          if (take[e] && nb[q] >= 0) vn[e][q] = g.data[nb[q]];
         }
+      }
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int vox = L.vox(s0 + e);
-          const int x = L.x + (vox >> 6), y = L.y + ((vox >> 3) & 7), z = L.z + (vox & 7);
-          const bool in = x < g.reso[0] && y < g.reso[1] && z < g.reso[2];
-          if (!TERMS) take[e] = take[e] && in;
-          int nb[6];
-          face_neighbours(g, L, vox, x, y, z, nb);
-          skip[e] = in ? 0u : 0x3Fu;
+      for (int e = 0; e < 2; ++e) {
+        if (!take[e]) continue;
+        float add = 0.f;
 #pragma unroll
-          for (int q = 0; q < 6; ++q) {
-            if (nb[q] == -2) skip[e] |= 1u << q;
-            vn[e][q] = g.background;
-            if (take[e] && nb[q] >= 0) vn[e][q] = g.data[int64_t(nb[q]) * g.C + ch];
-          }
-        }
+        for (int q = 0; q < 6; ++q)
+          if (!((skip[e] >> q) & 1u))
+            add = __fadd_rn(add, __fmul_rn(wt[q], tv_clamp(p[e] - vn[e][q])));
+        const int64_t t = int64_t(L.leaf) * kLeafVox + L.vox(s0 + e);
+        if (TERMS)
+          out[t] = add;
+        else
+          g.grad[t] = gc[e] + add;
+      }
+    }
+  }
+}
+
+// Any number of channels, a multiple of 3: a thread per voxel, its neighbours looked
+// up once for all of them and three channels loaded together (15 channels of 820
+// leaves: 29 us; channel by channel 47; looked up again per channel by a warp per
+// quarter leaf 64; 3 channels at 256^3: 273, 454, 361).
+template <bool TERMS>
+__global__ void __launch_bounds__(256)
+    k_tv_any(GridView g, float wx, float wy, float wz, int dense_mode,
+             const int32_t* __restrict__ list, const uint32_t* __restrict__ count,
+             float* __restrict__ out) {
+  grid_dep_sync();
+  const int64_t nl = list ? int64_t(*count) : int64_t(g.nleaf);
+  const float wt[6] = {wz, wz, wy, wy, wx, wx};
+  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < nl * kLeafVox;
+       i += int64_t(gridDim.x) * blockDim.x) {
+    const int vox = int(i & 511);
+    const LeafQuarter L = leaf_quarter(g, list ? list[i >> 9] : int(i >> 9), vox >> 7);
+    if (!L.active((vox >> 5) & 3)) continue;
+    const int x = L.x + (vox >> 6), y = L.y + ((vox >> 3) & 7), z = L.z + (vox & 7);
+    const bool in = x < g.reso[0] && y < g.reso[1] && z < g.reso[2];
+    if (!TERMS && !in) continue;
+    int nb[6];
+    face_neighbours(g, L, vox, x, y, z, nb);
+    const int64_t t0 = (int64_t(L.leaf) * kLeafVox + vox) * g.C;
+    for (int ch = 0; ch < g.C; ch += 3) {  // three channels' loads travel together
+      float gc[3], p[3], vn[6][3], add[3];
+      bool any = TERMS || dense_mode;
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          if (!take[e]) continue;
-          float add = 0.f;
+      for (int e = 0; e < 3; ++e) {
+        gc[e] = TERMS ? 0.f : g.grad[t0 + ch + e];
+        any = any || gc[e] != 0.f;
+      }
+      if (!any) continue;
 #pragma unroll
-          for (int q = 0; q < 6; ++q)
-            if (!((skip[e] >> q) & 1u))
-              add = __fadd_rn(add, __fmul_rn(wt[q], tv_clamp(p[e] - vn[e][q])));
-          const int64_t t = (int64_t(L.leaf) * kLeafVox + L.vox(s0 + e)) * g.C + ch;
-          if (TERMS)
-            out[t] = add;
-          else
-            g.grad[t] = gc[e] + add;
-        }
+      for (int e = 0; e < 3; ++e) p[e] = g.data[t0 + ch + e];
+#pragma unroll
+      for (int q = 0; q < 6; ++q)
+#pragma unroll
+        for (int e = 0; e < 3; ++e)
+          vn[q][e] = nb[q] < 0 ? g.background : g.data[int64_t(nb[q]) * g.C + ch + e];
+#pragma unroll
+      for (int e = 0; e < 3; ++e) {
+        add[e] = 0.f;
+#pragma unroll
+        for (int q = 0; q < 6; ++q)
+          if (in && nb[q] != -2)
+            add[e] = __fadd_rn(add[e], __fmul_rn(wt[q], tv_clamp(p[e] - vn[q][e])));
+        if (TERMS)
+          out[t0 + ch + e] = add[e];
+        else if (dense_mode || gc[e] != 0.f)
+          g.grad[t0 + ch + e] = gc[e] + add[e];
       }
     }
   }
@@ -470,6 +524,11 @@ __global__ void __launch_bounds__(256)
       o4[b] = make_float4(o[0], o[1], o[2], o[3]);
     }
   }
+}
+
+template <bool TERMS>
+static auto tv_kernel(int channels) {
+  return channels == 1 ? k_tv<TERMS> : channels == 12 ? k_tv_c12<TERMS> : k_tv_any<TERMS>;
 }
 
 __global__ void k_touched_compact(const uint8_t* __restrict__ touched, int nleaf, int32_t* list,
@@ -622,7 +681,7 @@ int tv_terms_launch(pvdb_grid_s* g, float wx, float wy, float wz, cudaStream_t s
   wx /= 6.f;
   wy /= 6.f;
   wz /= 6.f;
-  launch_k(g->C == 12 ? k_tv_c12<true> : k_tv<true>, stride_grid(), 256, 0, st, g->view(), wx, wy,
+  launch_k(tv_kernel<true>(g->C), stride_grid(), 256, 0, st, g->view(), wx, wy,
            wz, 0, g->d_tlist, g->d_tcount, g->d_tv);
   PVDB_CHECK_LAUNCH("k_tv_terms");
   return PVDB_OK;
@@ -971,7 +1030,7 @@ int pvdb_grid_tv_add_grad(pvdb_grid g, float wx, float wy, float wz, int32_t den
     int rc = touched_list(g, st);
     if (rc) return rc;
   }
-  launch_k(g->C == 12 ? k_tv_c12<false> : k_tv<false>, stride_grid(), 256, 0, st, g->view(), wx, wy,
+  launch_k(tv_kernel<false>(g->C), stride_grid(), 256, 0, st, g->view(), wx, wy,
            wz, dense_mode ? 1 : 0, use_list ? g->d_tlist : nullptr, g->d_tcount, nullptr);
   PVDB_CHECK_LAUNCH("k_tv");
   if (dense_mode) g->all_touched = true;
