@@ -254,9 +254,14 @@ def stream_of(x=None) -> int | None:
     """The current torch CUDA stream handle (None = legacy default stream)."""
     try:
         import torch
-        if torch.cuda.is_initialized():
-            # the raw handle: building a Stream object for it costs more than a launch
-            return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
-    except Exception:
-        pass
-    return None
+    except Exception:  # no usable torch: the library alone
+        return None
+    if not torch.cuda.is_initialized():
+        return None
+    # the raw handle where torch has these two (not public): building a Stream object
+    # for it costs more than a launch
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    device = getattr(torch._C, "_cuda_getDevice", None)
+    if raw is None or device is None:
+        return torch.cuda.current_stream().cuda_stream
+    return raw(device())
