@@ -3,9 +3,9 @@
 // Data: an index leaf store (voxel -> row id, 0 = empty; the voxels with a row
 // are the active ones) plus per-row density and k0 features (FP32, or BF16
 // features with FP32 density). Loading lays the density out per voxel of the
-// allocated leaves, and 12-channel features too, with one more record that
-// holds row 0 (every voxel outside the leaves): a trilinear corner is then one
-// load at its slot, not a row id and a load behind it.
+// allocated leaves, and 12-channel features too (if there is memory for them),
+// with one more record that holds row 0 (every voxel outside the leaves): a
+// trilinear corner is then one load at its slot, not a row id and a load behind it.
 //
 // Per frame:
 //   k_render_march         a warp per 32 pixels: get_rays (renderer.cu:122-167)
@@ -74,11 +74,11 @@ struct RenderP {
   GridView idx;               // topology; values unused
   int nslots;
   const float* vden;          // [nslots + 1]
-  const float* vcol;          // [nslots + 1][12] (12 channels, storage 0)
-  const __nv_bfloat16* vcolh; // [nslots + 1][kHalfStride] (12 channels, storage 1)
-  const int32_t* rows;        // [nslots] row id of every in-leaf voxel (other channel counts)
-  const float* col;           // [N*dcol] (other channel counts, storage 0)
-  const __nv_bfloat16* colh;  // [N*dcol] (other channel counts, storage 1)
+  const float* vcol;          // [nslots + 1][12] (features per voxel, storage 0)
+  const __nv_bfloat16* vcolh; // [nslots + 1][kHalfStride] (features per voxel, storage 1)
+  const int32_t* rows;        // [nslots] row id of every in-leaf voxel (features in rows)
+  const float* col;           // [N*dcol] (features in rows, storage 0)
+  const __nv_bfloat16* colh;  // [N*dcol] (features in rows, storage 1)
   int storage;
 };
 
@@ -628,7 +628,9 @@ struct pvdb_renderer_s {
   int dcol, dpe, dhid, dout;
   bool flags[5] = {false, false, false, false, false};
   pvdb_grid_s* topo = nullptr;
-  // 12 channels: per-voxel records only; other counts: row ids and rows
+  // 12 channels: per-voxel features; other counts, or no memory for them (an index
+  // whose voxels share rows has far more voxels than rows): row ids and rows
+  bool voxels = false;
   int32_t* d_rows = nullptr;
   float* d_vden = nullptr;
   float* d_col = nullptr;           // rows, or the per-voxel records
@@ -812,7 +814,6 @@ int pvdb_renderer_load_data(pvdb_renderer r, const int32_t reso[3], const int32_
   r->d_colh = nullptr;
   const int64_t ns = r->topo->nslots();
   const size_t nf = size_t(n_rows) * r->dcol;
-  const bool voxels = r->dcol == 12;
   // device copies of the inputs, freed on every way out
   struct Temp {
     int32_t *dense = nullptr, *rows = nullptr;
@@ -830,11 +831,18 @@ int pvdb_renderer_load_data(pvdb_renderer r, const int32_t reso[3], const int32_
       (rc = dev_alloc((void**)&tmp.col, nf * 4)) ||
       (rc = dev_alloc((void**)&r->d_vden, (ns + 1) * 4)))
     return rc;
-  if (storage == 0)
-    rc = dev_alloc((void**)&r->d_col, voxels ? size_t(ns + 1) * 48 : nf * 4);
-  else
-    rc = dev_alloc((void**)&r->d_colh, voxels ? size_t(ns + 1) * kHalfStride * 2 : nf * 2);
-  if (rc) return rc;
+  bool voxels = r->dcol == 12;
+  for (;;) {
+    if (storage == 0)
+      rc = dev_alloc((void**)&r->d_col, voxels ? size_t(ns + 1) * 48 : nf * 4);
+    else
+      rc = dev_alloc((void**)&r->d_colh, voxels ? size_t(ns + 1) * kHalfStride * 2 : nf * 2);
+    if (!rc) break;
+    if (!voxels || rc != PVDB_ERR_NOMEM) return rc;
+    clear_error();
+    voxels = false;
+  }
+  r->voxels = voxels;
   const cudaMemcpyKind kind = mem == PVDB_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
   PVDB_CHECK_CUDA(cudaMemcpy(tmp.dense, index, nvox * 4, kind));
   PVDB_CHECK_CUDA(cudaMemcpy(tmp.den, density, n_rows * 4, kind));
@@ -1040,8 +1048,8 @@ int pvdb_renderer_render(pvdb_renderer r, int32_t precision, pvdb_stream s) {
   a.c0 = r->dcol;
   a.dpe = r->dpe;
   a.din = din;
-  // 12 BF16 channels and the BF16 rgbnet: the rgbnet gathers the features itself
-  const bool gather = precision == 1 && r->dcol == 12 && r->storage == 1;
+  // 12 BF16 channels a voxel and the BF16 rgbnet: the rgbnet gathers the features itself
+  const bool gather = precision == 1 && r->voxels && r->storage == 1;
   uint4* pex = reinterpret_cast<uint4*>(r->d_hpe);  // 96 of the 640 bytes a pixel
   if (total) {
     const int64_t M = total;
@@ -1053,14 +1061,14 @@ int pvdb_renderer_render(pvdb_renderer r, int32_t precision, pvdb_stream s) {
         const int64_t ntiles = (r->rows_cap + 127) / 128;
         if ((rc = dev_reserve(&r->d_xt, &r->xt_cap, size_t(ntiles) * kRgbXTile))) return rc;
         uint8_t* xt = static_cast<uint8_t*>(r->d_xt);
-        if (r->dcol == 12)
+        if (r->voxels)
           k_render_x<12><<<rgrid, 256, 0, st>>>(P, Wk, M, pex, xt);
         else
           k_render_x<0><<<rgrid, 256, 0, st>>>(P, Wk, M, pex, xt);
         PVDB_CHECK_LAUNCH("k_render_x");
       }
     } else {
-      if (r->dcol == 12)
+      if (r->voxels)
         k_render_k0<12><<<rgrid, 256, 0, st>>>(P, Wk, M);
       else
         k_render_k0<0><<<rgrid, 256, 0, st>>>(P, Wk, M);
