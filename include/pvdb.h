@@ -78,6 +78,11 @@ int pvdb_debug_wait_limit(uint32_t spins, int32_t hold_first);
  * bitwise identical results. Applies to launches made after the call (a
  * captured train-step graph keeps the variant it was captured with). */
 int pvdb_debug_k0_blocks(int blocks);
+/* Test hook (no counterpart in the reference): with on != 0 renderers allocate
+ * frame buffers for exactly the rows and batches that a frame was seen to need,
+ * one of each at first, so that small frames take the path of a frame that
+ * outgrows its buffers and is marched again. */
+int pvdb_debug_render_exact(int on);
 
 /* Stage profiler. Between begin and end, pvdb_train_step and
  * pvdb_renderer_render record CUDA events on their stream at stage boundaries

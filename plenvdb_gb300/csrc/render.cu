@@ -33,6 +33,7 @@
 // pixel's rows are added in do not. A frame with more rows than the buffers
 // hold is marched again after they have grown.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -665,9 +666,13 @@ struct pvdb_renderer_s {
   size_t xt_cap = 0;
 };
 
+// Test hook (pvdb_debug_render_exact): buffers of exactly what is asked for, one row
+// and one batch at first, so that a small frame outgrows them.
+static std::atomic<int> g_dbg_exact{0};
+
 static int renderer_grow_batches(pvdb_renderer_s* r, int64_t need) {
   if (need <= r->batch_cap) return PVDB_OK;
-  const int64_t cap = need + need / 4 + 4096;
+  const int64_t cap = g_dbg_exact ? need : need + need / 4 + 4096;
   dev_free(r->d_batch);
   r->d_batch = nullptr;
   r->batch_cap = 0;
@@ -708,7 +713,7 @@ static std::vector<int32_t> leaf_distances(const pvdb_grid_s* g) {
 
 static int renderer_grow_rows(pvdb_renderer_s* r, int64_t need) {
   if (need <= r->rows_cap) return PVDB_OK;
-  const int64_t cap = std::max<int64_t>(need + need / 4, 1 << 20);
+  const int64_t cap = g_dbg_exact ? need : std::max<int64_t>(need + need / 4, 1 << 20);
   void* ptrs[] = {r->d_rk0, r->d_rw, r->d_rxyz, r->d_rpix, r->d_part};
   for (void* p : ptrs) dev_free(p);
   r->d_rk0 = r->d_rw = r->d_rxyz = r->d_part = nullptr;
@@ -734,6 +739,11 @@ static int wait_gave_up(pvdb_renderer_s* r, cudaStream_t st) {
 }
 
 extern "C" {
+
+int pvdb_debug_render_exact(int on) {
+  g_dbg_exact.store(on);
+  return PVDB_OK;
+}
 
 int pvdb_renderer_create(int32_t dcol, int32_t dpe, int32_t dhid, int32_t dout,
                          pvdb_renderer* out) {
@@ -1011,7 +1021,7 @@ int pvdb_renderer_render(pvdb_renderer r, int32_t precision, pvdb_stream s) {
   prof_begin_call();
   prof_mark(st, 0);
   int rc = renderer_grow_rows(r, 1);
-  if (!rc) rc = renderer_grow_batches(r, tiles);
+  if (!rc) rc = renderer_grow_batches(r, g_dbg_exact ? 1 : tiles);
   if (rc) return rc;
   uint32_t total = 0;
   for (;;) {
