@@ -629,14 +629,14 @@ RGBNET_FWD_ROW, RGBNET_FWD_RAY, RGBNET_BWD_ROW = 36608.0, 6912.0, 73216.0
 # (cold L2; the grids are L2-resident in the live step, so these are the
 # bytes a launch pulls from HBM, not the algorithmic bytes above)
 NCU_TRAFFIC = {
-    "march_fwd": 2.133e6 + 11.115e6,   # k_march_alpha + k_march_chain
-    "k0_gather": 9.627e6,              # k_march_k0_x
-    "rgbnet_fwd": 14.691e6,            # k_mlp_fwd_tc
-    "rgbnet_bwd": 18.388e6,            # k_mlp_bwd_tc
-    "march_bwd": 7.145e6,              # k_march_bwd
-    "voxel_gather": 11.030e6 + 26.148e6,  # k_group_records + k_voxel_gather
-    "tv": 12.608e6,                    # k_tv_c12<true> (the density grid's k_tv<true> not captured)
-    "voxel_adam": 52.651e6 + 3.142e6 + 6.055e6,  # k_vdb_adam_c12 + k_vdb_adam1
+    "march_fwd": 2.142e6 + 11.147e6,   # k_march_alpha + k_march_chain
+    "k0_gather": 9.710e6,              # k_march_k0_x
+    "rgbnet_fwd": 14.771e6,            # k_mlp_fwd_tc
+    "rgbnet_bwd": 18.465e6,            # k_mlp_bwd_tc
+    "march_bwd": 7.188e6,              # k_march_bwd
+    "voxel_gather": 11.080e6 + 26.326e6,  # k_group_records + k_voxel_gather
+    "tv": 12.611e6 + 1.417e6,          # k_tv_c12<true> + k_tv<true>
+    "voxel_adam": 58.288e6 + 6.146e6,  # k_vdb_adam_c12 + k_vdb_adam1
 }
 
 
