@@ -83,6 +83,9 @@ class MGRenderer:
         self.timer += time.perf_counter() - t0
 
     def output_an_image(self, device: bool = False):
+        """The last frame [H*W*3], on the host or (device=True, without waiting for it)
+        as a CUDA tensor. A frame whose rgbnet gave up a bounded wait raises
+        PvdbError here, or for device=True in the next render_an_image."""
         H, W = self._hw
         if device:
             import torch
