@@ -639,12 +639,12 @@ __device__ __forceinline__ void merge_voxel(int C, const Ids& ids, const MakeLoa
 // A voxel with more points than long_from is summed by a warp (merge_long): its
 // thread would take them one after another, some 0.6 us each, twice what the pair
 // sort's walk takes. A warp takes a voxel's points 12 times as fast but is a warp:
-// where many voxels are long, their threads together are faster, and their one
-// longest voxel does not count. So 32 points up to 64 k points in the call, 128
-// from 256 k. (160^3, 30 k points at 600 voxels: 152 us from 128 up, 101 from 64 or
-// 32, 384 without; 1.8 M points over the scene: 519, 900, 1053, 522 us.)
+// where very many voxels are long, their threads together are faster, and their one
+// longest voxel does not count. So 32 points up to 512 k points in the call, 128
+// from 2 M. (160^3, 30 k points at 600 voxels: 384 us by threads, 98 by warps; 1.8 M
+// points over the scene: 522 by threads, 669 by warps from 32 points on, 520 so.)
 __device__ __forceinline__ uint32_t long_from(int64_t n) {
-  return uint32_t(min(max(n >> 11, int64_t(32)), int64_t(128)));
+  return uint32_t(min(max(n >> 14, int64_t(32)), int64_t(128)));
 }
 constexpr uint32_t kLongLeast = 32;
 struct LongVoxel {
@@ -662,17 +662,19 @@ struct LongVoxel {
 // The most that n points have of them.
 inline int64_t most_long_voxels(int64_t n) { return n * 8 / (kLongLeast + 1); }
 // A warp's space to sum one.
-struct LongWarp {
+struct alignas(16) LongWarp {
   uint32_t ids[8][32];   // the next points of each list
   uint32_t order[256];   // their merge: position | list << 29
   float term[12 * 33];   // [channel][point]
 };
 
-// merge_voxel by a warp, the same sums in the same order. A round takes the next
-// 32 points of every list. What lies up to the smallest of the lists' last ids is
-// complete, and ranked by counting the smaller ids of each list; then 32 points
-// at a time are loaded and multiplied by the lanes side by side, and a lane per
-// channel adds them in order.
+// merge_voxel by a warp, the same sums in the same order. The points are put in
+// order first: up to kLongOnce at once, each counting the smaller ids among all;
+// more in rounds, of the next 32 points of every list. What lies up to the smallest
+// of the lists' last ids is complete, and ranked by counting the smaller ids of each
+// list. Then 32 points at a time are loaded and multiplied by the lanes side by
+// side, and a lane per channel adds them in order.
+constexpr uint32_t kLongOnce = 128;
 template <bool SCALAR, class Ids, class MakeLoad>
 __device__ __forceinline__ void merge_long(LongWarp& S, const LongVoxel& V, int C, const Ids& ids,
                                            const MakeLoad& make_load, float* grad,
@@ -681,44 +683,9 @@ __device__ __forceinline__ void merge_long(LongWarp& S, const LongVoxel& V, int 
   for (int ch0 = 0; ch0 < (SCALAR ? 1 : C); ch0 += 12) {
     const int nch = SCALAR ? 1 : min(12, C - ch0);
     const auto load = make_load(ch0, nch);
-    uint32_t pos[8];
-#pragma unroll
-    for (int c = 0; c < 8; ++c) pos[c] = V.first[c];
     float acc = 0.f;
-    for (;;) {
-      uint32_t id[8], rank[8], bound = kInvalidKey - 1u, live = 0;
-#pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        const uint32_t left = V.end[c] - pos[c];
-        id[c] = uint32_t(lane) < left ? ids(pos[c] + lane) : kInvalidKey;
-        S.ids[c][lane] = id[c];
-        const uint32_t last = __shfl_sync(0xffffffffu, id[c], 31);
-        if (left > 32) bound = min(bound, last);
-        live |= uint32_t(left > 0) << c;
-        rank[c] = 0;
-      }
-      if (!live) break;
-      __syncwarp();
-      for (uint32_t rest = live; rest; rest &= rest - 1) {
-        const uint32_t* w = S.ids[__ffs(rest) - 1];
-#pragma unroll
-        for (int c = 0; c < 8; ++c) {  // (the own list: the lane)
-          uint32_t lo = 0;
-#pragma unroll
-          for (int step = 16; step > 0; step >>= 1) lo += w[lo + step - 1] < id[c] ? step : 0;
-          rank[c] += lo + (w[lo] < id[c]);
-        }
-      }
-      uint32_t m = 0;
-#pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        const bool take = id[c] <= bound;
-        if (take) S.order[rank[c]] = (pos[c] + lane) | uint32_t(c) << 29;
-        const uint32_t taken = __popc(__ballot_sync(0xffffffffu, take));
-        pos[c] += taken;
-        m += taken;
-      }
-      __syncwarp();  // (the ids are read too: the next round may write them)
+    // adds the points order[0 .. m - 1]
+    const auto add_points = [&](uint32_t m) {
       PointTerm t;
       int corner = 0;
       const auto fetch = [&](uint32_t e) {
@@ -729,34 +696,114 @@ __device__ __forceinline__ void merge_long(LongWarp& S, const LongVoxel& V, int 
       };
       fetch(lane);
       for (uint32_t b = 0; b < m; b += 32) {
-        if (b + lane < m) {
-          if (SCALAR) {
-            // (a zero gradient is left out of the sum: x + -0 = x for every x)
-            S.term[lane] = t.g[0] == 0.f ? -0.f : density_corner_term(t.g[0], t.u, t.v, t.w, corner);
-          } else {
-            const float scale = corner_scale(t, corner);
+        // (x + -0 = x for every x: behind the last point, and for a zero gradient of a
+        // scalar grid, which is left out of the sum)
+        const bool in = b + lane < m;
+        if (SCALAR) {
+          S.term[lane] = !in || t.g[0] == 0.f
+                             ? -0.f
+                             : density_corner_term(t.g[0], t.u, t.v, t.w, corner);
+        } else {
+          const float scale = in ? corner_scale(t, corner) : 0.f;
 #pragma unroll
-            for (int q = 0; q < 12; ++q) S.term[q * 33 + lane] = __fmul_rn(t.g[q], scale);
-          }
+          for (int q = 0; q < 12; ++q)
+            S.term[q * 33 + lane] = in ? __fmul_rn(t.g[q], scale) : -0.f;
         }
         __syncwarp();
         fetch(b + 32 + lane);  // these travel while the lanes add
         if (lane < nch) {
           const float* row = S.term + lane * 33;
-          if (m - b >= 32) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) acc = __fadd_rn(acc, row[j]);
-          } else {
-            for (uint32_t j = 0; j < m - b; ++j) acc = __fadd_rn(acc, row[j]);
-          }
+          for (int j = 0; j < 32; ++j) acc = __fadd_rn(acc, row[j]);
         }
         __syncwarp();
+      }
+    };
+    uint32_t pos[8], total = 0, most = 0;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      pos[c] = V.first[c];
+      const uint32_t n = V.end[c] - pos[c];
+      total += n;
+      most = max(most, n);
+    }
+    if (total <= kLongOnce) {
+      uint32_t* id = &S.ids[0][0];
+      uint32_t* where = reinterpret_cast<uint32_t*>(S.term);
+      for (uint32_t l = lane; l < most; l += 32) {
+        uint32_t at = l;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          const uint32_t n = V.end[c] - pos[c];
+          if (l < n) {
+            id[at] = ids(pos[c] + l);
+            where[at] = (pos[c] + l) | uint32_t(c) << 29;
+          }
+          at += n;
+        }
+      }
+      if (lane < 3) id[total + lane] = kInvalidKey;  // to a whole group of four
+      __syncwarp();
+      uint32_t mine[kLongOnce / 32], rank[kLongOnce / 32];
+#pragma unroll
+      for (uint32_t j = 0; j < kLongOnce / 32; ++j) {
+        mine[j] = lane + 32 * j < total ? id[lane + 32 * j] : 0u;
+        rank[j] = 0;
+      }
+      for (uint32_t i = 0; i < total; i += 4) {
+        const uint4 w = *reinterpret_cast<const uint4*>(id + i);
+#pragma unroll
+        for (uint32_t j = 0; j < kLongOnce / 32; ++j)
+          rank[j] += (w.x < mine[j]) + (w.y < mine[j]) + (w.z < mine[j]) + (w.w < mine[j]);
+      }
+#pragma unroll
+      for (uint32_t j = 0; j < kLongOnce / 32; ++j)
+        if (lane + 32 * j < total) S.order[rank[j]] = where[lane + 32 * j];
+      __syncwarp();  // (the terms may be written over `where`)
+      add_points(total);
+    } else {
+      for (;;) {
+        uint32_t id[8], rank[8], bound = kInvalidKey - 1u, live = 0;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          const uint32_t left = V.end[c] - pos[c];
+          id[c] = uint32_t(lane) < left ? ids(pos[c] + lane) : kInvalidKey;
+          S.ids[c][lane] = id[c];
+          const uint32_t last = __shfl_sync(0xffffffffu, id[c], 31);
+          if (left > 32) bound = min(bound, last);
+          live |= uint32_t(left > 0) << c;
+          rank[c] = 0;
+        }
+        if (!live) break;
+        __syncwarp();
+        for (uint32_t rest = live; rest; rest &= rest - 1) {
+          const uint32_t* w = S.ids[__ffs(rest) - 1];
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {  // (the own list: the lane)
+            uint32_t lo = 0;
+#pragma unroll
+            for (int step = 16; step > 0; step >>= 1) lo += w[lo + step - 1] < id[c] ? step : 0;
+            rank[c] += lo + (w[lo] < id[c]);
+          }
+        }
+        uint32_t m = 0;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          const bool take = id[c] <= bound;
+          if (take) S.order[rank[c]] = (pos[c] + lane) | uint32_t(c) << 29;
+          const uint32_t taken = __popc(__ballot_sync(0xffffffffu, take));
+          pos[c] += taken;
+          m += taken;
+        }
+        __syncwarp();  // (the ids are read too: the next round may write them)
+        add_points(m);
       }
     }
     if (lane < nch) {
       float* dst = grad + int64_t(V.slot) * C + ch0 + lane;
       *dst = __fadd_rn(*dst, acc);
     }
+    __syncwarp();
   }
   if (touched && lane == 0) touched[V.slot >> 9] = 1;
 }

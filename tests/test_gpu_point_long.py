@@ -89,3 +89,23 @@ def test_given_up_sort_leaves_the_gradient(lib, channels):
     np.testing.assert_array_equal(a.get_dense_grid(which=L.WHICH_GRAD),
                                   b.get_dense_grid(which=L.WHICH_GRAD))
     assert np.any(b.get_dense_grid(which=L.WHICH_GRAD))
+
+
+@pytest.mark.parametrize("channels", [1, 12, 15])
+@pytest.mark.parametrize("n", [127, 128, 129, 130])
+def test_at_once_and_in_rounds(lib, channels, n):
+    """Points around the most that a warp orders at once, spread over the eight lists
+    in every way that leaves some of them empty, long or of one point."""
+    rng = np.random.default_rng(n + channels)
+    for part in range(6):
+        w = rng.random(8) ** (1 + 3 * part)
+        w[rng.random(8) < 0.1 * part] = 0
+        w[part] += 0.1
+        cell = rng.choice(8, n, p=w / w.sum())
+        if part == 5:
+            cell.sort()  # one list after the other
+        base = np.array([6, 7, 8]) - np.stack([cell >> 2, (cell >> 1) & 1, cell & 1], -1)
+        xyz = base + rng.uniform(0.01, 0.99, (n, 3))
+        g = rng.normal(0, 1, (n, channels))
+        g[rng.random(n) < 0.05] = 0.0
+        _run(channels, xyz, g, 0 if part % 2 else 20000)
