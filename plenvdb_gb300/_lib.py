@@ -259,10 +259,9 @@ def stream_of(x=None) -> int | None:
         return None
     if not torch.cuda.is_initialized():
         return None
-    # the raw handle where torch has these two (not public): building a Stream object
-    # for it costs more than a launch
-    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
-    device = getattr(torch._C, "_cuda_getDevice", None)
-    if raw is None or device is None:
+    try:
+        # the raw handle (not public): building a Stream object for it costs more than
+        # a launch
+        return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+    except AttributeError:
         return torch.cuda.current_stream().cuda_stream
-    return raw(device())
